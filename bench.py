@@ -42,7 +42,7 @@ INDEX_ORDER = [3, 2, 1, 0]  # c(i,j,k,l) = a(i,j,k,l) + b(l,k,j,i)
 WORKLOAD = ("sparse merge c(i,j,k,l)=a(i,j,k,l)+b(l,k,j,i): order-4 SparseMIA dims 512^4, "
             "2^26 nnz per operand, uniform coordinates, f64 values U[-1,1], both unsorted (sortMerge: "
             "re-key A to {3,2,1,0}, concatenate, radix-sort the 2^27 (u64,f64) pairs, collect duplicates)")
-IMPLEMENTATION = ("bucket histogram (A re-keyed on the fly), two 8-bit onesweep passes over the top 15 key bits, "
+IMPLEMENTATION = ("bucket histogram (A re-keyed on the fly), two partition passes over the top 15 key bits, "
                   "per-bucket shared-memory sort with the duplicate fold fused")
 HBM_FALLBACK_GBS = 6650.0
 L2_NOTE = "inputs (2 GiB) and sort buffers larger than the 126 MB L2; no flush needed"
@@ -416,7 +416,7 @@ def run_ours(args):
     ms = max_over_ranks(ms, world)
     value = job_throughput(n, world, ms)
     kernels = {}
-    for name in ("sort_hist", "sort_onesweep", "bucket_sort_collect", "collect_lead", "collect",
+    for name in ("sort_hist", "sort_partition", "bucket_sort_collect", "collect_lead", "collect",
                  "sort_hist_fallback", "sort_onesweep_fallback", "collect_lead_fallback", "collect_fallback"):
         t, c = L.profile_query(name)
         kernels[name] = {"ms_total": t, "launches": c}
@@ -525,15 +525,15 @@ def run_ours(args):
     # output pair once.  DRAM traffic per pair from the committed
     # ncu summary of the merge.
     peak, peak_kind = peaks()
-    prof_file = "onesweep8_bucket_merge_512x4_2x64M"
+    prof_file = "partition_bucket_merge_512x4_2x64M"
     cands = {
-        "sort_onesweep": ("one digit pass (7 then 8 bits) of the bucketed sort over 2^27 (u64,f64) pairs", 32.0 * n,
+        "sort_partition": ("one partition pass (7 then 8 bits) of the bucketed sort over 2^27 (u64,f64) pairs", 32.0 * n,
                           "traffic_bytes_per_pair"),
         "bucket_sort_collect": ("per-bucket shared-memory sort + duplicate fold of the 2^27 pairs",
                                 16.0 * n + 16.0 * n_out, "bucket_traffic_bytes_per_pair"),
     }
     # every timed merge kernel's algorithmic bytes and fraction of the HBM peak
-    per_launch_bytes = {"sort_hist": 8.0 * n, "sort_onesweep": 32.0 * n,
+    per_launch_bytes = {"sort_hist": 8.0 * n, "sort_partition": 32.0 * n,
                         "bucket_sort_collect": 16.0 * n + 16.0 * n_out}
     for name, b in per_launch_bytes.items():
         kk = kernels[name]

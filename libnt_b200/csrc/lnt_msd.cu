@@ -1,0 +1,870 @@
+// Bucketed sort of (u64 key, f64 value) pairs, optionally folding equal keys:
+//
+//   1. msd_hist_kernel: one read of all (re-keyed, concatenated) keys counts
+//      the 2^T buckets named by the top T key bits (T <= 15); the last CTA
+//      derives the bucket starts, the partition passes' cursors and the gate.
+//   2. one (T <= 8) or two partition passes group the pairs by bucket, most
+//      significant digit first: a CTA takes a tile, ranks its pairs within
+//      their digits by shared-memory atomics, reserves room for each digit
+//      with one global atomic and writes the tile's digit runs.  The rank is
+//      not stable, so the passes need no ballots, no per-warp counters and no
+//      look-back; the order is restored at the end because every pair carries
+//      its input index below its key (word = key << ib | index; the bits that
+//      a pass has used up may fall off the top).  The second pass partitions
+//      each first-pass segment for itself.
+//   3. bucket_sort_kernel: one CTA per bucket sorts its words (low key bits,
+//      then index: the stable order) in shared memory: the words are counted
+//      into sub-buckets, placed, and ranked within their sub-bucket (a merge
+//      sort instead when a sub-bucket is crowded).  FOLD adds up runs of
+//      equal keys in input order and writes at offsets from a look-back over
+//      the buckets; a plain sort knows its offsets already.
+//
+// DRAM traffic: 8 B (histogram) + 32 B per pass + 16 B + 16 B per pair.
+// Measured on 2^27 pairs with 36-bit keys (B200): histogram 0.45 ms (bound by
+// issue: re-key and count), partition passes 0.81 and 0.86 ms (80% of the
+// measured copy rate), bucket kernel 1.85 ms (bound by the latency of its
+// block-wide phases and of the look-back); 4.08 ms against 5.93 ms for the
+// stable 7- and 8-bit onesweep passes (1.59 + 1.30 ms: eight ballots, a
+// per-warp counter and a look-back per pass) and a bucket kernel whose threads
+// each ranked ten words by looping over their sub-buckets (2.43 ms).
+#include <algorithm>
+#include <cstdlib>
+
+#include "lnt_msd.cuh"
+
+namespace lnt {
+namespace {
+
+constexpr int kHistThreads = 1024;
+constexpr int kMaxT = 15;
+constexpr int kMaxDigits = 256;
+// Partition tile: 256 threads x 8 records, four CTAs per SM at 64 registers.
+// What matters is that nothing spills: 12 records per thread ran the same
+// (0.84 + 0.85 ms for the two passes over 2^27 pairs against 0.81 + 0.86), 16
+// per thread spilled and took 1.16 + 1.17 ms.
+constexpr int kPartThreads = 256, kPartItems = 8, kPartBlocks = 4;
+constexpr int kPartTile = kPartThreads * kPartItems;
+constexpr unsigned long long kFlagAgg = 1ull << 62;
+constexpr unsigned long long kFlagPre = 2ull << 62;
+constexpr unsigned long long kFlagMask = 3ull << 62;
+constexpr unsigned long long kValMask = (1ull << 62) - 1ull;
+
+// A bucket's records are counted into 2^SUBB sub-buckets (8-bit counts, four
+// to a word), about four per record, so that most records are alone in theirs.
+template <int BT, int ITEMS, int SUBB>
+struct BucketGeom {
+  static constexpr int kBT = BT;
+  static constexpr int kWarps = BT / 32;
+  static constexpr int kItems = ITEMS;
+  static constexpr int kCap = BT * ITEMS;
+  static constexpr int kSubBits = SUBB;
+  static constexpr int kSubWords = 1 << (SUBB - 2);
+  static constexpr int kSubPer = kSubWords / BT;  // count words per thread
+  static constexpr int kGroups = kCap / 32;       // 32-position groups
+  static constexpr int kMinBlocks = BT >= 512 ? 2 : 4;
+  static constexpr size_t smem = (size_t)kCap * 16 + (size_t)kSubWords * 6 + (size_t)kGroups * 8 + 64 * 4;
+  static_assert(kSubPer == 8, "one uint4 of 16-bit starts per thread");
+};
+using GeomLarge = BucketGeom<512, 10, 14>;
+using GeomSmall = BucketGeom<256, 10, 13>;
+// largest expected bucket (uniform keys): four fifths of the capacity
+constexpr double kAvgLarge = 4096.0, kAvgSmall = 2048.0;
+constexpr int kSubMax = 48;  // largest sub-bucket ranked by comparing its words
+
+struct MsdCtrl {
+  u32* counts;    // 2^T
+  u32* start;     // 2^T + 1
+  u32* cur1;      // first pass cursors (up to 256)
+  u32* cur2;      // second pass cursors (2^T)
+  u32* segtile;   // second pass: first tile of every segment (up to 257)
+  u32* misc;      // [0] histogram CTAs done, [1] bucket counter
+  unsigned long long* status;  // 2^T look-back words (FOLD)
+  u32* gate;      // 0: every bucket fits a CTA, 1: take the LSD path
+};
+
+// Bucket counts in shared memory as 16-bit fields (two per word, 64 KB at
+// T = 15: two 1024-thread CTAs per SM).  A field keeps 15 bits; the increment
+// that takes it to 2^15 moves 2^15 to the bucket's global count and clears bit
+// 15 again, so no field carries into its neighbour (the other increments that
+// can land in between are far fewer than 2^15).
+__device__ __forceinline__ void count16(u32* sh, u32 b, const MsdCtrl& c) {
+  const u32 sh_bits = 16u * (b & 1u);
+  const u32 old = atomicAdd(&sh[b >> 1], 1u << sh_bits);
+  if (((old >> sh_bits) & 0x7FFFu) == 0x7FFFu) {  // rare: once per 2^15 keys of one bucket in one CTA
+    atomicSub(&sh[b >> 1], 0x8000u << sh_bits);
+    atomicAdd(&c.counts[b], 0x8000u);
+  }
+}
+
+// Re-keys I keys in place (those whose bit is set in `use`): the loop over the
+// modes is outside the one over the keys, so that the code stays small
+// whatever the order.
+template <int I>
+__device__ __forceinline__ void rekey_items(u64 (&k)[I], const RekeyParams& p, u32 use) {
+  if (p.order <= 1 || use == 0u) return;
+  u64 out[I];
+#pragma unroll
+  for (int j = 0; j < I; ++j) out[j] = 0;
+  if (p.pow2) {
+#pragma unroll 1
+    for (int m = 0; m < p.order; ++m) {
+      const u32 f = p.field[m];
+      const u32 from = f & 63u, to = (f >> 16) & 63u;
+      const u64 mask = (1ull << ((f >> 8) & 63u)) - 1ull;
+#pragma unroll
+      for (int j = 0; j < I; ++j) out[j] |= ((k[j] >> from) & mask) << to;
+    }
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) k[j] = out[j];
+    return;
+  }
+#pragma unroll 1
+  for (int m = p.order - 1; m >= 1; --m) {
+    const Divider dv = p.acc[m];
+    const u64 mult = p.mult[m];
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) {
+        const u64 q = divide(k[j], dv);
+        out[j] += q * mult;
+        k[j] -= q * dv.d;
+      }
+  }
+  const u64 m0 = p.mult[0];
+#pragma unroll
+  for (int j = 0; j < I; ++j)
+    if (use & (1u << j)) k[j] = out[j] + k[j] * m0;
+}
+
+// Loads I keys at positions base + j * stride + tid (those below `end`; 0
+// beyond) of the concatenated source and re-keys them.
+template <int I>
+__device__ __forceinline__ void source_keys(const PairSource& s, u32 base, u32 stride, u32 end, u64 (&k)[I]) {
+  const u32 first = base + threadIdx.x;
+  const bool all_a = end <= s.na, all_b = base >= s.na;
+  u32 in_a = 0;
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 i = first + j * stride;
+    k[j] = 0;
+    if (all_a || (!all_b && i < s.na)) {
+      in_a |= 1u << j;
+      if (i < end) k[j] = __ldcs(s.ak + i);
+    } else if (i < end) {
+      k[j] = __ldcs(s.bk + (i - s.na));
+    }
+  }
+  if (!all_b) rekey_items(k, s.ra, in_a);
+  if (!all_a) rekey_items(k, s.rb, ~in_a);
+}
+
+__global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSource src, u32 n, int T, int db,
+                                                                   int shift, u32 cap, MsdCtrl c) {
+  extern __shared__ u32 sh[];  // 2^T 16-bit fields
+  __shared__ bool s_last;
+  __shared__ u32 s_w[kHistThreads / 32], s_mx[kHistThreads / 32];
+  const int nb = 1 << T, nw = (nb + 1) >> 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < nw; i += kHistThreads) sh[i] = 0;
+  __syncthreads();
+  const u32 bmask = (u32)(nb - 1);
+  constexpr int U = 4;
+  for (u64 base = (u64)blockIdx.x * (kHistThreads * U); base < n; base += (u64)gridDim.x * (kHistThreads * U)) {
+    const u32 end = (u32)min((u64)n, base + kHistThreads * U);
+    u64 k[U];
+    source_keys<U>(src, (u32)base, kHistThreads, end, k);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if ((u32)base + u * kHistThreads + tid < end) count16(sh, (u32)(k[u] >> shift) & bmask, c);
+  }
+  __syncthreads();
+  for (int b = tid; b < nb; b += kHistThreads) {
+    const u32 v = (sh[b >> 1] >> (16 * (b & 1))) & 0xFFFFu;
+    if (v) atomicAdd(&c.counts[b], v);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&c.misc[0], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // ---- last CTA: bucket starts and cursors, the largest bucket ----
+  const int per = (nb + kHistThreads - 1) / kHistThreads;
+  u32 local = 0, mx = 0;
+  for (int j = 0; j < per; ++j) {
+    const int b = tid * per + j;
+    const u32 v = b < nb ? __ldcg(&c.counts[b]) : 0u;
+    local += v;
+    mx = max(mx, v);
+  }
+  u32 inc = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 31) s_w[warp] = inc;
+  if (lane == 0) s_mx[warp] = mx;
+  __syncthreads();
+  u32 run = inc - local;
+  for (int w = 0; w < warp; ++w) run += s_w[w];
+  const u32 dmask = (1u << db) - 1u;
+  for (int j = 0; j < per; ++j) {
+    const int b = tid * per + j;
+    if (b < nb) {
+      c.start[b] = run;
+      c.cur2[b] = run;
+      if (((u32)b & dmask) == 0u) c.cur1[b >> db] = run;  // a first-pass segment begins here
+      run += __ldcg(&c.counts[b]);
+    }
+  }
+  if (tid == 0) {
+    u32 m = 0;
+    for (int w = 0; w < kHistThreads / 32; ++w) m = max(m, s_mx[w]);
+    *c.gate = m > cap ? 1u : 0u;
+    c.start[nb] = n;
+  }
+  __threadfence_block();
+  __syncthreads();
+  // ---- tiles of the second pass per segment (at most 256 segments) ----
+  const int nseg = nb >> db;
+  u32 tiles = 0;
+  if (tid < nseg) {
+    const u32 s0 = c.start[tid << db], s1 = c.start[(tid + 1) << db];
+    tiles = (s1 - s0 + kPartTile - 1) / kPartTile;
+  }
+  u32 tinc = tiles;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 t = __shfl_up_sync(0xffffffffu, tinc, o);
+    if (lane >= o) tinc += t;
+  }
+  __syncthreads();
+  if (lane == 31) s_w[warp] = tinc;
+  __syncthreads();
+  u32 tb = tinc - tiles;
+  for (int w = 0; w < warp; ++w) tb += s_w[w];
+  if (tid < nseg) c.segtile[tid] = tb;
+  if (tid == nseg) c.segtile[nseg] = tb;
+}
+
+template <int THREADS, int ITEMS, int MINB>
+struct PartShape {
+  static constexpr int kThreads = THREADS, kItems = ITEMS, kMinBlocks = MINB;
+  static constexpr int kTile = THREADS * ITEMS;
+  static constexpr int kPer = kMaxDigits / THREADS;  // digits per thread
+  static constexpr size_t smem = (size_t)kTile * 16 + kMaxDigits * 8 + 128;
+};
+
+// One partition pass over records (word, value).  FIRST reads the source and
+// builds the words; otherwise the records of every segment (first-pass digit)
+// are partitioned among the buckets of that segment.  DIGITS: the digit of
+// every staged record is kept beside it (FIRST, when the word has lost it).
+template <class P, bool FIRST, bool DIGITS>
+__global__ void __launch_bounds__(P::kThreads, P::kMinBlocks)
+    partition_kernel(const PairSource src, const ulonglong2* __restrict__ in, ulonglong2* __restrict__ out, u32 n,
+                     int ib, int dshift, u32 dmask, int nseg, int db, const MsdCtrl c) {
+  if (gated_off(c.gate, 0)) return;  // a bucket is too large: the LSD path runs instead
+  constexpr int T = P::kThreads, I = P::kItems, PER = P::kPer;
+  extern __shared__ __align__(16) unsigned char smem[];
+  ulonglong2* s_r = reinterpret_cast<ulonglong2*>(smem);         // tile records in digit order
+  u32* s_cnt = reinterpret_cast<u32*>(s_r + P::kTile);           // per digit: count, then destination - tile start
+  u32* s_ts = s_cnt + kMaxDigits;                                // per digit: first slot in the tile
+  u32* s_misc = s_ts + kMaxDigits;                               // 32
+  unsigned char* s_d = reinterpret_cast<unsigned char*>(s_misc + 32);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) s_cnt[q * T + tid] = 0;
+  u32 base, tile_n;
+  u32* cursor;
+  if (FIRST) {
+    base = blockIdx.x * (u32)P::kTile;
+    tile_n = min((u32)P::kTile, n - base);
+    cursor = c.cur1;
+  } else {
+    if (blockIdx.x >= c.segtile[nseg]) return;
+    for (int q = tid; q < nseg; q += T) {  // the segment this tile belongs to
+      const u32 t0 = c.segtile[q], t1 = c.segtile[q + 1];
+      if (t0 <= blockIdx.x && blockIdx.x < t1) {
+        const u32 s0 = c.start[(u32)q << db], s1 = c.start[(u32)(q + 1) << db];
+        const u32 b = s0 + (blockIdx.x - t0) * (u32)P::kTile;
+        s_misc[16] = (u32)q;
+        s_misc[17] = b;
+        s_misc[18] = min((u32)P::kTile, s1 - b);
+      }
+    }
+  }
+  __syncthreads();
+  if (!FIRST) {
+    cursor = c.cur2 + (s_misc[16] << db);
+    base = s_misc[17];
+    tile_n = s_misc[18];
+  }
+  u64 w[I];
+  double v[I];
+  u32 slot[I];
+  if (FIRST) {
+    source_keys<I>(src, base, (u32)T, base + tile_n, w);
+    const bool all_a = base + tile_n <= src.na, all_b = base >= src.na;
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * T + tid, i = base + p;
+      v[j] = 0.0;
+      if (all_a || (!all_b && i < src.na)) {
+        if (p < tile_n) v[j] = __ldcs(src.av + i);
+      } else if (p < tile_n) {
+        v[j] = __ldcs(src.bv + (i - src.na));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * T + tid;
+      ulonglong2 r = make_ulonglong2(0, 0);
+      if (p < tile_n) r = __ldcs(in + base + p);
+      w[j] = r.x;
+      v[j] = __longlong_as_double((long long)r.y);
+    }
+  }
+  // rank within the digit by one shared atomic per pair; one per warp and
+  // item where the warp's 32 pairs share their digit, as in key-ordered input
+  // (32 atomics on one address would take turns)
+  const u32 d0 = (u32)(w[0] >> dshift) & dmask;
+  if (__all_sync(0xffffffffu, d0 == __shfl_sync(0xffffffffu, d0, 0))) {
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * T + tid;
+      const u32 d = (u32)(w[j] >> dshift) & dmask;
+      const u32 df = __shfl_sync(0xffffffffu, d, 0);
+      if (__all_sync(0xffffffffu, d == df && p < tile_n)) {
+        u32 b = 0;
+        if (lane == 0) b = atomicAdd(&s_cnt[df], 32u);
+        slot[j] = __shfl_sync(0xffffffffu, b, 0) + lane;
+      } else {
+        slot[j] = p < tile_n ? atomicAdd(&s_cnt[d], 1u) : 0u;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * T + tid;
+      slot[j] = p < tile_n ? atomicAdd(&s_cnt[(u32)(w[j] >> dshift) & dmask], 1u) : 0u;
+    }
+  }
+  __syncthreads();
+  {  // reserve room in each digit's range; exclusive scan of the counts
+    u32 cnt[PER], g[PER], sum = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      cnt[q] = s_cnt[tid * PER + q];
+      g[q] = cnt[q] ? atomicAdd(cursor + tid * PER + q, cnt[q]) : 0u;  // (digits beyond dmask have no pairs)
+      sum += cnt[q];
+    }
+    u32 inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_misc[warp] = inc;
+    __syncthreads();
+    u32 ts = inc - sum;
+#pragma unroll
+    for (int q = 0; q < T / 32; ++q) ts += q < warp ? s_misc[q] : 0u;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      s_ts[tid * PER + q] = ts;
+      s_cnt[tid * PER + q] = g[q] - ts;
+      ts += cnt[q];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 p = j * T + tid;
+    if (p < tile_n) {
+      const u32 d = (u32)(w[j] >> dshift) & dmask;
+      const u32 q = s_ts[d] + slot[j];
+      u64 x = w[j];
+      double y = v[j];
+      if (FIRST) {
+        x = (x << ib) | (u64)(base + p);
+        if (base + p >= src.na) y *= src.bscale;
+        if (DIGITS) s_d[q] = (unsigned char)d;
+      }
+      s_r[q] = make_ulonglong2(x, (u64)__double_as_longlong(y));
+    }
+  }
+  __syncthreads();
+  const int wshift = FIRST ? dshift + ib : dshift;
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 p = j * T + tid;
+    if (p < tile_n) {
+      const ulonglong2 r = s_r[p];
+      const u32 d = DIGITS ? (u32)s_d[p] : (u32)(r.x >> wshift) & dmask;
+      out[s_cnt[d] + p] = r;
+    }
+  }
+}
+
+// Sorts the records s_r[0, cap) by word in place (cap = BT * ITEMS; the unused
+// ones hold ~0): ITEMS records per thread by odd-even transposition, then
+// merge rounds over doubling groups of threads, each thread finding its output
+// range by a merge-path search.
+template <class G>
+__device__ __noinline__ void bucket_merge_sort(ulonglong2* s_r) {
+  constexpr int I = G::kItems;
+  const int tid = threadIdx.x;
+  ulonglong2 x[I];
+#pragma unroll
+  for (int j = 0; j < I; ++j) x[j] = s_r[tid * I + j];
+#pragma unroll
+  for (int r = 0; r < I; ++r)
+#pragma unroll
+    for (int j = r & 1; j + 1 < I; j += 2) {
+      const ulonglong2 p = x[j], q = x[j + 1];
+      x[j] = p.x < q.x ? p : q;
+      x[j + 1] = p.x < q.x ? q : p;
+    }
+#pragma unroll
+  for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
+  for (int g = 1; g < G::kBT; g <<= 1) {  // merge runs of g * I records
+    __syncthreads();
+    const int first = (tid / (2 * g)) * 2 * g * I;
+    const ulonglong2* a = s_r + first;
+    const ulonglong2* b = a + g * I;
+    const int len = g * I, d = (tid % (2 * g)) * I;
+    int lo = d > len ? d - len : 0, hi = d < len ? d : len;
+    while (lo < hi) {
+      const int m = (lo + hi) >> 1;
+      if (a[m].x <= b[d - 1 - m].x) lo = m + 1; else hi = m;
+    }
+    int ia = lo, ib = d - lo;
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const bool ta = ib >= len || (ia < len && a[ia].x <= b[ib].x);
+      x[j] = ta ? a[ia] : b[ib];
+      ia += ta ? 1 : 0;
+      ib += ta ? 0 : 1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
+  }
+  __syncthreads();
+}
+
+// Sorts the k records of one sub-bucket by word (one thread); FOLD adds up its
+// runs of equal keys in that (input) order into their first record and clears
+// the kept bits of the others and of the dropped ones.  `at`: the position of
+// r[0] in the bucket; first: it is the first of the whole sorted array.
+template <bool FOLD>
+__device__ __forceinline__ void fold_sub_bucket(ulonglong2* r, int k, int ib, int skip_zero_heads, bool first, u32 at,
+                                                u32* kept) {
+  for (int i = 1; i < k; ++i) {  // insertion sort
+    const ulonglong2 x = r[i];
+    int q = i;
+    for (; q > 0; --q) {
+      const ulonglong2 y = r[q - 1];
+      if (y.x < x.x) break;
+      r[q] = y;
+    }
+    if (q != i) r[q] = x;
+  }
+  if (!FOLD) return;
+  for (int i = 0; i < k;) {
+    const u64 low = r[i].x >> ib;
+    double sum = __longlong_as_double((long long)r[i].y);
+    bool anynz = sum != 0.0;
+    int q = i + 1;
+    for (; q < k && (r[q].x >> ib) == low; ++q) {
+      const double y = __longlong_as_double((long long)r[q].y);
+      sum += y;
+      anynz |= y != 0.0;
+      atomicAnd(&kept[(at + q) >> 5], ~(1u << ((at + q) & 31)));
+    }
+    if (q > i + 1) r[i].y = (u64)__double_as_longlong(sum);
+    if (skip_zero_heads && !anynz && !(first && i == 0)) atomicAnd(&kept[(at + i) >> 5], ~(1u << ((at + i) & 31)));
+    i = q;
+  }
+}
+
+template <class G, bool FOLD>
+__global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
+    bucket_sort_kernel(const ulonglong2* __restrict__ rec, const MsdCtrl c, int T, int shift, int ib,
+                       int skip_zero_heads, u64* __restrict__ out_k, double* __restrict__ out_v,
+                       u64* __restrict__ d_nout) {
+  if (gated_off(c.gate, 0)) return;
+  constexpr int BT = G::kBT, I = G::kItems, W = G::kWarps, P2 = (I + 1) / 2;
+  extern __shared__ __align__(16) unsigned char smem[];
+  ulonglong2* s_r = reinterpret_cast<ulonglong2*>(smem);       // kCap records in sub-bucket order
+  u32* s_cnt = reinterpret_cast<u32*>(s_r + G::kCap);              // sub-bucket counts, four to a word
+  unsigned short* s_base = reinterpret_cast<unsigned short*>(s_cnt + G::kSubWords);  // records before each word's
+  u32* s_kept = reinterpret_cast<u32*>(s_base + G::kSubWords);     // per 32 positions: kept mask
+  u32* s_pre = s_kept + G::kGroups;                                // per 32 positions: kept before them
+  u32* s_misc = s_pre + G::kGroups;                                // 64
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int sb = min(shift, G::kSubBits);
+  const int sshift = ib + shift - sb;
+  const u64 wmask = ib + shift >= 64 ? ~0ull : (1ull << (ib + shift)) - 1ull;
+  if (FOLD && tid == 0) s_misc[0] = atomicAdd(&c.misc[1], 1u);
+#pragma unroll
+  for (int j = 0; j < G::kSubPer; ++j) s_cnt[j * BT + tid] = 0;
+  if (tid == 0) s_misc[1] = 0;
+  __syncthreads();
+  const u32 b = FOLD ? s_misc[0] : blockIdx.x;  // FOLD: in order of arrival, for the look-back
+  const u32 start = c.start[b];
+  const u32 cnt = min(c.start[b + 1] - start, (u32)G::kCap);  // (the gate is open: no bucket exceeds kCap)
+  rec += start;
+  if (FOLD)  // every position is kept until its record turns out not to be the first of its run
+    for (int x = tid; x < G::kGroups; x += BT)
+      s_kept[x] = x * 32 + 32 <= cnt ? ~0u : x * 32 < cnt ? (1u << (cnt - x * 32)) - 1u : 0u;
+  ulonglong2 r[I];
+  u32 pos[P2];  // 16 bits per item
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 p = j * BT + tid;
+    r[j] = make_ulonglong2(~0ull, 0);
+    if (p < cnt) {
+      r[j] = __ldcs(rec + p);
+      r[j].x &= wmask;
+    }
+  }
+  {  // count the sub-buckets; slot of every record in its own
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * BT + tid;
+      const u32 sub = (u32)(r[j].x >> sshift), sh = 8u * (sub & 3u);
+      const u32 slot = p < cnt ? (atomicAdd(&s_cnt[sub >> 2], 1u << sh) >> sh) & 0xFFu : 0u;
+      pos[j / 2] = j & 1 ? pos[j / 2] | (slot << 16) : slot;
+    }
+    u32 most = 0;
+#pragma unroll
+    for (int j = 0; j < P2; ++j) most = __vmaxu2(most, pos[j]);
+    // crowded (some slot at the limit): the counts may have run over, and are not used
+    if (max(most & 0xFFFFu, most >> 16) >= (u32)kSubMax) s_misc[1] = 1;
+  }
+  __syncthreads();
+  {  // records before every count word
+    u32 sum = 0;
+    u32 c8[8];
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&s_cnt[tid * 8 + j]);
+      c8[j] = __dp4a(q.x, 0x01010101u, 0u);
+      c8[j + 1] = __dp4a(q.y, 0x01010101u, 0u);
+      c8[j + 2] = __dp4a(q.z, 0x01010101u, 0u);
+      c8[j + 3] = __dp4a(q.w, 0x01010101u, 0u);
+      sum += c8[j] + c8[j + 1] + c8[j + 2] + c8[j + 3];
+    }
+    u32 inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_misc[8 + warp] = inc;
+    __syncthreads();
+    u32 run = inc - sum;
+#pragma unroll
+    for (int q = 0; q < W; ++q) run += q < warp ? s_misc[8 + q] : 0u;
+    u32 pk[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const u32 lo = run;
+      run += c8[2 * j];
+      pk[j] = (lo & 0xFFFFu) | (run << 16);
+      run += c8[2 * j + 1];
+    }
+    *reinterpret_cast<uint4*>(&s_base[tid * 8]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  }
+  __syncthreads();
+  const bool ranked = s_misc[1] == 0;
+#pragma unroll
+  for (int j = 0; j < I; ++j) {  // place every record in its sub-bucket (crowded: as they are, to be sorted)
+    const u32 p = j * BT + tid;
+    u32 q = p;
+    if (ranked && p < cnt) {
+      const u32 sub = (u32)(r[j].x >> sshift), sh = 8u * (sub & 3u), c4 = s_cnt[sub >> 2];
+      q = s_base[sub >> 2] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u) +
+          ((pos[j / 2] >> (16 * (j & 1))) & 0xFFFFu);
+      // alone in its sub-bucket and zero: dropped (unless it is the first of all)
+      if (FOLD && skip_zero_heads && ((c4 >> sh) & 0xFFu) == 1u && __longlong_as_double((long long)r[j].y) == 0.0 &&
+          start + q != 0)
+        atomicAnd(&s_kept[q >> 5], ~(1u << (q & 31)));
+    }
+    s_r[q] = r[j];
+  }
+  __syncthreads();
+  if (ranked) {
+    // sort (and fold) the sub-buckets of more than one record, each by the
+    // thread that holds its counts: about one per thread, of two records
+    u32 todo = 0;  // bit 4 j + i: count i of word j is above 1
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const u32 gt = __vcmpgtu4(s_cnt[tid * 8 + j], 0x01010101u) & 0x08040201u;
+      todo |= ((gt | (gt >> 8) | (gt >> 16) | (gt >> 24)) & 0xFu) << (4 * j);
+    }
+    while (todo) {
+      const int i = __ffs(todo) - 1, sh = 8 * (i & 3);
+      todo &= todo - 1u;
+      const u32 c4 = s_cnt[tid * 8 + (i >> 2)];
+      const u32 lo = s_base[tid * 8 + (i >> 2)] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
+      const u32 k = (c4 >> sh) & 0xFFu;
+      const ulonglong2 e0 = s_r[lo], e1 = s_r[lo + 1];
+      if (k == 2 && (!FOLD || ((e0.x ^ e1.x) >> ib) != 0)) {  // nearly always
+        if (e1.x < e0.x) {
+          s_r[lo] = e1;
+          s_r[lo + 1] = e0;
+        }
+        if (FOLD && skip_zero_heads && (__longlong_as_double((long long)e0.y) == 0.0 ||
+                                        __longlong_as_double((long long)e1.y) == 0.0))
+          fold_sub_bucket<FOLD>(s_r + lo, 2, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
+      } else {
+        fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
+      }
+    }
+  } else {
+    bucket_merge_sort<G>(s_r);
+    if (FOLD) {
+      for (u32 p = tid; p < cnt; p += BT) {
+        const u64 low = s_r[p].x >> ib;
+        bool kept = false;
+        if (p == 0 || (s_r[p - 1].x >> ib) != low) {  // the first of its run
+          double sum = __longlong_as_double((long long)s_r[p].y);
+          bool anynz = sum != 0.0;
+          u32 q = p + 1;
+          for (; q < cnt && (s_r[q].x >> ib) == low; ++q) {
+            const double y = __longlong_as_double((long long)s_r[q].y);
+            sum += y;
+            anynz |= y != 0.0;
+          }
+          if (q > p + 1) s_r[p].y = (u64)__double_as_longlong(sum);  // (nobody else reads a head's value)
+          kept = !skip_zero_heads || anynz || start + p == 0;
+        }
+        if (!kept) atomicAnd(&s_kept[p >> 5], ~(1u << (p & 31)));
+      }
+    }
+  }
+  __syncthreads();
+  const u64 prefix = (u64)b << shift;
+  if (!FOLD) {
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u32 p = j * BT + tid;
+      if (p < cnt) {
+        const ulonglong2 e = s_r[p];
+        __stcs(out_k + start + p, prefix | (e.x >> ib));
+        __stcs(out_v + start + p, __longlong_as_double((long long)e.y));
+      }
+    }
+    return;
+  }
+  // ---- warp 0: kept positions before every group of 32; output offset by
+  // decoupled look-back over buckets
+  if (warp == 0) {
+    constexpr int R = (G::kGroups + 31) / 32;
+    u32 total = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int x = r * 32 + lane;
+      const u32 k = x < G::kGroups ? __popc(s_kept[x]) : 0u;
+      u32 inc = k;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (x < G::kGroups) s_pre[x] = total + inc - k;
+      total += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0)
+      *reinterpret_cast<volatile unsigned long long*>(&c.status[b]) = (b == 0 ? kFlagPre : kFlagAgg) | total;
+    unsigned long long off = 0;
+    if (b != 0) {
+      int base = (int)b - 1;
+      u32 spins = 0;
+      while (base >= 0) {
+        const int p = base - lane;
+        const unsigned long long wv =
+            p >= 0 ? *reinterpret_cast<const volatile unsigned long long*>(&c.status[p]) : kFlagPre;
+        const unsigned long long f = wv & kFlagMask;
+        const u32 notready = __ballot_sync(0xffffffffu, f == 0);
+        const u32 pre = __ballot_sync(0xffffffffu, f == kFlagPre);
+        const int first_nr = notready ? __ffs(notready) - 1 : 32;
+        const int first_pre = pre ? __ffs(pre) - 1 : 32;
+        const int take = first_pre < first_nr ? first_pre + 1 : first_nr;
+        unsigned long long x = lane < take ? (wv & kValMask) : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        off += x;
+        if (first_pre < first_nr) break;
+        base -= first_nr;
+        if (first_nr < 32 && ++spins > spin_limit()) {
+          latch_error(kErrReduceLookback);
+          break;
+        }
+      }
+      if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&c.status[b]) = kFlagPre | (off + total);
+    }
+    if (lane == 0) {
+      *reinterpret_cast<unsigned long long*>(&s_misc[2]) = off;
+      if (b == (1u << T) - 1u) *d_nout = off + total;
+    }
+  }
+  __syncthreads();
+  const unsigned long long off = *reinterpret_cast<const unsigned long long*>(&s_misc[2]);
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 m = s_kept[j * W + warp];
+    if (m & (1u << lane)) {
+      const ulonglong2 e = s_r[j * BT + tid];
+      const u64 o = off + s_pre[j * W + warp] + __popc(m & ((1u << lane) - 1u));
+      __stcs(out_k + o, prefix | (e.x >> ib));
+      __stcs(out_v + o, __longlong_as_double((long long)e.y));
+    }
+  }
+}
+
+template <bool FIRST>
+int launch_partition(const MsdPlan& p, const PairSource& src, const ulonglong2* in, ulonglong2* out, u32 tiles,
+                     int dshift, int dbits, int nseg, const MsdCtrl& c, cudaStream_t s) {
+  using P = PartShape<kPartThreads, kPartItems, kPartBlocks>;
+  const bool digits = FIRST && p.key_bits + p.ib > 64;
+  auto kern = digits ? partition_kernel<P, FIRST, FIRST> : partition_kernel<P, FIRST, false>;
+  const size_t sh = P::smem + (digits ? P::kTile : 0);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  ProfScope prof("sort_partition", s);
+  kern<<<tiles, P::kThreads, sh, s>>>(src, in, out, p.n, p.ib, dshift, (1u << dbits) - 1u, nseg, p.db, c);
+  count_launch();
+  return launch_status();
+}
+
+template <class G>
+int launch_bucket_sort(const MsdPlan& p, const ulonglong2* rec, const MsdCtrl& c, const MsdFold* fold,
+                       u64* out_k, double* out_v, cudaStream_t s) {
+  auto kern = fold ? bucket_sort_kernel<G, true> : bucket_sort_kernel<G, false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  ProfScope prof(fold ? "bucket_sort_collect" : "bucket_sort", s);
+  kern<<<1u << p.T, G::kBT, G::smem, s>>>(rec, c, p.T, p.shift, p.ib, fold ? fold->skip_zero_heads : 0, out_k,
+                                          out_v, fold ? fold->d_nout : nullptr);
+  count_launch();
+  return launch_status();
+}
+
+// Keeps the bit-field moves that reach bits >= shift (pow2 re-keys).
+void top_fields(RekeyParams* r, int shift) {
+  if (r->order <= 1 || !r->pow2) return;
+  int m = 0;
+  for (int i = 0; i < r->order; ++i) {
+    const u32 f = r->field[i];
+    if ((int)((f >> 8) & 63u) + (int)((f >> 16) & 63u) > shift) r->field[m++] = f;
+  }
+  while (m < 2) r->field[m++] = 0;  // (moves nothing; order 1 would mean no re-key)
+  r->order = m;
+}
+
+}  // namespace
+
+MsdPlan make_msd_plan(size_t n, u64 max_key) {
+  MsdPlan p;
+  p.n = (u32)n;
+  p.key_bits = key_bits_for(max_key);
+  if (n < (1u << 20) || n >= (1u << 30) || getenv("LNT_NO_BUCKETS")) return p;
+  const char* force = getenv("LNT_BUCKET_SMALL");
+  int bestT = 99;
+  for (int large = 0; large < 2; ++large) {
+    if (force && (atoi(force) != 0) == (large != 0)) continue;
+    // the widest buckets whose expected size (uniform keys) stays below the limit
+    const double per_key = (double)n / (double)max_key, lim = large ? kAvgLarge : kAvgSmall;
+    if (per_key > lim) continue;
+    int shift = 0;
+    while (shift < p.key_bits - 1 && per_key * (double)(2ull << shift) <= lim) ++shift;
+    const int T = p.key_bits - shift;
+    if (T > kMaxT) continue;
+    if (bestT == 99 || (bestT > 8 && T <= 8)) {
+      bestT = T;
+      p.large = large != 0;
+      p.shift = shift;
+    }
+  }
+  if (bestT == 99) return p;
+  p.T = bestT;
+  p.passes = p.T <= 8 ? 1 : 2;
+  p.db = p.passes == 1 ? p.T : (p.T + 1) / 2;
+  while ((1ull << p.ib) < n) ++p.ib;
+  if (p.key_bits + p.ib - (p.passes == 1 ? p.T : p.T - p.db) > 64) return p;  // the word would not fit
+  const size_t nb = (size_t)1 << p.T;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += align_up(bytes, 256);
+    return o;
+  };
+  p.off_counts = take(nb * 4);
+  p.off_misc = take(256);
+  p.off_status = take(nb * 8);
+  p.zero_bytes = off;
+  p.off_start = take((nb + 1) * 4);
+  p.off_cur1 = take(kMaxDigits * 4);
+  p.off_cur2 = take(nb * 4 + kMaxDigits * 4);
+  p.off_segtile = take((kMaxDigits + 1) * 4);
+  p.ctrl_bytes = off;
+  p.ok = true;
+  return p;
+}
+
+int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void* ctrl, const MsdFold* fold, u64* out_k, double* out_v, u32* gate, cudaStream_t s) {
+  unsigned char* w = static_cast<unsigned char*>(ctrl);
+  MsdCtrl c;
+  c.counts = reinterpret_cast<u32*>(w + p.off_counts);
+  c.start = reinterpret_cast<u32*>(w + p.off_start);
+  c.cur1 = reinterpret_cast<u32*>(w + p.off_cur1);
+  c.cur2 = reinterpret_cast<u32*>(w + p.off_cur2);
+  c.segtile = reinterpret_cast<u32*>(w + p.off_segtile);
+  c.misc = reinterpret_cast<u32*>(w + p.off_misc);
+  c.status = reinterpret_cast<unsigned long long*>(w + p.off_status);
+  c.gate = gate;
+  if (cudaMemsetAsync(ctrl, 0, p.zero_bytes, s) != cudaSuccess) return LNT_DEVICE_ERROR;
+  const u32 cap = p.large ? (u32)GeomLarge::kCap : (u32)GeomSmall::kCap;
+  {
+    const size_t sh = std::max<size_t>(((size_t)1 << p.T) * 2, 4);  // 16-bit fields
+    if (cudaFuncSetAttribute(msd_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
+      return LNT_DEVICE_ERROR;
+    const u32 want = (p.n + kHistThreads * 8 - 1) / (kHistThreads * 8);
+    ProfScope prof("sort_hist", s);
+    // the buckets need only the top key bits: with power-of-two extents, only
+    // the modes that reach them are moved
+    PairSource top = src;
+    top_fields(&top.ra, p.shift);
+    top_fields(&top.rb, p.shift);
+    // (with one pass the cursors are the bucket starts: every bucket is its own segment)
+    msd_hist_kernel<<<std::min(want, (u32)sm_count() * 2), kHistThreads, sh, s>>>(
+        top, p.n, p.T, p.passes == 1 ? 0 : p.db, p.shift, cap, c);
+    count_launch();
+  }
+  ulonglong2* rx = static_cast<ulonglong2*>(x);
+  ulonglong2* ry = static_cast<ulonglong2*>(y);
+  {
+    const int dbits = p.passes == 1 ? p.T : p.T - p.db;  // this pass's digit: the top bits
+    const int st = launch_partition<true>(p, src, nullptr, p.passes == 1 ? ry : rx, (p.n + kPartTile - 1) / kPartTile,
+                                          p.key_bits - dbits, dbits, 0, c, s);
+    if (st != LNT_OK) return st;
+  }
+  if (p.passes == 2) {
+    const int nseg = 1 << (p.T - p.db);
+    const int st = launch_partition<false>(p, src, rx, ry, (p.n + kPartTile - 1) / kPartTile + nseg, p.ib + p.shift,
+                                           p.db, nseg, c, s);
+    if (st != LNT_OK) return st;
+  }
+  return p.large ? launch_bucket_sort<GeomLarge>(p, ry, c, fold, out_k, out_v, s)
+                 : launch_bucket_sort<GeomSmall>(p, ry, c, fold, out_k, out_v, s);
+}
+
+}  // namespace lnt

@@ -17,7 +17,7 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "lnt_sort.cuh"
+#include "lnt_msd.cuh"
 
 namespace lnt {
 namespace {
@@ -409,15 +409,17 @@ using namespace lnt;
 namespace {
 struct SortReduceLayout {
   SortPlan plan;
+  MsdPlan msd;
   size_t off_ctrl, off_k0, off_v0, off_k1, off_v1, off_coll, off_gate, total;
 };
 
 SortReduceLayout sort_reduce_layout(size_t n, u64 max_key) {
   SortReduceLayout L;
   L.plan = make_sort_plan(n, max_key);
+  L.msd = make_msd_plan(n, max_key);
   size_t off = 0;
   L.off_ctrl = off;
-  off += align_up(std::max(L.plan.ctrl_bytes, bucket_ctrl_bytes(n)), 256);
+  off += align_up(std::max(L.plan.ctrl_bytes, L.msd.ctrl_bytes), 256);
   L.off_k0 = off;
   off += align_up(n * 8, 256);
   L.off_v0 = off;
@@ -503,15 +505,14 @@ int lnt_sort_reduce(const uint64_t* a_keys, const double* a_vals, size_t na, con
   double* v0 = reinterpret_cast<double*>(w + L.off_v0);
   u64* k1 = reinterpret_cast<u64*>(w + L.off_k1);
   double* v1 = reinterpret_cast<double*>(w + L.off_v1);
-  const int key_bits = key_bits_for(max_key);
-  // Wide keys, many pairs: the bucketed path, whose histogram decides on the
-  // device whether it can finish (every bucket fits a CTA); the LSD path is
+  // The bucketed path where it applies; its histogram decides on the device
+  // whether it can finish (every bucket fits a CTA), and the LSD path is
   // enqueued behind it gated on the opposite answer.  Nothing waits on the host.
   const u32* gate = nullptr;
-  if (bucket_path_applies(n, key_bits) && !getenv("LNT_NO_BUCKETS")) {
+  if (L.msd.ok) {
     u32* g = reinterpret_cast<u32*>(w + L.off_gate);
-    st = run_bucketed_sort_reduce(src, (u32)n, key_bits, skip_zero_heads, k0, v0, k1, v1, w + L.off_ctrl,
-                                  (u64*)keys_out, vals_out, (u64*)d_nout, g, s);
+    const MsdFold fold{skip_zero_heads, (u64*)d_nout};
+    st = run_msd_sort(L.msd, src, k1, k0, w + L.off_ctrl, &fold, (u64*)keys_out, vals_out, g, s);
     if (st != LNT_OK) return st;
     gate = g;
   }

@@ -516,48 +516,6 @@ int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, d
 
 namespace lnt {
 
-namespace {
-template <int THREADS, int ITEMS, int W, int BITS = 8>
-int launch_pass8(const PairSource& src, bool first, u64* out_k, double* out_v, u32 n, u32 shift, u32 mask,
-                 const u32* bstart, u32* status, u32* tile_counter, cudaStream_t s) {
-  using Sh = OnesweepShape<BITS, THREADS, ITEMS>;
-  static_assert(Sh::TILE >= kOnesweepPassTile, "the look-back array is sized for kOnesweepPassTile-pair tiles");
-  constexpr size_t sh = Sh::smem;
-  auto k = first ? onesweep_kernel<BITS, THREADS, ITEMS, W, true> : onesweep_kernel<BITS, THREADS, ITEMS, W, false>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
-    return LNT_DEVICE_ERROR;
-  const u32 ntiles = (n + Sh::TILE - 1) / Sh::TILE;
-  ProfScope prof("sort_onesweep", s);
-  k<<<ntiles, THREADS, sh, s>>>(src, out_k, out_v, n, shift, mask, bstart, status, tile_counter);
-  count_launch();
-  return launch_status();
-}
-}  // namespace
-
-// Shape of the bucketed path's digit pass: 0 (256 threads x 16 keys, window 16), 1 (window 32),
-// 2 (512 x 8), 3 (384 x 12); the tuned choice, or LNT_PASS8_VARIANT from the environment.
-int run_onesweep_pass8(const PairSource& src, bool first, u64* out_k, double* out_v, u32 n, u32 shift, u32 mask,
-                       const u32* bstart, u32* status, u32* tile_counter, cudaStream_t s) {
-  int v = kTunedPass8Variant;
-  if (const char* e = getenv("LNT_PASS8_VARIANT")) v = atoi(e);
-  switch (v) {
-    case 1:
-      return launch_pass8<256, 16, 32>(src, first, out_k, out_v, n, shift, mask, bstart, status, tile_counter, s);
-    case 2:
-      return launch_pass8<512, 8, 16>(src, first, out_k, out_v, n, shift, mask, bstart, status, tile_counter, s);
-    case 3:
-      return launch_pass8<384, 12, 16>(src, first, out_k, out_v, n, shift, mask, bstart, status, tile_counter, s);
-    default:
-      // a 7-bit digit (the first pass of 2^15 buckets) on a 128-digit kernel:
-      // seven ballots per key and half the counters, scans and look-back
-      // (1.49 -> 1.42 ms for that pass over 2^27 pairs)
-      if (mask == 0x7Fu)
-        return launch_pass8<256, 16, 16, 7>(src, first, out_k, out_v, n, shift, mask, bstart, status, tile_counter,
-                                            s);
-      return launch_pass8<256, 16, 16>(src, first, out_k, out_v, n, shift, mask, bstart, status, tile_counter, s);
-  }
-}
-
 int sort_variant_count() { return kNumVariants; }
 const SortVariant& sort_variant(int i) { return kVariants[i]; }
 

@@ -1,0 +1,56 @@
+"""GPU: the bucketed sort (partition passes + one CTA per bucket) against the
+oracle, at the sizes and key distributions where it can go wrong: one and two
+partition passes, tile remainders, either bucket geometry, words that lose
+their top key bits, repeated keys inside and beyond a sub-bucket, key-ordered
+input, and keys concentrated on the top of the key range.  Every path
+restores the input order of equal keys."""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import rel_ok
+from test_gpu_sort import to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch as t
+    return t
+
+# (pairs, max_key): 1 or 2 passes, odd remainders, non-power-of-two ranges
+SIZES = [(1 << 20, 1 << 36), ((1 << 20) + 4097, 3 * 10 ** 6), (3 * 10 ** 6 + 1, 7 * 10 ** 8), (1 << 22, 1 << 50),
+         (1500001, (1 << 51) + 12345)]
+
+
+def _keys(rng, n, max_key, kind):
+    if kind == "uniform":
+        return rng.integers(0, max_key, n, dtype=np.uint64)
+    if kind == "sorted":
+        return np.sort(rng.integers(0, max_key, n, dtype=np.uint64))
+    if kind == "repeated":  # up to a few hundred of a key, never more than a bucket holds
+        k = rng.integers(0, max_key, n // 100, dtype=np.uint64)
+        return k[rng.integers(0, k.size, n)]
+    # the upper half of the range only: buckets twice as full as uniform ones
+    return rng.integers(max_key // 2, max_key, n, dtype=np.uint64)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "sorted", "repeated", "upper"])
+@pytest.mark.parametrize("n,max_key", SIZES)
+def test_sort_reduce_bucketed(cuda, torch, n, max_key, kind):
+    rng = np.random.default_rng(n + len(kind))
+    keys = _keys(rng, n, max_key, kind)
+    vals = rng.uniform(-1, 1, n)
+    vals[rng.random(n) < 0.2] = 0.0
+    cut = n // 3
+    k, v = cuda.sort_reduce(to_dev(keys[:cut], torch), to_dev(vals[:cut], torch), to_dev(keys[cut:], torch),
+                            to_dev(vals[cut:], torch), max_key=max_key, b_scale=-1.0)
+    signed = np.concatenate([vals[:cut], -vals[cut:]])
+    sk, sv = oracle.sort_pairs(keys, signed)
+    ek, ev, ea = oracle.collect_duplicates(sk, sv, with_abs=True)
+    np.testing.assert_array_equal(to_host(k, np.uint64), ek)
+    # runs are added in input order; only where a bucket overflowed and the
+    # general path ran are runs added tile by tile
+    assert rel_ok(to_host(v), ev, ea)
+    assert cuda.device_status() == 0
