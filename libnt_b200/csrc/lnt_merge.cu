@@ -26,7 +26,7 @@
 // Traffic: 16 B read per input pair + 16 B written per output pair.
 #include <algorithm>
 
-#include "lnt_sort.cuh"
+#include "lnt_msd.cuh"
 
 namespace lnt {
 namespace {
@@ -264,19 +264,19 @@ using namespace lnt;
 
 namespace {
 struct PermuteSortLayout {
-  SortPlan plan;
-  size_t off_ctrl, off_tk, off_tv, total;
+  PairSort sort;
+  size_t off_ctrl, off_a, off_b, total;
 };
 PermuteSortLayout permute_sort_layout(size_t n, u64 max_key) {
   PermuteSortLayout L;
-  L.plan = make_sort_plan(n, max_key);
+  L.sort = make_pair_sort(n, max_key);
   size_t off = 0;
   L.off_ctrl = off;
-  off += align_up(L.plan.ctrl_bytes, 256);
-  L.off_tk = off;
-  off += align_up(n * 8, 256);
-  L.off_tv = off;
-  off += align_up(n * 8, 256);
+  off += align_up(L.sort.ctrl_bytes, 256);
+  L.off_a = off;
+  off += L.sort.a_bytes;
+  L.off_b = off;
+  off += L.sort.b_bytes;
   L.total = off;
   return L;
 }
@@ -339,8 +339,8 @@ int lnt_permute_sort(const uint64_t* keys_in, const double* vals_in, size_t n, c
   int st = make_rekey_params(rekey, &src.ra);
   if (st != LNT_OK) return st;
   unsigned char* w = static_cast<unsigned char*>(workspace);
-  return run_sort(L.plan, src, (u64*)keys_out, vals_out, reinterpret_cast<u64*>(w + L.off_tk),
-                  reinterpret_cast<double*>(w + L.off_tv), w + L.off_ctrl, as_stream(stream));
+  return run_pair_sort(L.sort, src, (u64*)keys_out, vals_out, w + L.off_a, w + L.off_b, w + L.off_ctrl,
+                       as_stream(stream));
 }
 
 }  // extern "C"

@@ -37,6 +37,10 @@ namespace {
 
 constexpr int kHistThreads = 1024;
 constexpr int kMaxT = 15;
+// Smallest sort taken.  Down to 2048 pairs the bucketed path with the skipped
+// fallback behind it takes 18-21 us against 33-57 us for the digit passes (20
+// to 50 key bits); below, the histogram and one CTA are all there is to gain.
+constexpr size_t kMinPairs = 2048;
 constexpr int kMaxDigits = 256;
 // Partition tile: 256 threads x 8 records, four CTAs per SM at 64 registers.
 // What matters is that nothing spills: 12 records per thread ran the same
@@ -77,9 +81,9 @@ struct MsdCtrl {
   u32* cur1;      // first pass cursors (up to 256)
   u32* cur2;      // second pass cursors (2^T)
   u32* segtile;   // second pass: first tile of every segment (up to 257)
-  u32* misc;      // [0] histogram CTAs done, [1] bucket counter
+  u32* misc;      // [0] histogram CTAs done, [1] bucket counter, [2] a key has bits above the sorted ones
   unsigned long long* status;  // 2^T look-back words (FOLD)
-  u32* gate;      // 0: every bucket fits a CTA, 1: take the LSD path
+  u32* gate;      // 0: every bucket fits a CTA (and no key loses bits), 1: take the LSD path
 };
 
 // Bucket counts in shared memory as 16-bit fields (two per word, 64 KB at
@@ -160,7 +164,7 @@ __device__ __forceinline__ void source_keys(const PairSource& s, u32 base, u32 s
 }
 
 __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSource src, u32 n, int T, int db,
-                                                                   int shift, u32 cap, MsdCtrl c) {
+                                                                   int shift, int key_bits, u32 cap, MsdCtrl c) {
   extern __shared__ u32 sh[];  // 2^T 16-bit fields
   __shared__ bool s_last;
   __shared__ u32 s_w[kHistThreads / 32], s_mx[kHistThreads / 32];
@@ -169,6 +173,7 @@ __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSou
   for (int i = tid; i < nw; i += kHistThreads) sh[i] = 0;
   __syncthreads();
   const u32 bmask = (u32)(nb - 1);
+  u64 any = 0;
   constexpr int U = 4;
   for (u64 base = (u64)blockIdx.x * (kHistThreads * U); base < n; base += (u64)gridDim.x * (kHistThreads * U)) {
     const u32 end = (u32)min((u64)n, base + kHistThreads * U);
@@ -176,8 +181,13 @@ __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSou
     source_keys<U>(src, (u32)base, kHistThreads, end, k);
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if ((u32)base + u * kHistThreads + tid < end) count16(sh, (u32)(k[u] >> shift) & bmask, c);
+      if ((u32)base + u * kHistThreads + tid < end) {
+        count16(sh, (u32)(k[u] >> shift) & bmask, c);
+        any |= k[u];
+      }
   }
+  // bits above the sorted ones (a key >= max_key): the records would lose them
+  if (key_bits < 64 && (any >> key_bits) != 0) atomicOr(&c.misc[2], 1u);
   __syncthreads();
   for (int b = tid; b < nb; b += kHistThreads) {
     const u32 v = (sh[b >> 1] >> (16 * (b & 1))) & 0xFFFFu;
@@ -221,10 +231,11 @@ __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSou
       run += __ldcg(&c.counts[b]);
     }
   }
+  if (tid >= 1 && tid < kGateWords) c.gate[tid] = 0;
   if (tid == 0) {
     u32 m = 0;
     for (int w = 0; w < kHistThreads / 32; ++w) m = max(m, s_mx[w]);
-    *c.gate = m > cap ? 1u : 0u;
+    c.gate[0] = m > cap || __ldcg(&c.misc[2]) != 0u ? 1u : 0u;
     c.start[nb] = n;
   }
   __threadfence_block();
@@ -776,7 +787,7 @@ MsdPlan make_msd_plan(size_t n, u64 max_key) {
   MsdPlan p;
   p.n = (u32)n;
   p.key_bits = key_bits_for(max_key);
-  if (n < (1u << 20) || n >= (1u << 30) || getenv("LNT_NO_BUCKETS")) return p;
+  if (n < kMinPairs || n >= (1u << 30) || getenv("LNT_NO_BUCKETS")) return p;
   const char* force = getenv("LNT_BUCKET_SMALL");
   int bestT = 99;
   for (int large = 0; large < 2; ++large) {
@@ -799,7 +810,10 @@ MsdPlan make_msd_plan(size_t n, u64 max_key) {
   p.passes = p.T <= 8 ? 1 : 2;
   p.db = p.passes == 1 ? p.T : (p.T + 1) / 2;
   while ((1ull << p.ib) < n) ++p.ib;
-  if (p.key_bits + p.ib - (p.passes == 1 ? p.T : p.T - p.db) > 64) return p;  // the word would not fit
+  // the word must hold what is left of the key after the first pass; a wider
+  // first digit (at most 8 bits) leaves less
+  if (p.passes == 2 && p.key_bits + p.ib - (p.T - p.db) > 64) p.db = p.T - 8;
+  if (p.key_bits + p.ib - (p.passes == 1 ? p.T : p.T - p.db) > 64) return p;
   const size_t nb = (size_t)1 << p.T;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -837,7 +851,7 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
     const size_t sh = std::max<size_t>(((size_t)1 << p.T) * 2, 4);  // 16-bit fields
     if (cudaFuncSetAttribute(msd_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
       return LNT_DEVICE_ERROR;
-    const u32 want = (p.n + kHistThreads * 8 - 1) / (kHistThreads * 8);
+    const u32 want = (p.n + kHistThreads * 4 - 1) / (kHistThreads * 4);
     ProfScope prof("sort_hist", s);
     // the buckets need only the top key bits: with power-of-two extents, only
     // the modes that reach them are moved
@@ -846,7 +860,7 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
     top_fields(&top.rb, p.shift);
     // (with one pass the cursors are the bucket starts: every bucket is its own segment)
     msd_hist_kernel<<<std::min(want, (u32)sm_count() * 2), kHistThreads, sh, s>>>(
-        top, p.n, p.T, p.passes == 1 ? 0 : p.db, p.shift, cap, c);
+        top, p.n, p.T, p.passes == 1 ? 0 : p.db, p.shift, p.key_bits, cap, c);
     count_launch();
   }
   ulonglong2* rx = static_cast<ulonglong2*>(x);
@@ -865,6 +879,29 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
   }
   return p.large ? launch_bucket_sort<GeomLarge>(p, ry, c, fold, out_k, out_v, s)
                  : launch_bucket_sort<GeomSmall>(p, ry, c, fold, out_k, out_v, s);
+}
+
+PairSort make_pair_sort(size_t n, u64 max_key) {
+  PairSort p;
+  p.msd = make_msd_plan(n, max_key);
+  p.lsd = make_sort_plan(n, max_key, p.msd.ok);
+  p.ctrl_bytes = align_up(std::max(p.lsd.ctrl_bytes, p.msd.ctrl_bytes), 256) + 256;
+  p.a_bytes = 2 * align_up(n * 8, 256);
+  p.b_bytes = p.msd.ok && p.msd.passes == 2 ? p.a_bytes : 0;
+  return p;
+}
+
+int run_pair_sort(const PairSort& p, const PairSource& src, u64* out_k, double* out_v, void* a, void* b, void* ctrl,
+                  cudaStream_t s) {
+  u32* gate = nullptr;
+  if (p.msd.ok) {
+    gate = reinterpret_cast<u32*>(static_cast<unsigned char*>(ctrl) + p.ctrl_bytes - 256);
+    const int st = run_msd_sort(p.msd, src, b, a, ctrl, nullptr, out_k, out_v, gate, s);
+    if (st != LNT_OK) return st;
+  }
+  u64* ak = static_cast<u64*>(a);
+  double* av = reinterpret_cast<double*>(static_cast<unsigned char*>(a) + p.a_bytes / 2);
+  return run_sort(p.lsd, gated_source(src, gate, 1), out_k, out_v, ak, av, ctrl, s);
 }
 
 }  // namespace lnt

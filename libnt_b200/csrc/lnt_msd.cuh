@@ -29,7 +29,8 @@ MsdPlan make_msd_plan(size_t n, u64 max_key);
 // when every bucket fits a CTA (the remaining kernels run), 1 when one does
 // not (they return at once; the caller's LSD path, gated on 1, runs instead).
 // x, y: scratch of plan.n 16-byte records each, 16-byte aligned (x is used when
-// plan.passes == 2 only).  Nothing waits on the host.
+// plan.passes == 2 only).  gate: a gate block (kGateWords words).  Nothing
+// waits on the host.
 struct MsdFold {
   int skip_zero_heads;  // as in lnt_collect_duplicates
   u64* d_nout;
@@ -37,5 +38,18 @@ struct MsdFold {
 // fold == nullptr: plain stable sort.
 int run_msd_sort(const MsdPlan& plan, const PairSource& src, void* x, void* y, void* ctrl, const MsdFold* fold,
                  u64* out_k, double* out_v, u32* gate, cudaStream_t s);
+
+// A stable sort of n pairs by the bucketed path where it applies, with the LSD
+// path behind it.
+struct PairSort {
+  SortPlan lsd;
+  MsdPlan msd;
+  size_t ctrl_bytes = 0;  // control block: either path's, then the gate word
+  size_t a_bytes = 0, b_bytes = 0;  // scratch (b: 0 when not needed)
+};
+PairSort make_pair_sort(size_t n, u64 max_key);
+// out must not overlap the source; a, b, ctrl: 256-byte aligned.
+int run_pair_sort(const PairSort& p, const PairSource& src, u64* out_k, double* out_v, void* a, void* b, void* ctrl,
+                  cudaStream_t s);
 
 }  // namespace lnt

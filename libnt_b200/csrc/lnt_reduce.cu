@@ -415,8 +415,8 @@ struct SortReduceLayout {
 
 SortReduceLayout sort_reduce_layout(size_t n, u64 max_key) {
   SortReduceLayout L;
-  L.plan = make_sort_plan(n, max_key);
   L.msd = make_msd_plan(n, max_key);
+  L.plan = make_sort_plan(n, max_key, L.msd.ok);
   size_t off = 0;
   L.off_ctrl = off;
   off += align_up(std::max(L.plan.ctrl_bytes, L.msd.ctrl_bytes), 256);

@@ -8,7 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "lnt_sort.cuh"
+#include "lnt_msd.cuh"
 
 namespace lnt {
 namespace {
@@ -44,20 +44,17 @@ __device__ __forceinline__ double load_val(const PairSource& s, size_t i) {
 // ---------------------------------------------------------------------------
 // Histogram of every pass's digits in one read of the keys.
 // ---------------------------------------------------------------------------
+// Block `block` of `nblocks` (kThreads threads); sh_hist: passes * RADIX words.
 template <int BITS>
-__global__ void __launch_bounds__(kThreads) hist_kernel(const PairSource src, u32 n, int passes,
-                                                        int key_bits, u32* __restrict__ ghist,
-                                                        u32* __restrict__ bstart,
-                                                        u32* __restrict__ done) {
+__device__ __forceinline__ void hist_block(const PairSource& src, u32 n, int passes, int key_bits, u32* ghist,
+                                           u32* bstart, u32* done, u32* sh_hist, u32 block, u32 nblocks) {
   constexpr int RADIX = 1 << BITS;
-  extern __shared__ u32 sh_hist[];  // passes * RADIX
   __shared__ bool s_last;
-  if (gated_off(src.gate, src.gate_run)) return;
   for (int i = threadIdx.x; i < passes * RADIX; i += kThreads) sh_hist[i] = 0;
   __syncthreads();
-  const u32 stride = gridDim.x * kThreads;
+  const u32 stride = nblocks * kThreads;
   constexpr int U = 8;  // independent loads in flight per thread
-  u32 i = blockIdx.x * kThreads + threadIdx.x;
+  u32 i = block * kThreads + threadIdx.x;
   for (; i + (U - 1) * stride < n; i += U * stride) {
     u64 k[U];
 #pragma unroll
@@ -86,7 +83,7 @@ __global__ void __launch_bounds__(kThreads) hist_kernel(const PairSource src, u3
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
+  if (threadIdx.x == 0) s_last = (atomicAdd(done, 1u) == nblocks - 1);
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -122,6 +119,13 @@ __global__ void __launch_bounds__(kThreads) hist_kernel(const PairSource src, u3
     }
     __syncthreads();
   }
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(kThreads) hist_kernel(const PairSource src, u32 n, int passes, int key_bits,
+                                                        u32* ghist, u32* bstart, u32* done) {
+  extern __shared__ u32 sh_hist[];
+  hist_block<BITS>(src, n, passes, key_bits, ghist, bstart, done, sh_hist, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -165,22 +169,17 @@ __device__ __forceinline__ u32 match_digit(u32 d) {
   return peers;
 }
 
-// PERSIST: a grid smaller than the tile count whose CTAs take tiles until
-// none is left.  Tiles are taken in order and a CTA finishes its tile before
-// taking another, so every predecessor a look-back waits on belongs to a
-// running CTA.
-template <int BITS, int THREADS, int ITEMS, int W, bool FIRST, bool PERSIST = false>
-__global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>::MINB))
-    onesweep_kernel(const PairSource src, u64* __restrict__ out_k, double* __restrict__ out_v, u32 n, u32 shift,
-                    u32 mask, const u32* __restrict__ bstart, u32* __restrict__ status,
-                    u32* __restrict__ tile_counter) {
-  if (gated_off(src.gate, src.gate_run)) return;
+// One tile of a digit pass.  Tiles are handed out in order, so every
+// predecessor a look-back waits on belongs to a running CTA.
+template <int BITS, int THREADS, int ITEMS, int W, bool FIRST>
+__device__ __forceinline__ void onesweep_tile(const PairSource& src, u64* out_k, double* out_v, u32 n, u32 shift,
+                                              u32 mask, const u32* bstart, u32* status, u32 tile,
+                                              unsigned char* smem) {
   using S = OnesweepShape<BITS, THREADS, ITEMS>;
   constexpr int RADIX = S::RADIX;
   constexpr int WARPS = S::WARPS;
   constexpr int TILE = S::TILE;
   constexpr int DPT = S::DPT;
-  extern __shared__ __align__(16) unsigned char smem[];
   u64* s_x = reinterpret_cast<u64*>(smem);               // TILE: tile in digit order
   double* s_v = reinterpret_cast<double*>(s_x + TILE);   // TILE: values in input order
   u32* s_whist = reinterpret_cast<u32*>(s_v + TILE);     // WARPS * RADIX
@@ -189,13 +188,8 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
   u32* s_misc = s_glob + RADIX;                          // 16
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const u32 ntiles = (n + TILE - 1) / TILE;
-  for (;;) {
-  if (tid == 0) s_misc[0] = atomicAdd(tile_counter, 1u);
   for (int i = tid; i < WARPS * RADIX; i += THREADS) s_whist[i] = 0;
   __syncthreads();
-  const u32 tile = s_misc[0];
-  if (PERSIST && tile >= ntiles) break;
   const size_t tile_base = (size_t)tile * TILE;
   const u32 tile_n = (u32)min((size_t)TILE, (size_t)n - tile_base);
   const u32 warp_base = warp * ITEMS * 32;
@@ -234,7 +228,7 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
     if (d < RADIX) {
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) c += s_whist[w * RADIX + d];
-      const u32 word = tile == 0 ? (kFlagPre | (bstart[d] + c)) : (kFlagAgg | c);
+      const u32 word = tile == 0 ? (kFlagPre | (__ldcg(bstart + d) + c)) : (kFlagAgg | c);
       st_volatile(&status[(size_t)tile * RADIX + d], word);
     }
     cnt[j] = c;
@@ -306,7 +300,7 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
 #pragma unroll
     for (int j = 0; j < DPT; ++j) {
       const int d = tid * DPT + j;
-      excl[j] = (tile == 0 && d < RADIX) ? bstart[d] : 0u;
+      excl[j] = (tile == 0 && d < RADIX) ? __ldcg(bstart + d) : 0u;
       p[j] = (int)tile - 1;
       done[j] = (d >= RADIX) || tile == 0;
     }
@@ -393,8 +387,105 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
     const u32 idx = j * THREADS + tid;
     if (idx < tile_n) __stcs(out_v + dst[j], reinterpret_cast<const double*>(s_x)[idx]);
   }
-  if (!PERSIST) break;
-  __syncthreads();  // shared memory is reused by the next tile
+}
+
+template <int BITS, int THREADS, int ITEMS, int W, bool FIRST>
+__global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>::MINB))
+    onesweep_kernel(const PairSource src, u64* __restrict__ out_k, double* __restrict__ out_v, u32 n, u32 shift,
+                    u32 mask, const u32* __restrict__ bstart, u32* __restrict__ status,
+                    u32* __restrict__ tile_counter) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ u32 s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+  __syncthreads();
+  onesweep_tile<BITS, THREADS, ITEMS, W, FIRST>(src, out_k, out_v, n, shift, mask, bstart, status, s_tile, smem);
+}
+
+// The whole sort in one launch, for the path behind a gate: it is nearly
+// always skipped, and a skipped launch costs 1.6 us in the stream (seven to
+// ten of them when every step was a kernel of its own).  CTAs take the tasks
+// (zero the control block, histogram, the tiles of every pass) in order from a
+// queue; a task waits until the step before is complete, whose tasks all
+// belong to running CTAs.  gate[1]: queue, gate[2 + step]: tasks done; zeroed
+// by whoever writes the gate.
+constexpr int kQBits = 8, kQItems = 16, kQWindow = 16;
+using QueueShape = OnesweepShape<kQBits, kThreads, kQItems>;
+
+__device__ __forceinline__ void queue_wait(const u32* done, u32 want) {
+  if (threadIdx.x == 0) {
+    u32 spins = 0;
+    while (ld_volatile(done) < want) {
+      __nanosleep(100);
+      if (++spins > spin_limit()) {
+        latch_error(kErrSortLookback);
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void queue_done(u32* done) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) atomicAdd(done, 1u);
+}
+
+__global__ void __launch_bounds__(kThreads, QueueShape::MINB)
+    lsd_queue_kernel(const PairSource src, const SortPlan plan, u64* buf0_k, double* buf0_v, u64* buf1_k,
+                     double* buf1_v, unsigned char* ctrl, u32* gate) {
+  if (gated_off(src.gate, src.gate_run)) return;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ u32 s_task;
+  constexpr int RADIX = 1 << kQBits;
+  constexpr size_t kZero = 1u << 16;  // bytes zeroed per task
+  const u32 nz = (u32)((plan.ctrl_bytes + kZero - 1) / kZero);
+  const u32 nh = min((plan.n + kThreads * 16 - 1) / (kThreads * 16), gridDim.x);
+  u32* ghist = reinterpret_cast<u32*>(ctrl + plan.off_ghist);
+  u32* bstart = reinterpret_cast<u32*>(ctrl + plan.off_bstart);
+  u32* status = reinterpret_cast<u32*>(ctrl + plan.off_status);
+  u32* counters = reinterpret_cast<u32*>(ctrl + plan.off_counters);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_task = atomicAdd(&gate[1], 1u);
+    __syncthreads();
+    u32 t = s_task;
+    if (t < nz) {
+      uint4* z = reinterpret_cast<uint4*>(ctrl + (size_t)t * kZero);
+      const size_t words = min(kZero, plan.ctrl_bytes - (size_t)t * kZero) / 16;
+      for (size_t i = threadIdx.x; i < words; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
+      queue_done(&gate[2]);
+      continue;
+    }
+    t -= nz;
+    if (t < nh) {
+      queue_wait(&gate[2], nz);
+      hist_block<kQBits>(src, plan.n, plan.passes, plan.key_bits, ghist, bstart, counters + plan.passes,
+                         reinterpret_cast<u32*>(smem), t, nh);
+      queue_done(&gate[3]);
+      continue;
+    }
+    t -= nh;
+    const int p = (int)(t / plan.ntiles);
+    if (p >= plan.passes) return;
+    queue_wait(&gate[3 + p], p == 0 ? nh : plan.ntiles);
+    const int which = (plan.passes - 1 - p) & 1, shift = p * kQBits;
+    const u32 mask = (1u << min(kQBits, plan.key_bits - shift)) - 1u;
+    u64* ok = which ? buf1_k : buf0_k;
+    double* ov = which ? buf1_v : buf0_v;
+    u32* st = status + (size_t)p * plan.ntiles * RADIX;
+    t -= (u32)p * plan.ntiles;
+    if (p == 0) {
+      onesweep_tile<kQBits, kThreads, kQItems, kQWindow, true>(src, ok, ov, plan.n, (u32)shift, mask, bstart, st, t,
+                                                               smem);
+    } else {
+      PairSource in = src;
+      in.ak = which ? buf0_k : buf1_k;
+      in.av = which ? buf0_v : buf1_v;
+      onesweep_tile<kQBits, kThreads, kQItems, kQWindow, false>(in, ok, ov, plan.n, (u32)shift, mask,
+                                                                bstart + p * RADIX, st, t, smem);
+    }
+    queue_done(&gate[4 + p]);
   }
 }
 
@@ -407,16 +498,6 @@ __global__ void copy_source_kernel(const PairSource src, u64* __restrict__ ok, d
     ok[i] = load_key<true>(src, i);
     ov[i] = load_val<true>(src, i);
   }
-}
-
-// Zeroes `words` 32-bit words (the gated form of the control block's memset).
-__global__ void zero_words_kernel(u32* __restrict__ p, size_t words, const u32* gate, u32 want) {
-  if (gated_off(gate, want)) return;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  uint4* p4 = reinterpret_cast<uint4*>(p);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words / 4; i += stride)
-    p4[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (size_t i = (words / 4) * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) p[i] = 0u;
 }
 
 #define LNT_SV_ENTRY(B, T, I, W) {B, T, I, W},
@@ -434,15 +515,7 @@ int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, d
   u32* bstart = reinterpret_cast<u32*>(c + plan.off_bstart);
   u32* status = reinterpret_cast<u32*>(c + plan.off_status);
   u32* counters = reinterpret_cast<u32*>(c + plan.off_counters);
-  const bool gated = src.gate != nullptr;
-  if (gated) {  // skipped with the rest of the sort when the gate is closed
-    const size_t words = plan.ctrl_bytes / 4;  // ctrl is 256-byte aligned, ctrl_bytes a multiple of 256
-    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((words / 4 + 255) / 256, (size_t)sm_count() * 4));
-    zero_words_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<u32*>(ctrl), words, src.gate, src.gate_run);
-    count_launch();
-  } else if (cudaMemsetAsync(ctrl, 0, plan.ctrl_bytes, s) != cudaSuccess) {
-    return LNT_DEVICE_ERROR;
-  }
+  if (cudaMemsetAsync(ctrl, 0, plan.ctrl_bytes, s) != cudaSuccess) return LNT_DEVICE_ERROR;
 
   // histogram of all passes
   {
@@ -451,7 +524,7 @@ int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, d
     if (sh > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     const int blocks =
         std::max(1, std::min((int)((plan.n + kThreads * 16 - 1) / (kThreads * 16)), sm_count() * 4));
-    ProfScope prof(src.gate ? "sort_hist_fallback" : "sort_hist", s);
+    ProfScope prof("sort_hist", s);
     kern<<<blocks, kThreads, sh, s>>>(src, plan.n, plan.passes, plan.key_bits, ghist, bstart,
                                       counters + plan.passes);
     count_launch();
@@ -462,18 +535,7 @@ int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, d
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   cudaFuncSetAttribute(onesweep_kernel<BITS, THREADS, ITEMS, W, false>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  u32 grid = plan.ntiles;
-  if (gated) {  // persistent grid: a closed gate then costs one wave of empty CTAs
-    cudaFuncSetAttribute(onesweep_kernel<BITS, THREADS, ITEMS, W, true, true>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    cudaFuncSetAttribute(onesweep_kernel<BITS, THREADS, ITEMS, W, false, true>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, onesweep_kernel<BITS, THREADS, ITEMS, W, false, true>,
-                                                      THREADS, sh) != cudaSuccess)
-      return LNT_DEVICE_ERROR;
-    grid = std::min(grid, (u32)(std::max(per_sm, 1) * sm_count()));
-  }
+  const u32 grid = plan.ntiles;
   const u64* in_k = nullptr;
   const double* in_v = nullptr;
   for (int p = 0; p < plan.passes; ++p) {
@@ -484,23 +546,13 @@ int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, d
     const int w = std::min(BITS, plan.key_bits - shift);
     const u32 mask = (1u << w) - 1u;
     u32* st = status + (size_t)p * plan.ntiles * RADIX;
-    ProfScope prof(gated ? "sort_onesweep_fallback" : "sort_onesweep", s);
-    if (p == 0) {
-      if (gated)
-        onesweep_kernel<BITS, THREADS, ITEMS, W, true, true><<<grid, THREADS, sh, s>>>(
-            src, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
-      else
-        onesweep_kernel<BITS, THREADS, ITEMS, W, true><<<grid, THREADS, sh, s>>>(
-            src, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
-    } else {
-      const PairSource ps = gated_source(plain_source(in_k, in_v, plan.n), src.gate, src.gate_run);
-      if (gated)
-        onesweep_kernel<BITS, THREADS, ITEMS, W, false, true><<<grid, THREADS, sh, s>>>(
-            ps, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
-      else
-        onesweep_kernel<BITS, THREADS, ITEMS, W, false><<<grid, THREADS, sh, s>>>(
-            ps, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
-    }
+    ProfScope prof("sort_onesweep", s);
+    if (p == 0)
+      onesweep_kernel<BITS, THREADS, ITEMS, W, true><<<grid, THREADS, sh, s>>>(
+          src, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
+    else
+      onesweep_kernel<BITS, THREADS, ITEMS, W, false><<<grid, THREADS, sh, s>>>(
+          plain_source(in_k, in_v, plan.n), ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX, st, counters + p);
     count_launch();
     in_k = ok;
     in_v = ov;
@@ -541,11 +593,11 @@ int choose_sort_variant(size_t n, int key_bits) {
   return best;
 }
 
-SortPlan make_sort_plan(size_t n, u64 max_key, int variant) {
+SortPlan make_sort_plan(size_t n, u64 max_key, bool gated) {
   SortPlan p;
   p.key_bits = key_bits_for(max_key);
-  p.variant = variant >= 0 && variant < kNumVariants ? variant : choose_sort_variant(n, p.key_bits);
-  const SortVariant& v = kVariants[p.variant];
+  p.variant = gated ? -1 : choose_sort_variant(n, p.key_bits);
+  const SortVariant v = gated ? SortVariant{kQBits, kThreads, kQItems, kQWindow} : kVariants[p.variant];
   p.bits = v.bits;
   p.passes = p.key_bits == 0 ? 0 : (p.key_bits + v.bits - 1) / v.bits;
   p.n = (u32)n;
@@ -575,6 +627,18 @@ int run_sort(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* b
     count_launch();
     return launch_status();
   }
+  if (plan.variant < 0) {  // behind a gate
+    constexpr size_t sh = QueueShape::smem;
+    static_assert(sh >= 8u * (1u << kQBits) * 4u, "the histogram of eight passes fits");
+    if (cudaFuncSetAttribute(lsd_queue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
+      return LNT_DEVICE_ERROR;
+    const u32 grid = std::min(plan.ntiles, (u32)(QueueShape::MINB * sm_count()));
+    ProfScope prof("sort_fallback", s);
+    lsd_queue_kernel<<<grid, kThreads, sh, s>>>(src, plan, buf0_k, buf0_v, buf1_k, buf1_v,
+                                                static_cast<unsigned char*>(ctrl), const_cast<u32*>(src.gate));
+    count_launch();
+    return launch_status();
+  }
   int i = 0;
 #define LNT_SV_CASE(B, T, I, W)                                                          \
   if (plan.variant == i) return run_sort_variant<B, T, I, W>(plan, src, buf0_k, buf0_v, \
@@ -590,24 +654,20 @@ int run_sort(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* b
 using namespace lnt;
 
 namespace {
-// Workspace of lnt_sort_pairs: [ctrl | tmp keys | tmp vals | tmp2 keys | tmp2 vals].
+// Workspace of lnt_sort_pairs: [ctrl | scratch pairs a | scratch pairs b].
 struct SortPairsLayout {
-  SortPlan plan;
-  size_t off_tk, off_tv, off_t2k, off_t2v, total;
+  PairSort sort;
+  size_t off_a, off_b, total;
 };
 
 SortPairsLayout sort_pairs_layout(size_t n, u64 max_key) {
   SortPairsLayout L;
-  L.plan = make_sort_plan(n, max_key);
-  size_t off = align_up(L.plan.ctrl_bytes, 256);
-  L.off_tk = off;
-  off += align_up(n * 8, 256);
-  L.off_tv = off;
-  off += align_up(n * 8, 256);
-  L.off_t2k = off;
-  off += align_up(n * 8, 256);
-  L.off_t2v = off;
-  off += align_up(n * 8, 256);
+  L.sort = make_pair_sort(n, max_key);
+  size_t off = align_up(L.sort.ctrl_bytes, 256);
+  L.off_a = off;
+  off += L.sort.a_bytes;
+  L.off_b = off;
+  off += L.sort.a_bytes;  // (an in-place LSD sort of an odd number of passes needs both)
   L.total = off;
   return L;
 }
@@ -644,26 +704,37 @@ int lnt_sort_pairs(const uint64_t* keys_in, const double* vals_in, uint64_t* key
   if ((uintptr_t)workspace % 256) return LNT_BAD_ARG;
   cudaStream_t s = as_stream(stream);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  u64* tk = reinterpret_cast<u64*>(ws + L.off_tk);
-  double* tv = reinterpret_cast<double*>(ws + L.off_tv);
   PairSource src = plain_source((const u64*)keys_in, vals_in, n);
   const bool inplace =
       (const void*)keys_in == (const void*)keys_out || (const void*)vals_in == (const void*)vals_out;
-  const int passes = L.plan.passes;
-  if (!inplace || (passes % 2 == 0 && passes > 0)) {
-    // pass 0 writes tmp when passes is even, so in-place is safe then.
-    return run_sort(L.plan, src, (u64*)keys_out, vals_out, tk, tv, ws, s);
+  if (!inplace)
+    return run_pair_sort(L.sort, src, (u64*)keys_out, vals_out, ws + L.off_a, ws + L.off_b, ws, s);
+  // In place.  The bucketed path reads all input before it writes output, and
+  // leaves the output alone when its gate closes.
+  const SortPlan& lsd = L.sort.lsd;
+  u32* gate = nullptr;
+  if (L.sort.msd.ok) {
+    gate = reinterpret_cast<u32*>(ws + L.sort.ctrl_bytes - 256);
+    const int st = run_msd_sort(L.sort.msd, src, ws + L.off_b, ws + L.off_a, ws, nullptr, (u64*)keys_out, vals_out,
+                                gate, s);
+    if (st != LNT_OK) return st;
+    src = gated_source(src, gate, 1);
   }
-  // In place with an odd pass count (or nothing to sort): sort into the
-  // second scratch pair and copy back.
-  u64* t2k = reinterpret_cast<u64*>(ws + L.off_t2k);
-  double* t2v = reinterpret_cast<double*>(ws + L.off_t2v);
-  if (passes == 0) return LNT_OK;  // all keys equal: input order is the stable order
-  int st = run_sort(L.plan, src, t2k, t2v, tk, tv, ws, s);
+  if (lsd.passes == 0) return LNT_OK;  // all keys equal: input order is the stable order
+  u64* tk = reinterpret_cast<u64*>(ws + L.off_a);
+  double* tv = reinterpret_cast<double*>(ws + L.off_a + L.sort.a_bytes / 2);
+  if (lsd.passes % 2 == 0)  // the first pass writes the scratch pairs
+    return run_sort(lsd, src, (u64*)keys_out, vals_out, tk, tv, ws, s);
+  // odd pass count: sort into the second scratch pairs and copy back
+  u64* t2k = reinterpret_cast<u64*>(ws + L.off_b);
+  double* t2v = reinterpret_cast<double*>(ws + L.off_b + L.sort.a_bytes / 2);
+  const int st = run_sort(lsd, src, t2k, t2v, tk, tv, ws, s);
   if (st != LNT_OK) return st;
-  if (cudaMemcpyAsync(keys_out, t2k, n * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-  if (cudaMemcpyAsync(vals_out, t2v, n * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-  return LNT_OK;
+  const int blocks = std::max(1, std::min((int)((n + 255) / 256), sm_count() * 8));
+  copy_source_kernel<<<blocks, 256, 0, s>>>(gated_source(plain_source(t2k, t2v, n), gate, 1), (u64*)keys_out, vals_out,
+                                            (u32)n);
+  count_launch();
+  return launch_status();
 }
 
 }  // extern "C"

@@ -35,7 +35,7 @@ struct PairSource {
   RekeyParams ra;
   RekeyParams rb;
   // Kernels reading this source run only when gate == nullptr or
-  // *gate == gate_run (see gated_off); a gated sort uses persistent grids.
+  // *gate == gate_run (see gated_off).
   const u32* gate;
   u32 gate_run;
   u32 pad2;
@@ -107,12 +107,17 @@ struct SortPlan {
 // else the tuned table.
 int choose_sort_variant(size_t n, int key_bits);
 
-// Fills a plan for n pairs with keys < max_key (variant < 0: choose).
-SortPlan make_sort_plan(size_t n, u64 max_key, int variant = -1);
+// Words of a gate block: [0] the gate, then the fallback sort's queue and step
+// counts (zeroed by the kernel that writes the gate).
+constexpr int kGateWords = 32;
+
+// Fills a plan for n pairs with keys < max_key.  gated: for a source behind a
+// gate (one launch, see lsd_queue_kernel; src.gate is then a gate block).
+SortPlan make_sort_plan(size_t n, u64 max_key, bool gated = false);
 
 // Runs the passes.  Pass p reads the previous pass's output (pass 0 reads
 // src) and writes buffer ((passes-1-p) & 1): buf0 = final destination.
-// `ctrl` points at plan.ctrl_bytes of scratch, zeroed here.
+// `ctrl` points at plan.ctrl_bytes of scratch (16-byte aligned), zeroed here.
 int run_sort(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* buf0_v, u64* buf1_k,
              double* buf1_v, void* ctrl, cudaStream_t s);
 

@@ -34,7 +34,7 @@
 #include <cstring>
 
 #include "lnt_scan.cuh"
-#include "lnt_sort.cuh"
+#include "lnt_msd.cuh"
 
 namespace lnt {
 
@@ -280,6 +280,28 @@ Engine choose_engine(const Shape& s, u64 products) {
   return Engine::Esc;
 }
 
+// Workspace of the ESC engine: the products and the sort's other pairs (A, B).
+struct EscLayout {
+  PairSort sort;
+  size_t off_ctrl, off_a, off_b, off_coll, total;
+};
+
+EscLayout esc_layout(u64 products, u64 max_key) {
+  EscLayout L;
+  L.sort = make_pair_sort(products, max_key);
+  size_t off = 0;
+  L.off_ctrl = off;
+  off += align_up(L.sort.ctrl_bytes, 256);
+  L.off_a = off;
+  off += L.sort.a_bytes;
+  L.off_b = off;
+  off += L.sort.a_bytes;
+  L.off_coll = off;
+  off += align_up(collect_workspace_bytes(products), 256);
+  L.total = off;
+  return L;
+}
+
 // counts[1] = min(counts[0], dense): the output holds at most one entry per
 // (row, col, tab) and at most one per product.
 __global__ void capacity_kernel(u64* counts, u64 dense) { counts[1] = min(counts[0], dense); }
@@ -371,13 +393,7 @@ int lnt_lattice_mult_workspace(const lnt_lattice* a, const lnt_lattice* b, uint6
     return LNT_OK;
   }
   if (products >= (1ull << 30)) return LNT_UNSUPPORTED;
-  const u64 maxc = s.h * s.wB * s.d;
-  SortPlan sp = make_sort_plan(products, maxc);
-  size_t off = 0;
-  off += align_up(sp.ctrl_bytes, 256);
-  off += 4 * align_up(products * 8, 256);  // products (k, v) + sort ping-pong (k, v)
-  off += align_up(collect_workspace_bytes(products), 256);
-  *bytes = off;
+  *bytes = esc_layout(products, s.h * s.wB * s.d).total;
   return LNT_OK;
 }
 
@@ -418,36 +434,40 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   }
   // ESC
   if (products == 0) return cudaMemsetAsync(d_nc, 0, 8, cs) == cudaSuccess ? LNT_OK : LNT_DEVICE_ERROR;
-  const u64 maxc = s.h * s.wB * s.d;
-  SortPlan sp = make_sort_plan(products, maxc);
+  const EscLayout E = esc_layout(products, s.h * s.wB * s.d);
   unsigned char* w = static_cast<unsigned char*>(workspace);
-  size_t off = 0;
-  void* ctrl = w + off;
-  off += align_up(sp.ctrl_bytes, 256);
-  u64* pk = reinterpret_cast<u64*>(w + off);
-  off += align_up(products * 8, 256);
-  double* pv = reinterpret_cast<double*>(w + off);
-  off += align_up(products * 8, 256);
-  u64* k0 = reinterpret_cast<u64*>(w + off);
-  off += align_up(products * 8, 256);
-  double* v0 = reinterpret_cast<double*>(w + off);
-  off += align_up(products * 8, 256);
-  void* coll = w + off;
-  // Pass p of the sort writes buffer (passes-1-p)&1 (0 = (k0,v0), the final one);
-  // expand into the buffer pass 0 does not write.
-  const bool even = sp.passes % 2 == 0;
-  u64* ek = even ? k0 : pk;
-  double* ev = even ? v0 : pv;
+  void* ctrl = w + E.off_ctrl;
+  // Pass p of the LSD sort writes buffer (passes-1-p)&1 (0 = A, the final
+  // one); expand into the buffer its pass 0 does not write.
+  const bool even = E.sort.lsd.passes % 2 == 0;
+  unsigned char* pe = w + (even ? E.off_a : E.off_b);
+  unsigned char* po = w + (even ? E.off_b : E.off_a);
+  u64* ek = reinterpret_cast<u64*>(pe);
+  double* ev = reinterpret_cast<double*>(pe + E.sort.a_bytes / 2);
   {
     ProfScope prof("spgemm_expand", cs);
     expand_kernel<<<grid_for(products, 256), 256, 0, cs>>>(s.A, s.B, ac, boff, products, make_divider(s.w),
                                                           make_divider(s.wB), ek, ev);
     count_launch();
   }
-  // sort products by output key: the sorted run lands in (k0, v0)
-  st = run_sort(sp, plain_source(ek, ev, products), k0, v0, pk, pv, ctrl, cs);
+  const PairSource src = plain_source(ek, ev, products);
+  u32* gate = nullptr;
+  if (E.sort.msd.ok) {  // sort by output key and add up, in one go
+    gate = reinterpret_cast<u32*>(w + E.off_ctrl + E.sort.ctrl_bytes - 256);
+    const MsdFold fold{0, (u64*)d_nc};
+    // (two passes: the second may write over the products, which the first has read)
+    void* x = E.sort.msd.passes == 2 ? po : nullptr;
+    void* y = E.sort.msd.passes == 2 ? pe : po;
+    st = run_msd_sort(E.sort.msd, src, x, y, ctrl, &fold, (u64*)c_keys, c_vals, gate, cs);
+    if (st != LNT_OK) return st;
+  }
+  u64* k0 = reinterpret_cast<u64*>(w + E.off_a);
+  double* v0 = reinterpret_cast<double*>(w + E.off_a + E.sort.a_bytes / 2);
+  u64* k1 = reinterpret_cast<u64*>(w + E.off_b);
+  double* v1 = reinterpret_cast<double*>(w + E.off_b + E.sort.a_bytes / 2);
+  st = run_sort(E.sort.lsd, gated_source(src, gate, 1), k0, v0, k1, v1, ctrl, cs);
   if (st != LNT_OK) return st;
-  return run_collect(k0, v0, products, 0, (u64*)c_keys, c_vals, (u64*)d_nc, coll, cs);
+  return run_collect_gated(k0, v0, products, 0, (u64*)c_keys, c_vals, (u64*)d_nc, w + E.off_coll, cs, gate, 1);
 }
 
 }  // extern "C"

@@ -36,7 +36,7 @@
 #include <cstdlib>
 
 #include "lnt_scan.cuh"
-#include "lnt_sort.cuh"
+#include "lnt_msd.cuh"
 #include "lnt_tuned.h"
 
 namespace lnt {
@@ -110,13 +110,14 @@ TileDims tile_dims(u64 h, u64 w, u64 wB, u64 d, u64 nb) {
 
 struct TileLayout {
   size_t ctrl, ak, av, tk, tv, bk, bv, arow, brow, dslot, tp, bbits, bd, cbits, cnt, base, scan, coll, arec, misc,
-      total;
-  SortPlan pa, pb;
+      xa, total;
+  PairSort pa;   // A's keys are uniform enough for the bucketed path,
+  SortPlan pb;   // B's have the skewed contracted index on top: LSD
 };
 
 TileLayout tile_layout(const TileDims& t, u64 na, u64 nb) {
   TileLayout L;
-  L.pa = make_sort_plan(na, t.h * t.w * t.d);
+  L.pa = make_pair_sort(na, t.h * t.w * t.d);
   L.pb = make_sort_plan(nb, t.w * t.wB * t.d);
   const u64 ncnt = t.d * t.wB * t.np;
   const u64 nmax = std::max(na, nb);
@@ -129,8 +130,8 @@ TileLayout tile_layout(const TileDims& t, u64 na, u64 nb) {
   L.ctrl = take(std::max(L.pa.ctrl_bytes, L.pb.ctrl_bytes));
   L.ak = take(na * 8);
   L.av = take(na * 8);
-  L.tk = take(nmax * 8);
-  L.tv = take(nmax * 8);
+  L.tk = take(2 * align_up(nmax * 8, 256));  // scratch pairs: keys, then values
+  L.tv = L.tk + align_up(nmax * 8, 256);
   L.bk = take(nb * 8);
   L.bv = take(nb * 8);
   L.arow = take((t.h * t.d + 1) * 8);
@@ -145,6 +146,7 @@ TileLayout tile_layout(const TileDims& t, u64 na, u64 nb) {
   L.scan = take(scan::workspace_bytes(ncnt));
   L.coll = take(collect_workspace_bytes(nb));
   L.arec = take(na * sizeof(ARec));
+  L.xa = take(L.pa.b_bytes);
   L.misc = take(256);  // [0] unique B count, [1] slot counter
   L.total = off;
   return L;
@@ -597,7 +599,7 @@ int run_tile_mult(const u64* akeys, const double* avals, u64 na, const u64* bkey
     const int32_t cur[3] = {0, 1, 2}, nxt[3] = {1, 0, 2};
     PairSource src = plain_source(akeys, avals, na);
     if ((st = make_rekey_params(3, dims, cur, nxt, &src.ra)) != LNT_OK) return st;
-    if (na && (st = run_sort(L.pa, src, ak, av, tk, tv, at(L.ctrl), s)) != LNT_OK) return st;
+    if (na && (st = run_pair_sort(L.pa, src, ak, av, tk, at(L.xa), at(L.ctrl), s)) != LNT_OK) return st;
   }
   {
     ProfScope prof("tile_rowptr", s);

@@ -46,6 +46,7 @@ def variants(L):
 
 def time_sort(L, torch, n, key_bits, variant, reps=5):
     os.environ["LNT_SORT_VARIANT"] = str(variant)
+    os.environ["LNT_NO_BUCKETS"] = "1"  # the digit passes, not the bucketed path in front of them
     g = torch.Generator(device="cuda")
     g.manual_seed(n + key_bits)
     hi = min(2 ** key_bits, 2 ** 63 - 1)
@@ -237,6 +238,7 @@ def main():
                 best.append({"key_bits_max": kb, "n_max": n if ln != ln_list[-1] else 2 ** 62, "variant": win,
                              "ms": row["ms"][win], "log_n": ln, "key_bits": kb})
         os.environ.pop("LNT_SORT_VARIANT", None)
+        os.environ.pop("LNT_NO_BUCKETS", None)
         tuned["sort"] = best
         raw["sort"] = {"variants": vs, "results": results}
     if args.batched:

@@ -54,3 +54,34 @@ def test_sort_reduce_bucketed(cuda, torch, n, max_key, kind):
     # general path ran are runs added tile by tile
     assert rel_ok(to_host(v), ev, ea)
     assert cuda.device_status() == 0
+
+
+# (pairs, max_key): the smallest size taken and its neighbours, one bucket's
+# worth, an even and an odd number of digit passes behind the gate, a key so
+# wide that the first partition pass takes eight bits
+SORTS = [(2047, 1 << 20), (2048, 1 << 20), (2049, 1 << 36), (5121, 1 << 12), (70001, 1 << 40), ((1 << 20) + 3, 1 << 50),
+         (600000, 1 << 63)]
+
+
+@pytest.mark.parametrize("inplace", [False, True])
+@pytest.mark.parametrize("kind", ["uniform", "sorted", "one_key", "high_bits"])
+@pytest.mark.parametrize("n,max_key", SORTS)
+def test_sort_pairs_bucketed(cuda, torch, n, max_key, kind, inplace):
+    """Stable and exact whichever path ends up doing it: the bucketed one, or
+    (nearly all pairs on one key; keys with bits above the sorted ones, which
+    keep them) the gated digit passes behind it."""
+    rng = np.random.default_rng(n)
+    keys = _keys(rng, n, max_key, "sorted" if kind == "sorted" else "uniform")
+    if kind == "one_key":
+        keys[rng.random(n) < 0.95] = keys[0]
+    vals = rng.uniform(-1, 1, n)
+    low = keys.copy()
+    if kind == "high_bits" and max_key < 1 << 60:
+        keys[::3] |= np.uint64(1 << 61)
+    k, v = to_dev(keys, torch), to_dev(vals, torch)
+    out = (k, v) if inplace else (None, None)
+    k, v = cuda.sort_pairs(k, v, max_key=max_key, out_keys=out[0], out_vals=out[1])
+    at = np.argsort(low, kind="stable")
+    np.testing.assert_array_equal(to_host(k, np.uint64), keys[at])
+    np.testing.assert_array_equal(to_host(v), vals[at])
+    assert cuda.device_status() == 0
