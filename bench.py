@@ -417,7 +417,7 @@ def run_ours(args):
     value = job_throughput(n, world, ms)
     kernels = {}
     for name in ("sort_hist", "sort_partition", "bucket_sort_collect", "collect_lead", "collect",
-                 "sort_hist_fallback", "sort_onesweep_fallback", "collect_lead_fallback", "collect_fallback"):
+                 "sort_fallback", "collect_lead_fallback", "collect_fallback"):
         t, c = L.profile_query(name)
         kernels[name] = {"ms_total": t, "launches": c}
     L.profile_reset()
@@ -1417,8 +1417,8 @@ def run_unary(args):
                                           C.c_void_p(ws.data_ptr()), ws.numel(), stream), "lnt_contract_attract")
 
     ms, launches, clocks = _timed_steps(torch, step, args)
-    kernels = {k: L.profile_query(k)[0] / args.steps for k in ("unary_map", "collect_lead", "collect", "unary_scan",
-                                                                 "unary_write")}
+    kernels = {k: L.profile_query(k)[0] / args.steps for k in ("unary_fold", "unary_scan", "unary_gather",
+                                                                 "unary_groups")}
     ms = max_over_ranks(ms, world)
     m = int(cnt.item())
     # spot check: output k holds the sum of the diagonal entries a(i,i,k)
@@ -1433,11 +1433,11 @@ def run_unary(args):
     peak, peak_kind = peaks()
     alg = 16.0 * (n + m)
     config = {"workload": "contract_attract b(k) = a(i,i,k): a 8192 x 8192 x 1024, 2^26 entries (a tenth on the "
-                          "diagonal), uniform, key-sorted; step = lnt_contract_attract (map, fold, scan, write)",
+                          "diagonal), uniform, key-sorted; step = lnt_contract_attract (fold, scan, gather, groups)",
               "nnz": int(n), "output_nnz": int(m), "l2": "input far larger than L2", "parallelism": "1 GPU"}
     print(json.dumps(_line("nnz/s", n * world / (ms * 1e-3), ms, args, world, config, {
         "gpu_launches": launches, "cpu_baseline": None, "clocks": clocks, "kernels_ms_per_step": kernels,
-        "roofline": {"bound": "hbm", "kernel": "whole contract_attract call (4 kernels + the fold)",
+        "roofline": {"bound": "hbm", "kernel": "whole contract_attract call (4 kernels)",
                      "achieved": alg / (ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": alg / (ms * 1e-3) / 1e9 / peak, "alg_bytes_per_launch": alg, "avg_launch_ms": ms,
                      "peak_source": peak_kind, "traffic": None},
@@ -1480,7 +1480,7 @@ def run_scanmerge(args):
         L.merge_sorted(sk, sv, bk, bv, 0, out_keys=ok, out_vals=ov, count=cnt, ws=ws_m, sync=False)
 
     ms, launches, clocks = _timed_steps(torch, step, args)
-    kernels = {k: L.profile_query(k)[0] / args.steps for k in ("sort_hist", "sort_onesweep", "merge")}
+    kernels = {k: L.profile_query(k)[0] / args.steps for k in ("sort_hist", "sort_partition", "bucket_sort", "sort_fallback", "merge")}
     ms = max_over_ranks(ms, world)
     m = int(cnt.item())
     assert L.device_status() == 0 and bool(torch.all(ok[1:m] >= ok[:m - 1]).item())  # duplicates within an operand stay

@@ -787,7 +787,7 @@ MsdPlan make_msd_plan(size_t n, u64 max_key) {
   MsdPlan p;
   p.n = (u32)n;
   p.key_bits = key_bits_for(max_key);
-  if (n < kMinPairs || n >= (1u << 30) || getenv("LNT_NO_BUCKETS")) return p;
+  if (n < kMinPairs || n >= (1u << 30) || getenv("LNT_NO_BUCKETS") || getenv("LNT_SORT_VARIANT")) return p;
   const char* force = getenv("LNT_BUCKET_SMALL");
   int bestT = 99;
   for (int large = 0; large < 2; ++large) {

@@ -5,27 +5,33 @@
 // a(!i,j,!i,k,j).
 //
 // Input: keys sorted under [contraction modes, attraction modes, other modes]
-// with those modes' extents sdims.  Pipeline:
-//   1. map: decode each key's digits (multiply-high division by the extents);
-//      a value whose contraction sets disagree becomes 0 (it is not summed);
-//      group key g = key / |contraction modes| (equal attraction + other
-//      indices);
-//   2. fold runs of equal g (the duplicate-collecting kernel, no zero
-//      skipping): the reference's inner summation loop;
-//   3. keep a group when its attraction sets agree and its sum is not zero
-//      (the reference's "if (sum)"), one scan for the output positions, and
-//      write key other + |other| * attraction index in the groups' order (the
-//      reference's emission order); flag whether those keys never decrease
-//      (the result's sorted flag, as push_back maintains it).
+// with those modes' extents sdims.
+//   1. unary_fold_kernel: one read of the keys, and of the values whose
+//      contraction sets agree (the others are not summed).  Every warp folds a
+//      chunk of consecutive entries into one partial sum per group key g = key
+//      / |contraction modes| (equal attraction + other indices), the
+//      reference's inner summation loop.  No warp waits for another: the
+//      partial sums go to the chunk's own slots, and their number to a table.
+//   2. scan_kernel + unary_gather_kernel: the chunks' partial sums made
+//      contiguous (at most one per group and one per chunk).
+//   3. collect_runs_kernel (lnt_collect.cuh) adds up the partial sums of each
+//      group and keeps a group when its attraction sets agree and its sum is
+//      not zero (the reference's "if (sum)"); key other + |other| * attraction
+//      index, in the groups' order (the reference's emission order).
+//   4. unary_sorted_kernel flags whether those keys never decrease (the
+//      result's sorted flag, as push_back maintains it).
+// HBM bound: 8 B per entry and 8 B per agreeing entry read.  Measured on 6.7e7
+// entries in 65,536 groups, a tenth of them agreeing (B200): fold 0.25 ms,
+// everything 0.29 ms, against 1.58 ms when the entries were mapped, folded,
+// scanned and written by kernels that each passed over them.  Folding in one
+// pass with a look-back per tile of 2048 took 0.58 ms (0.37 ms of it without
+// the look-back); two CTAs per SM 0.28 ms, four (64 registers, spilling) 0.27.
 #include <algorithm>
 
+#include "lnt_collect.cuh"
 #include "lnt_scan.cuh"
 
 namespace lnt {
-
-int run_collect(const u64* keys, const double* vals, size_t n, int skip_zero_heads, u64* out_k, double* out_v,
-                u64* d_nout, void* ws, cudaStream_t s);
-size_t collect_workspace_bytes(size_t n);
 
 namespace {
 
@@ -42,72 +48,169 @@ struct UnaryParams {
   u64 other_dim;              // product of the other extents
 };
 
-__device__ __forceinline__ void digits_of(u64 k, const Divider* sd, int first, int count, u64* out) {
-  for (int q = 0; q < count; ++q) {
-    const u64 nk = divide(k, sd[first + q]);
-    out[q] = k - nk * sd[first + q].d;
-    k = nk;
-  }
-}
-
-// true when every set of `part` consecutive digits agrees
-__device__ __forceinline__ bool sets_agree(const u64* dg, const int* part, int nsets) {
-  int s = 0;
+// Clears ok[j] where one of the sets of consecutive digits of c[j] disagrees
+// (the loops over the modes are outside the one over the entries).
+template <int I>
+__device__ __forceinline__ void sets_agree(u64 (&c)[I], bool (&ok)[I], const Divider* sd, const int* part, int nsets) {
+  int q = 0;
+#pragma unroll 1
   for (int p = 0; p < nsets; ++p) {
-    for (int q = s + 1; q < s + part[p]; ++q)
-      if (dg[q] != dg[s]) return false;
-    s += part[p];
-  }
-  return true;
-}
-
-__global__ void unary_map_kernel(const u64* __restrict__ keys, const double* __restrict__ vals, u64 n,
-                                 UnaryParams P, u64* __restrict__ gk, double* __restrict__ gv) {
-  const u64 stride = (u64)gridDim.x * blockDim.x;
-  for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const u64 k = keys[e];
-    u64 dg[LNT_MAX_ORDER];
-    digits_of(k, P.sd, 0, P.ncon, dg);
-    const bool ok = sets_agree(dg, P.con_part, P.ncon_sets);
-    gk[e] = divide(k, P.cdim);
-    gv[e] = ok ? vals[e] : 0.0;
-  }
-}
-
-// Output key of folded group i, or ~0 when the group is not kept.
-struct KeepKey {
-  const u64* ck;
-  const double* cv;
-  const u64* d_nc;
-  UnaryParams P;
-  __device__ __forceinline__ u64 key(size_t i) const {
-    if (i >= *d_nc || cv[i] == 0.0) return ~0ull;
-    const u64 g = ck[i];
-    u64 dg[LNT_MAX_ORDER];
-    digits_of(g, P.sd, P.ncon, P.natt, dg);
-    if (!sets_agree(dg, P.att_part, P.natt_sets)) return ~0ull;
-    u64 att = 0, stride = 1;
-    int s = 0;
-    for (int p = 0; p < P.natt_sets; ++p) {  // sub2ind over the attraction ranges
-      att += dg[s] * stride;
-      stride *= P.sd[P.ncon + s].d;
-      s += P.att_part[p];
+    const Divider dv = sd[q];  // the extents of a set are equal
+    u64 d0[I];
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      const u64 nk = divide(c[j], dv);
+      d0[j] = c[j] - nk * dv.d;
+      c[j] = nk;
     }
-    return divide(g, P.afull) + P.other_dim * att;
+#pragma unroll 1
+    for (int t = 1; t < part[p]; ++t) {
+#pragma unroll
+      for (int j = 0; j < I; ++j) {
+        const u64 nk = p == nsets - 1 && t == part[p] - 1 ? 0 : divide(c[j], dv);  // (the last digit is what is left)
+        ok[j] = ok[j] && c[j] - nk * dv.d == d0[j];
+        c[j] = nk;
+      }
+    }
+    q += part[p];
   }
-  __device__ __forceinline__ u64 operator()(size_t i) const { return key(i) != ~0ull ? 1ull : 0ull; }
+}
+
+constexpr int kFoldThreads = 256, kFoldRows = 8, kFoldBatch = 32 * kFoldRows;
+
+// One warp per chunk of `chunk` (a multiple of 256) entries, in batches of
+// eight rows of 32.  A row inside the open run only adds to the lanes' partial
+// sums; a row with heads closes the open run by a reduction over the warp, and
+// the runs inside it by a segmented scan.
+__global__ void __launch_bounds__(kFoldThreads, 3) unary_fold_kernel(const u64* __restrict__ keys,
+                                                                     const double* __restrict__ vals, size_t n,
+                                                                     u32 chunk, u32 nchunks, const UnaryParams P,
+                                                                     u64* __restrict__ gk, double* __restrict__ gv,
+                                                                     u32* __restrict__ counts) {
+  constexpr int R = kFoldRows;
+  constexpr u32 FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const u32 le = lane == 31 ? FULL : (2u << lane) - 1u;  // this lane and those before it
+  const u32 ci = (u32)((blockIdx.x * (size_t)kFoldThreads + threadIdx.x) >> 5);
+  if (ci >= nchunks) return;
+  const size_t begin = (size_t)ci * chunk, end = min(n, begin + chunk);
+  gk += begin;
+  gv += begin;
+  u64 last = divide(__ldg(keys + begin), P.cdim);  // the open run's group
+  double acc = 0.0;                                // this lane's part of it
+  u32 cnt = 0;
+  for (size_t base = begin; base < end; base += kFoldBatch) {
+    u64 g[R], con[R];
+    double v[R];
+    bool ok[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const size_t i = base + r * 32 + lane;
+      con[r] = i < end ? __ldcs(keys + i) : 0;
+      ok[r] = i < end;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      g[r] = divide(con[r], P.cdim);
+      con[r] -= g[r] * P.cdim.d;
+    }
+    sets_agree(con, ok, P.sd, P.con_part, P.ncon_sets);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = ok[r] ? __ldcs(vals + base + r * 32 + lane) : 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool valid = base + r * 32 + lane < end;
+      if (__all_sync(FULL, !valid || g[r] == last)) {
+        acc += v[r];
+        continue;
+      }
+      u64 prev = __shfl_up_sync(FULL, g[r], 1);
+      if (lane == 0) prev = last;
+      const u32 heads = __ballot_sync(FULL, valid && g[r] != prev);
+      const int first = __ffs(heads) - 1, newest = 31 - __clz(heads);
+      double open = acc + (lane < first ? v[r] : 0.0);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) open += __shfl_xor_sync(FULL, open, o);
+      if (lane == 0) {
+        gk[cnt] = last;
+        gv[cnt] = open;
+      }
+      if (first != newest) {  // runs that begin and end in this row
+        const u32 mine = heads & le;
+        const int start = mine ? 31 - __clz(mine) : 0;
+        double x = v[r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(FULL, x, o);
+          if (lane - o >= start) x = y + x;
+        }
+        if (mine && ((heads >> 1) >> lane & 1u)) {  // the last entry of its run
+          gk[cnt + __popc(mine)] = g[r];
+          gv[cnt + __popc(mine)] = x;
+        }
+      }
+      cnt += __popc(heads);
+      last = __shfl_sync(FULL, g[r], newest);
+      acc = lane >= newest ? v[r] : 0.0;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+  if (lane == 0) {
+    gk[cnt] = last;
+    gv[cnt] = acc;
+    counts[ci] = cnt + 1;
+  }
+}
+
+struct CountOf {
+  const u32* counts;
+  __device__ __forceinline__ u64 operator()(size_t i) const { return counts[i]; }
 };
 
-__global__ void unary_write_kernel(KeepKey kk, u64 n, const unsigned long long* __restrict__ pos,
-                                   u64* __restrict__ out_k, double* __restrict__ out_v) {
-  const u64 stride = (u64)gridDim.x * blockDim.x;
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const u64 k = kk.key(i);
-    if (k == ~0ull) continue;
-    out_k[pos[i]] = k;
-    out_v[pos[i]] = kk.cv[i];
+// Chunk i's partial sums (at i * chunk) to pos[i] (one warp per chunk).
+__global__ void __launch_bounds__(256) unary_gather_kernel(const u64* __restrict__ gk, const double* __restrict__ gv,
+                                                           u32 chunk, u32 nchunks,
+                                                           const unsigned long long* __restrict__ pos,
+                                                           u64* __restrict__ ck, double* __restrict__ cv) {
+  const int lane = threadIdx.x & 31;
+  const u32 ci = (u32)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+  if (ci >= nchunks) return;
+  const u64 to = pos[ci], cnt = pos[ci + 1] - to;
+  const size_t from = (size_t)ci * chunk;
+#pragma unroll 4
+  for (u64 j = lane; j < cnt; j += 32) {
+    ck[to + j] = gk[from + j];
+    cv[to + j] = gv[from + j];
   }
 }
+
+struct UnaryGroups {
+  UnaryParams P;
+  __device__ __forceinline__ bool keep(u64 g, double sum) const {
+    if (sum == 0.0) return false;
+    u64 c[1] = {g - divide(g, P.afull) * P.afull.d};
+    bool ok[1] = {true};
+    sets_agree(c, ok, P.sd + P.ncon, P.att_part, P.natt_sets);
+    return ok[0];
+  }
+  __device__ __forceinline__ u64 out_key(u64 g) const {
+    const u64 other = divide(g, P.afull);
+    u64 c = g - other * P.afull.d, att = 0, stride = 1;
+    int q = P.ncon;
+    for (int p = 0; p < P.natt_sets; ++p) {  // sub2ind over the attraction ranges
+      for (int t = 0; t < P.att_part[p]; ++t, ++q) {
+        const u64 nk = divide(c, P.sd[q]);
+        if (t == 0) {
+          att += (c - nk * P.sd[q].d) * stride;
+          stride *= P.sd[q].d;
+        }
+        c = nk;
+      }
+    }
+    return other + P.other_dim * att;
+  }
+};
 
 __global__ void unary_sorted_kernel(const u64* __restrict__ out_k, const u64* __restrict__ d_nout,
                                     u32* __restrict__ d_sorted) {
@@ -117,26 +220,37 @@ __global__ void unary_sorted_kernel(const u64* __restrict__ out_k, const u64* __
     if (out_k[i] < out_k[i - 1]) *d_sorted = 0u;
 }
 
+// Entries per warp: 256, growing with n to 2048 (fewer partial sums) while
+// every SM still has 32 warps.
+u32 fold_chunk(size_t n) {
+  u32 c = kFoldBatch;
+  while (c < 2048 && n / (2 * c) >= (size_t)sm_count() * 32) c *= 2;
+  return c;
+}
+
 struct UnaryLayout {
-  size_t gk, gv, ck, cv, pos, coll, scan, misc, total;
+  u32 chunk, nchunks;
+  size_t counts, pos, scan, gk, gv, ck, cv, coll, total;
 };
 
 UnaryLayout unary_layout(size_t n) {
   UnaryLayout L;
+  L.chunk = fold_chunk(n);
+  L.nchunks = (u32)((n + L.chunk - 1) / L.chunk);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
     off += align_up(std::max<size_t>(bytes, 8), 256);
     return o;
   };
+  L.counts = take((size_t)L.nchunks * 4);
+  L.pos = take(((size_t)L.nchunks + 1) * 8);
+  L.scan = take(scan::workspace_bytes(L.nchunks));
   L.gk = take(n * 8);
   L.gv = take(n * 8);
   L.ck = take(n * 8);
   L.cv = take(n * 8);
-  L.pos = take((n + 1) * 8);
-  L.coll = take(collect_workspace_bytes(n));
-  L.scan = take(scan::workspace_bytes(n));
-  L.misc = take(256);
+  L.coll = take(collect::layout(n).total);
   L.total = off;
   return L;
 }
@@ -207,33 +321,35 @@ int lnt_contract_attract(const uint64_t* keys, const double* vals, size_t n, int
   const UnaryLayout L = unary_layout(n);
   if (!workspace || workspace_bytes < L.total || (uintptr_t)workspace % 256) return LNT_WORKSPACE;
   cudaStream_t s = as_stream(stream);
+  if (d_sorted && cudaMemsetAsync(d_sorted, 0xff, 4, s) != cudaSuccess) return LNT_DEVICE_ERROR;
+  if (n == 0) return cudaMemsetAsync(d_nout, 0, 8, s) == cudaSuccess ? LNT_OK : LNT_DEVICE_ERROR;
   unsigned char* W = static_cast<unsigned char*>(workspace);
+  u32* counts = reinterpret_cast<u32*>(W + L.counts);
+  unsigned long long* pos = reinterpret_cast<unsigned long long*>(W + L.pos);
   u64* gk = reinterpret_cast<u64*>(W + L.gk);
   double* gv = reinterpret_cast<double*>(W + L.gv);
   u64* ck = reinterpret_cast<u64*>(W + L.ck);
   double* cv = reinterpret_cast<double*>(W + L.cv);
-  unsigned long long* pos = reinterpret_cast<unsigned long long*>(W + L.pos);
-  u64* d_nc = reinterpret_cast<u64*>(W + L.misc);
-  if (d_sorted && cudaMemsetAsync(d_sorted, 0xff, 4, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-  if (n == 0) return cudaMemsetAsync(d_nout, 0, 8, s) == cudaSuccess ? LNT_OK : LNT_DEVICE_ERROR;
+  const u32 blocks = (L.nchunks + kFoldThreads / 32 - 1) / (kFoldThreads / 32);
   {
-    ProfScope prof("unary_map", s);
-    unary_map_kernel<<<grid_n(n), 256, 0, s>>>((const u64*)keys, vals, n, P, gk, gv);
+    ProfScope prof("unary_fold", s);
+    unary_fold_kernel<<<blocks, kFoldThreads, 0, s>>>((const u64*)keys, vals, n, L.chunk, L.nchunks, P, gk, gv, counts);
     count_launch();
   }
-  int st = run_collect(gk, gv, n, 0, ck, cv, d_nc, W + L.coll, s);
-  if (st != LNT_OK) return st;
-  KeepKey kk{ck, cv, d_nc, P};
-  st = scan::run(kk, n, pos, (unsigned long long*)d_nout, W + L.scan, s, "unary_scan");
+  int st = scan::run(CountOf{counts}, L.nchunks, pos, nullptr, W + L.scan, s, "unary_scan");
   if (st != LNT_OK) return st;
   {
-    ProfScope prof("unary_write", s);
-    unary_write_kernel<<<grid_n(n), 256, 0, s>>>(kk, n, pos, (u64*)out_keys, out_vals);
+    ProfScope prof("unary_gather", s);
+    unary_gather_kernel<<<blocks, 256, 0, s>>>(gk, gv, L.chunk, L.nchunks, pos, ck, cv);
     count_launch();
-    if (d_sorted) {
-      unary_sorted_kernel<<<grid_n(n), 256, 0, s>>>((const u64*)out_keys, (const u64*)d_nout, d_sorted);
-      count_launch();
-    }
+  }
+  st = collect::run(ck, cv, (const u64*)(pos + L.nchunks), n, UnaryGroups{P}, (u64*)out_keys, out_vals, (u64*)d_nout,
+                    W + L.coll, s, "unary_groups");
+  if (st != LNT_OK) return st;
+  if (d_sorted) {
+    ProfScope prof("unary_sorted", s);
+    unary_sorted_kernel<<<grid_n(n), 256, 0, s>>>((const u64*)out_keys, (const u64*)d_nout, d_sorted);
+    count_launch();
   }
   return launch_status();
 }
