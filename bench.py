@@ -1037,7 +1037,7 @@ def measure_dense(args):
         per_call = (L.launch_count() - c0) // (reps + max(1, args.warmup // 3))
         L.profile_enable(False)
         kern = {k: L.profile_query(k)[0] / (reps + max(1, args.warmup // 3))
-                for k in ("dense_residues", "dense_exp_a", "dense_exp_b", "dense_residue_a", "dense_residue_b",
+                for k in ("dense_residues", "dense_exp", "dense_residue_a", "dense_residue_b",
                           "dense_mod_gemm", "dense_crt")}
         L.profile_reset()
         e2e = None

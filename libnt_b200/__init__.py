@@ -568,7 +568,7 @@ def dense_crt_workspace(h: int, w: int, wB: int, moduli: int = 13) -> int:
 
 def dense_crt_moduli(A, B, h: int, w: int, wB: int, d: int = 1, tol: float = 1e-12) -> int:
     """Moduli count for dense_mult_crt within tol * |A||B| per entry (lnt_dense_crt_moduli)."""
-    ws = workspace(16 * h + 768, A.device)
+    ws = workspace(16 * h * d + 768, A.device)  # (room for all tabs in one launch)
     m = C.c_int(0)
     _check(lib().lnt_dense_crt_moduli(_ptr(A), _ptr(B), h, w, wB, d, float(tol), _ptr(ws), ws.numel(), C.byref(m),
                                       _stream()), "lnt_dense_crt_moduli")

@@ -41,7 +41,7 @@
 
 namespace lnt {
 
-int run_mod_gemm(const signed char* ra, const signed char* rb, int nmod, const int* moduli, u64 Mp, u64 Np, u64 Kp,
+int run_mod_gemm(const signed char* ra, const signed char* rb, int nmod, int tabs, const int* moduli, u64 Mp, u64 Np, u64 Kp,
                  unsigned char* out, cudaStream_t s);
 
 namespace {
@@ -366,25 +366,114 @@ __device__ __forceinline__ int sym_res(double x, int l, const CrtParams& P) {
   return __double2loint(r + kRound);
 }
 
-// Per-row maximum exponent of A (col-major) over a chunk of columns; eA must
-// start below every double exponent (-4096; an all-zero row keeps it).  e = E + 1 for the row maximum f 2^E, f in [1/2, 1).
-__global__ void row_exp_chunk_kernel(const double* __restrict__ A, u64 h, u64 w, u64 kchunk,
-                                     int* __restrict__ eA) {
-  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= h) return;
-  const u64 k0 = (u64)blockIdx.y * kchunk, k1 = min(w, k0 + kchunk);
-  double m = 0.0;
-  for (u64 k = k0; k < k1; ++k) m = fmax(m, fabs(A[i + h * k]));
-  if (m > 0.0) {
-    int e;
-    frexp(m, &e);
-    atomicMax(&eA[i], e + 1);
+// Scale exponents are kept biased, so that zeroed memory means "no non-zero
+// entry seen": the exponent of such a row or column is -4096, below every
+// double's, and its residues and products are zero.
+constexpr int kExpBias = 8192;
+__device__ __forceinline__ int unbias(int e) { return e ? e - kExpBias : -4096; }
+
+// Row maxima of |A| (col-major, h x w) over the columns [k0, k1), four loads in
+// flight: SUM adds up |a| too.
+template <bool SUM>
+__device__ __forceinline__ void row_chunk(const double* A, u64 h, u64 i, u64 k0, u64 k1, double& m, double& sum) {
+  double mx[4] = {0.0, 0.0, 0.0, 0.0}, sm[4] = {0.0, 0.0, 0.0, 0.0};
+  const double* p = A + i + h * k0;
+  u64 k = k0;
+  for (; k + 4 <= k1; k += 4, p += 4 * h) {
+    double x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = fabs(p[h * q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      mx[q] = fmax(mx[q], x[q]);
+      if (SUM) sm[q] += x[q];
+    }
+  }
+  for (; k < k1; ++k, p += h) {
+    const double x = fabs(*p);
+    mx[0] = fmax(mx[0], x);
+    if (SUM) sm[0] += x;
+  }
+  m = fmax(fmax(mx[0], mx[1]), fmax(mx[2], mx[3]));
+  sum = (sm[0] + sm[1]) + (sm[2] + sm[3]);
+}
+
+// Column maximum (and sum) of |B| over w entries, one warp.
+template <bool SUM>
+__device__ __forceinline__ void col_stat(const double* col, u64 w, double& m, double& sum) {
+  const int lane = threadIdx.x & 31;
+  double mx[4] = {0.0, 0.0, 0.0, 0.0}, sm[4] = {0.0, 0.0, 0.0, 0.0};
+  u64 k = lane;
+  for (; k + 96 < w; k += 128) {
+    double x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = fabs(col[k + 32 * q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      mx[q] = fmax(mx[q], x[q]);
+      if (SUM) sm[q] += x[q];
+    }
+  }
+  for (; k < w; k += 32) {
+    const double x = fabs(col[k]);
+    mx[0] = fmax(mx[0], x);
+    if (SUM) sm[0] += x;
+  }
+  m = fmax(fmax(mx[0], mx[1]), fmax(mx[2], mx[3]));
+  sum = (sm[0] + sm[1]) + (sm[2] + sm[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (SUM) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   }
 }
 
-__global__ void fill_int_kernel(int* __restrict__ p, u64 n, int v) {
-  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
+__device__ __forceinline__ int biased_exp(double m) {  // m > 0: m = f 2^e, f in [1/2, 1)
+  int e;
+  frexp(m, &e);
+  return e + 1 + kExpBias;
+}
+
+// Grid of both statistics kernels: x = blocks over A (256 rows by kchunk
+// columns each), then blocks over B (8 columns each); y = tabs.
+struct StatGrid {
+  u64 h, w, wB, kchunk;
+  unsigned row_blocks, a_blocks, blocks;
+};
+
+// Column chunks short enough that the whole call has about eight blocks per SM
+// (one thread per row and 256 columns left 63 us on 300 rows), and no shorter
+// than 16 columns.
+StatGrid stat_grid(u64 h, u64 w, u64 wB, u64 tabs) {
+  StatGrid g;
+  g.h = h;
+  g.w = w;
+  g.wB = wB;
+  g.row_blocks = (unsigned)((h + 255) / 256);
+  const u64 chunks = std::max<u64>(1, (u64)sm_count() * 8 / (g.row_blocks * tabs));
+  g.kchunk = std::min<u64>(256, std::max<u64>(16, (w + chunks - 1) / chunks));
+  g.a_blocks = g.row_blocks * (unsigned)((w + g.kchunk - 1) / g.kchunk);
+  g.blocks = g.a_blocks + (unsigned)((wB + 7) / 8);
+  return g;
+}
+
+// Scale exponents of the rows of A and the columns of B (eA, eB zeroed before).
+__global__ void __launch_bounds__(256) scale_exp_kernel(const double* __restrict__ A, const double* __restrict__ B,
+                                                        const StatGrid g, int* __restrict__ eA, int* __restrict__ eB) {
+  const u64 t = blockIdx.y;
+  double m, sum;
+  if (blockIdx.x < g.a_blocks) {
+    const u64 i = (u64)(blockIdx.x % g.row_blocks) * 256 + threadIdx.x;
+    const u64 k0 = (u64)(blockIdx.x / g.row_blocks) * g.kchunk;
+    if (i >= g.h) return;
+    row_chunk<false>(A + t * g.h * g.w, g.h, i, k0, min(g.w, k0 + g.kchunk), m, sum);
+    if (m > 0.0) atomicMax(&eA[t * g.h + i], biased_exp(m));
+  } else {
+    const u64 j = (u64)(blockIdx.x - g.a_blocks) * 8 + (threadIdx.x >> 5);
+    if (j >= g.wB) return;
+    col_stat<false>(B + (t * g.wB + j) * g.w, g.w, m, sum);
+    if ((threadIdx.x & 31) == 0 && m > 0.0) eB[t * g.wB + j] = biased_exp(m);
+  }
 }
 
 // Four residues (of four consecutive K entries) packed into one 32-bit word.
@@ -395,15 +484,20 @@ __device__ __forceinline__ u32 pack_res4(const double (&x)[4], int l, const CrtP
 }
 
 // A (h x w col-major) -> residues res[l]: Mp rows of Kp int8 (row-major, K
-// contiguous).  Tile of 32 rows x 128 columns through shared memory: read
-// along rows (coalesced); each lane then turns four consecutive K entries of a
-// row into one 4-byte word per modulus (a warp stores 128 consecutive bytes).
+// contiguous; the padding rows and columns zero).  Tile of 32 rows x 128
+// columns through shared memory: read along rows (coalesced); each lane then
+// turns four consecutive K entries of a row into one 4-byte word per modulus
+// (a warp stores 128 consecutive bytes).  Grid z: tabs, P.n planes each.
 __global__ void __launch_bounds__(256) residue_a_kernel(const double* __restrict__ A, u64 h, u64 w, u64 Mp, u64 Kp,
                                                         const int* __restrict__ eA, CrtParams P,
                                                         signed char* __restrict__ res) {
   __shared__ double tile[32][129];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u64 i0 = (u64)blockIdx.x * 32, k0 = (u64)blockIdx.y * 128;
+  A += blockIdx.z * h * w;
+  eA += blockIdx.z * h;
+  res += blockIdx.z * P.n * Mp * Kp;
+#pragma unroll 8
   for (int kk = warp; kk < 128; kk += 8) {
     const u64 i = i0 + lane, k = k0 + kk;
     tile[lane][kk] = (i < h && k < w) ? A[i + h * k] : 0.0;
@@ -413,8 +507,8 @@ __global__ void __launch_bounds__(256) residue_a_kernel(const double* __restrict
   if (k >= Kp) return;
   for (int rr = warp; rr < 32; rr += 8) {
     const u64 i = i0 + rr;
-    if (i >= h) continue;
-    const int sc = P.beta - eA[i];
+    if (i >= Mp) continue;
+    const int sc = i < h ? P.beta - unbias(eA[i]) : 0;
     double x[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) x[c] = rint(scale2(tile[rr][4 * lane + c], sc));
@@ -428,20 +522,23 @@ __global__ void __launch_bounds__(256) residue_a_kernel(const double* __restrict
   }
 }
 
-// B (w x wB col-major) -> residues res[l]: Np rows (columns of B) of Kp int8.
-// Grid: y over columns of B, x over groups of four K entries (one 4-byte word
-// per modulus; entries beyond w are zero).
+// B (w x wB col-major) -> residues res[l]: Np rows (columns of B, the padding
+// ones zero) of Kp int8.  Grid: y over the rows, x over groups of four K
+// entries (one 4-byte word per modulus; entries beyond w are zero), z tabs.
 __global__ void residue_b_kernel(const double* __restrict__ B, u64 w, u64 wB, u64 Np, u64 Kp,
                                  const int* __restrict__ eB, CrtParams P, signed char* __restrict__ res) {
   const u64 plane = Np * Kp / 4;
-  for (u64 j = blockIdx.y; j < wB; j += gridDim.y) {
-    const int sc = P.beta - eB[j];
+  B += blockIdx.z * w * wB;
+  eB += blockIdx.z * wB;
+  res += blockIdx.z * P.n * Np * Kp;
+  for (u64 j = blockIdx.y; j < Np; j += gridDim.y) {
+    const int sc = j < wB ? P.beta - unbias(eB[j]) : 0;
     const double* col = B + w * j;
     u32* dst = reinterpret_cast<u32*>(res + j * Kp);
     for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; 4 * g < Kp; g += (u64)gridDim.x * blockDim.x) {
       double x[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) x[c] = 4 * g + c < w ? rint(scale2(col[4 * g + c], sc)) : 0.0;
+      for (int c = 0; c < 4; ++c) x[c] = 4 * g + c < w && j < wB ? rint(scale2(col[4 * g + c], sc)) : 0.0;
 #pragma unroll
       for (int l = 0; l < kMaxModuli; ++l) {
         if (l >= P.n) break;
@@ -471,9 +568,13 @@ __global__ void __launch_bounds__(256) crt_kernel(const unsigned char* __restric
   const u64 i0 = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i0 >= h) return;  // Mp is a multiple of 16: rows i0 .. i0+3 lie inside every plane
   const u64 plane = Mp * Np;
+  res += blockIdx.z * P.n * plane;  // tabs
+  eA += blockIdx.z * h;
+  eB += blockIdx.z * wB;
+  C += blockIdx.z * h * wB;
   int ea[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) ea[c] = i0 + c < h ? eA[i0 + c] - 2 * P.beta : 0;
+  for (int c = 0; c < 4; ++c) ea[c] = i0 + c < h ? unbias(eA[i0 + c]) - 2 * P.beta : 0;
   constexpr long long kMask = (1ll << kLimbBits) - 1;
   constexpr double kRadix = (double)(1ll << kLimbBits);
   const u64 w0 = i0 - 4 * (threadIdx.x & 31);  // the warp's first row: 128 rows, <= 128 bytes per plane
@@ -534,7 +635,7 @@ __global__ void __launch_bounds__(256) crt_kernel(const unsigned char* __restric
       double x = (double)a[LV];
 #pragma unroll
       for (int b = LV - 1; b >= 0; --b) x = fma(x, kRadix, (double)a[b]);
-      C[i0 + c + h * j] = scale2(x, ea[c] + eB[j]);
+      C[i0 + c + h * j] = scale2(x, ea[c] + unbias(eB[j]));
     }
   }
 }
@@ -547,47 +648,40 @@ __global__ void __launch_bounds__(256) crt_kernel(const unsigned char* __restric
 // These kernels find the largest such ratio over the rows of A and the
 // columns of B (all-zero rows and columns excluded).
 
-// Per-row max |a| (as ordered bit patterns) and sum |a| over a chunk of columns.
-__global__ void row_absstat_kernel(const double* __restrict__ A, u64 h, u64 w, u64 kchunk,
-                                   unsigned long long* __restrict__ rmax, double* __restrict__ rsum) {
-  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= h) return;
-  const u64 k0 = (u64)blockIdx.y * kchunk, k1 = min(w, k0 + kchunk);
-  double m = 0.0, sm = 0.0;
-  for (u64 k = k0; k < k1; ++k) {
-    const double x = fabs(A[i + h * k]);
-    m = fmax(m, x);
-    sm += x;
+// Per-row max |a| (as ordered bit patterns) and sum |a| of A over a chunk of
+// columns; max / mean of the columns of B straight into *out.
+__global__ void __launch_bounds__(256) abs_stat_kernel(const double* __restrict__ A, const double* __restrict__ B,
+                                                       const StatGrid g, unsigned long long* __restrict__ rmax,
+                                                       double* __restrict__ rsum,
+                                                       unsigned long long* __restrict__ out) {
+  const u64 t = blockIdx.y;
+  double m, sum;
+  if (blockIdx.x < g.a_blocks) {
+    const u64 i = (u64)(blockIdx.x % g.row_blocks) * 256 + threadIdx.x;
+    const u64 k0 = (u64)(blockIdx.x / g.row_blocks) * g.kchunk;
+    if (i >= g.h) return;
+    row_chunk<true>(A + t * g.h * g.w, g.h, i, k0, min(g.w, k0 + g.kchunk), m, sum);
+    // non-negative: bit order = value order
+    atomicMax(&rmax[t * g.h + i], (unsigned long long)__double_as_longlong(m));
+    atomicAdd(&rsum[t * g.h + i], sum);
+  } else {
+    const u64 j = (u64)(blockIdx.x - g.a_blocks) * 8 + (threadIdx.x >> 5);
+    if (j >= g.wB) return;
+    col_stat<true>(B + (t * g.wB + j) * g.w, g.w, m, sum);
+    if ((threadIdx.x & 31) == 0 && sum > 0.0)
+      atomicMax(out, (unsigned long long)__double_as_longlong(m * (double)g.w / sum));
   }
-  atomicMax(&rmax[i], (unsigned long long)__double_as_longlong(m));  // non-negative: bit order = value order
-  atomicAdd(&rsum[i], sm);
 }
 
-__global__ void row_ratio_kernel(const unsigned long long* __restrict__ rmax, const double* __restrict__ rsum, u64 h,
+// max / mean over the rows (rows of all tabs).
+__global__ void row_ratio_kernel(const unsigned long long* __restrict__ rmax, const double* __restrict__ rsum, u64 rows,
                                  u64 w, unsigned long long* __restrict__ out) {
   const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= h || !(rsum[i] > 0.0)) return;
-  const double r = __longlong_as_double((long long)rmax[i]) * (double)w / rsum[i];
-  atomicMax(out, (unsigned long long)__double_as_longlong(r));
-}
-
-// One warp per column of B (w x wB, col-major): max / mean of |b|.
-__global__ void col_ratio_kernel(const double* __restrict__ B, u64 w, u64 wB, unsigned long long* __restrict__ out) {
-  const u64 j = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (j >= wB) return;
-  double m = 0.0, sm = 0.0;
-  for (u64 k = lane; k < w; k += 32) {
-    const double x = fabs(B[k + w * j]);
-    m = fmax(m, x);
-    sm += x;
-  }
+  double r = 0.0;
+  if (i < rows && rsum[i] > 0.0) r = __longlong_as_double((long long)rmax[i]) * (double)w / rsum[i];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    sm += __shfl_xor_sync(0xffffffffu, sm, o);
-  }
-  if (lane == 0 && sm > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(m * (double)w / sm));
+  for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+  if ((threadIdx.x & 31) == 0 && r > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(r));
 }
 
 struct CrtLayout {
@@ -595,25 +689,32 @@ struct CrtLayout {
   size_t off_ea, off_eb, off_ra, off_rb, off_prod, total;
 };
 
-CrtLayout crt_layout(u64 h, u64 w, u64 wB, int n) {
+// `tabs` products side by side (every region holds them one after another).
+CrtLayout crt_layout(u64 h, u64 w, u64 wB, int n, u64 tabs = 1) {
   CrtLayout L;
   L.Kp = (w + 15) / 16 * 16;
   L.Mp = (h + 15) / 16 * 16;
   L.Np = (wB + 15) / 16 * 16;
   size_t off = 0;
   L.off_ea = off;
-  off += align_up(h * 4, 256);
+  off += align_up(tabs * h * 4, 256);
   L.off_eb = off;
-  off += align_up(wB * 4, 256);
+  off += align_up(tabs * wB * 4, 256);
   L.off_ra = off;
-  off += align_up((u64)n * L.Mp * L.Kp, 256);
+  off += align_up(tabs * n * L.Mp * L.Kp, 256);
   L.off_rb = off;
-  off += align_up((u64)n * L.Np * L.Kp, 256);
+  off += align_up(tabs * n * L.Np * L.Kp, 256);
   L.off_prod = off;  // residues of the products: n planes of Mp x Np bytes
-  off += align_up((u64)n * L.Mp * L.Np, 256);
+  off += align_up(tabs * n * L.Mp * L.Np, 256);
   L.total = off;
   return L;
 }
+
+// Tabs run together: as many as the workspace holds, and the workspace query
+// asks for room for up to 16 while that stays below 64 MB (a tab at a time
+// left most SMs idle on small products, and paid its launches once per tab).
+constexpr u64 kTabGroup = 16;
+constexpr size_t kTabGroupBytes = 64ull << 20;
 
 // Host: moduli tables for n moduli and inner dimension K.
 int make_crt_params(int n, u64 K, CrtParams* P) {
@@ -788,19 +889,24 @@ int lnt_dense_crt_moduli(const double* A, const double* B, int64_t h, int64_t w,
   const size_t need = align_up((size_t)h * 8, 256) * 2 + 256;
   if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256) return LNT_WORKSPACE;
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  auto* rmax = reinterpret_cast<unsigned long long*>(ws);
-  auto* rsum = reinterpret_cast<double*>(ws + align_up((size_t)h * 8, 256));
-  auto* out = reinterpret_cast<unsigned long long*>(ws + 2 * align_up((size_t)h * 8, 256));
   cudaStream_t s = as_stream(stream);
-  const u64 uh = h, uw = w, uwB = wB, kchunk = 256;
-  if (cudaMemsetAsync(out, 0, 8, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-  for (int64_t t = 0; t < d; ++t) {
-    if (cudaMemsetAsync(ws, 0, 2 * align_up((size_t)h * 8, 256), s) != cudaSuccess) return LNT_DEVICE_ERROR;
-    row_absstat_kernel<<<dim3((unsigned)((uh + 255) / 256), (unsigned)((uw + kchunk - 1) / kchunk)), 256, 0, s>>>(
-        A + (u64)t * uh * uw, uh, uw, kchunk, rmax, rsum);
-    row_ratio_kernel<<<(unsigned)((uh + 255) / 256), 256, 0, s>>>(rmax, rsum, uh, uw, out);
-    col_ratio_kernel<<<(unsigned)((uwB * 32 + 255) / 256), 256, 0, s>>>(B + (u64)t * uw * uwB, uw, uwB, out);
-    count_launch(3);
+  const u64 uh = h, uw = w, uwB = wB;
+  // tabs per launch: what the workspace has room for
+  u64 group = std::min<u64>((u64)d, 65535);
+  while (group > 1 && align_up(group * uh * 8, 256) * 2 + 256 > workspace_bytes) group = (group + 1) / 2;
+  const size_t part = align_up(group * uh * 8, 256);
+  auto* out = reinterpret_cast<unsigned long long*>(ws);
+  auto* rmax = reinterpret_cast<unsigned long long*>(ws + 256);
+  auto* rsum = reinterpret_cast<double*>(ws + 256 + part);
+  for (u64 t = 0; t < (u64)d; t += group) {
+    const u64 n = std::min<u64>(group, (u64)d - t);
+    const size_t skip = t ? 256 : 0;  // *out is zeroed once
+    if (cudaMemsetAsync(ws + skip, 0, 256 + 2 * part - skip, s) != cudaSuccess) return LNT_DEVICE_ERROR;
+    const StatGrid g = stat_grid(uh, uw, uwB, n);
+    ProfScope prof("dense_moduli", s);
+    abs_stat_kernel<<<dim3(g.blocks, (unsigned)n), 256, 0, s>>>(A + t * uh * uw, B + t * uw * uwB, g, rmax, rsum, out);
+    row_ratio_kernel<<<(unsigned)((n * uh + 255) / 256), 256, 0, s>>>(rmax, rsum, n * uh, uw, out);
+    count_launch(2);
   }
   unsigned long long bits = 0;
   if (cudaMemcpyAsync(&bits, out, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess) return LNT_DEVICE_ERROR;
@@ -831,6 +937,11 @@ int lnt_dense_crt_workspace(int64_t h, int64_t w, int64_t wB, int moduli, size_t
   st = make_crt_params(moduli, (u64)w, &P);
   if (st != LNT_OK) return st;
   *bytes = crt_layout(h, w, wB, moduli).total;
+  for (u64 tabs = 2; tabs <= kTabGroup; ++tabs) {
+    const size_t b = crt_layout(h, w, wB, moduli, tabs).total;
+    if (b > kTabGroupBytes) break;
+    *bytes = b;
+  }
   return LNT_OK;
 }
 
@@ -839,14 +950,15 @@ int lnt_dense_lattice_mult_crt(const double* A, const double* B, double* C, int6
   int st = check_dense(h, w, wB, d);
   if (st != LNT_OK) return st;
   if (!A || !B || !C) return LNT_BAD_ARG;
-  size_t need = 0;
-  st = lnt_dense_crt_workspace(h, w, wB, moduli, &need);
-  if (st != LNT_OK) return st;
-  if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256) return LNT_WORKSPACE;
+  if ((u64)w >= (1ull << 17)) return LNT_UNSUPPORTED;  // INT32 exactness: K * 2^14 < 2^31
   CrtParams P;
   st = make_crt_params(moduli, (u64)w, &P);
   if (st != LNT_OK) return st;
-  const CrtLayout L = crt_layout(h, w, wB, moduli);
+  if (!workspace || workspace_bytes < crt_layout(h, w, wB, moduli).total || (uintptr_t)workspace % 256)
+    return LNT_WORKSPACE;
+  u64 group = std::min<u64>((u64)d, kTabGroup);
+  while (group > 1 && crt_layout(h, w, wB, moduli, group).total > workspace_bytes) --group;
+  const CrtLayout L = crt_layout(h, w, wB, moduli, group);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   int* eA = reinterpret_cast<int*>(ws + L.off_ea);
   int* eB = reinterpret_cast<int*>(ws + L.off_eb);
@@ -856,49 +968,41 @@ int lnt_dense_lattice_mult_crt(const double* A, const double* B, double* C, int6
   cudaStream_t s = as_stream(stream);
   const int sms = sm_count();
   const u64 uh = h, uw = w, uwB = wB, Kp = L.Kp;
-  for (int64_t t = 0; t < d; ++t) {
-    const double* At = A + (u64)t * uh * uw;
-    const double* Bt = B + (u64)t * uw * uwB;
-    double* Ct = C + (u64)t * uh * uwB;
+  for (u64 t = 0; t < (u64)d; t += group) {
+    const unsigned n = (unsigned)std::min<u64>(group, (u64)d - t);
+    const double* At = A + t * uh * uw;
+    const double* Bt = B + t * uw * uwB;
+    double* Ct = C + t * uh * uwB;
     {
       ProfScope prof("dense_residues", s);
-      const u64 kchunk = 256;
-      fill_int_kernel<<<(unsigned)((uh + 255) / 256), 256, 0, s>>>(eA, uh, -4096);  // below any double exponent
+      if (cudaMemsetAsync(ws, 0, L.off_ra, s) != cudaSuccess) return LNT_DEVICE_ERROR;  // eA, eB
       {
-        ProfScope prof_a("dense_exp_a", s);
-        row_exp_chunk_kernel<<<dim3((unsigned)((uh + 255) / 256), (unsigned)((uw + kchunk - 1) / kchunk)), 256, 0,
-                               s>>>(At, uh, uw, kchunk, eA);
-      }
-      {
-        ProfScope prof_b("dense_exp_b", s);
-        col_exp_kernel<<<(unsigned)((uwB * 32 + 255) / 256), 256, 0, s>>>(Bt, uw, uwB, eB);
-      }
-      if (Kp != uw || L.Mp != uh || L.Np != uwB) {  // zero every padding row and column
-        if (cudaMemsetAsync(ra, 0, (u64)moduli * L.Mp * Kp, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-        if (cudaMemsetAsync(rb, 0, (u64)moduli * L.Np * Kp, s) != cudaSuccess) return LNT_DEVICE_ERROR;
+        const StatGrid g = stat_grid(uh, uw, uwB, n);
+        ProfScope prof_e("dense_exp", s);
+        scale_exp_kernel<<<dim3(g.blocks, n), 256, 0, s>>>(At, Bt, g, eA, eB);
       }
       {
         ProfScope prof_ra("dense_residue_a", s);
-        residue_a_kernel<<<dim3((unsigned)((uh + 31) / 32), (unsigned)((Kp + 127) / 128)), 256, 0, s>>>(
+        residue_a_kernel<<<dim3((unsigned)((L.Mp + 31) / 32), (unsigned)((Kp + 127) / 128), n), 256, 0, s>>>(
             At, uh, uw, L.Mp, Kp, eA, P, ra);
       }
       const unsigned gx = (unsigned)std::min<u64>((Kp / 4 + 255) / 256, 64);
-      const unsigned gyb = (unsigned)std::min<u64>(uwB, std::max<u64>(1, (u64)sms * 64 / gx));
+      const unsigned gyb = (unsigned)std::min<u64>(L.Np, std::max<u64>(1, (u64)sms * 64 / gx));
       {
         ProfScope prof_rb("dense_residue_b", s);
-        residue_b_kernel<<<dim3(gx, gyb), 256, 0, s>>>(Bt, uw, uwB, L.Np, Kp, eB, P, rb);
+        residue_b_kernel<<<dim3(gx, gyb, n), 256, 0, s>>>(Bt, uw, uwB, L.Np, Kp, eB, P, rb);
       }
-      count_launch(5);
+      count_launch(3);
     }
     // all moduli's products on the tensor cores, reduced modulo m_l in the epilogue
-    st = run_mod_gemm(ra, rb, moduli, P.m, L.Mp, L.Np, Kp, prod, s);
+    st = run_mod_gemm(ra, rb, moduli, (int)n, P.m, L.Mp, L.Np, Kp, prod, s);
     if (st != LNT_OK) return st;
     {
       ProfScope prof("dense_crt", s);
       const u64 rows4 = (uh + 3) / 4;
       const unsigned gx = (unsigned)((rows4 + 255) / 256);
       const unsigned gy = (unsigned)std::min<u64>(uwB, std::max<u64>(1, (u64)sms * 32 / gx));
-      const dim3 grid(gx, gy);
+      const dim3 grid(gx, gy, n);
       switch (P.lv) {
         case 1:
         case 2:

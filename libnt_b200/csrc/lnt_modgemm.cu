@@ -51,7 +51,7 @@ constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024 /* alignment 
 
 struct ModGemmArgs {
   u64 Mp, Np, Kp;
-  int nmod;
+  int nmod, planes;  // moduli; planes = moduli x tabs
   int tiles_m, tiles_n;
   int mod[24];
   u32 off[24];     // m ceil(2^31 / m): makes a product non-negative without changing its residue
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) mod_gemm_kernel(const __grid_cons
   __syncthreads();
   tc_fence_after();
   const u32 tmem = *tmem_holder;
-  const int total = args.nmod * args.tiles_m * args.tiles_n;
+  const int total = args.planes * args.tiles_m * args.tiles_n;
   const int nk = (int)((args.Kp + kBK - 1) / kBK);
 
   if (warp == 0) {
@@ -313,8 +313,9 @@ __global__ void __launch_bounds__(kThreads, 1) mod_gemm_kernel(const __grid_cons
       const int got = lane == 0 ? (int)mbar_wait(tfull, (u32)(it & 1), abort_flag) : 0;
       if (!__shfl_sync(0xffffffffu, got, 0)) break;
       tc_fence_after();
-      const u32 m = (u32)args.mod[l], off = args.off[l];
-      const u64 magic = args.magic[l];
+      const int lm = l % args.nmod;
+      const u32 m = (u32)args.mod[lm], off = args.off[lm];
+      const u64 magic = args.magic[lm];
       unsigned char* plane = args.out + (size_t)l * args.Mp * args.Np;
 #pragma unroll 1
       for (int mb = 0; mb < 2; ++mb) {
@@ -379,18 +380,19 @@ bool make_plane_map(CUtensorMap* map, const void* base, u64 Kp, u64 rows, int nm
 
 }  // namespace
 
-// The residue GEMMs of scheme II (see the file comment).  ra: nmod planes of
-// Mp x Kp int8, rb: nmod planes of Np x Kp int8 (both 16-byte aligned, Kp a
+// The residue GEMMs of scheme II (see the file comment) of `tabs` products.
+// ra: per tab nmod planes of Mp x Kp int8, rb: nmod planes of Np x Kp int8 (both 16-byte aligned, Kp a
 // multiple of 16), out: nmod planes of Mp x Np uint8.  Returns an lnt_status.
-int run_mod_gemm(const signed char* ra, const signed char* rb, int nmod, const int* moduli, u64 Mp, u64 Np, u64 Kp,
+int run_mod_gemm(const signed char* ra, const signed char* rb, int nmod, int tabs, const int* moduli, u64 Mp, u64 Np, u64 Kp,
                  unsigned char* out, cudaStream_t s) {
-  if (nmod < 1 || nmod > 24 || Kp % 16 || (uintptr_t)ra % 16 || (uintptr_t)rb % 16) return LNT_BAD_ARG;
+  if (nmod < 1 || nmod > 24 || tabs < 1 || Kp % 16 || (uintptr_t)ra % 16 || (uintptr_t)rb % 16) return LNT_BAD_ARG;
   if (Kp >= (1ull << 17)) return LNT_UNSUPPORTED;  // |P| <= Kp 2^14 < 2^31
   ModGemmArgs a;
   a.Mp = Mp;
   a.Np = Np;
   a.Kp = Kp;
   a.nmod = nmod;
+  a.planes = nmod * tabs;
   a.tiles_m = (int)((Mp + kBM - 1) / kBM);
   a.tiles_n = (int)((Np + kBN - 1) / kBN);
   for (int l = 0; l < 24; ++l) {
@@ -401,11 +403,11 @@ int run_mod_gemm(const signed char* ra, const signed char* rb, int nmod, const i
   }
   a.out = out;
   CUtensorMap ma, mb;
-  if (!make_plane_map(&ma, ra, Kp, Mp, nmod) || !make_plane_map(&mb, rb, Kp, Np, nmod)) return LNT_DEVICE_ERROR;
+  if (!make_plane_map(&ma, ra, Kp, Mp, a.planes) || !make_plane_map(&mb, rb, Kp, Np, a.planes)) return LNT_DEVICE_ERROR;
   if (cudaFuncSetAttribute(mod_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) !=
       cudaSuccess)
     return LNT_DEVICE_ERROR;
-  const long long tiles = (long long)nmod * a.tiles_m * a.tiles_n;
+  const long long tiles = (long long)a.planes * a.tiles_m * a.tiles_n;
   if (tiles >= (1ll << 31)) return LNT_UNSUPPORTED;
   const int grid = (int)std::min<long long>(tiles, sm_count());
   ProfScope prof("dense_mod_gemm", s);
