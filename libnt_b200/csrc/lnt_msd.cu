@@ -612,29 +612,46 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
   }
   __syncthreads();
   if (ranked) {
-    // sort (and fold) the sub-buckets of more than one record, each by the
-    // thread that holds its counts: about one per thread, of two records
-    u32 todo = 0;  // bit 4 j + i: count i of word j is above 1
+    // sort (and fold) the sub-buckets of more than one record, each by one
+    // thread: about one per thread, of two records.  Count words go to the
+    // threads in turn, so that each gets its share also when the key has
+    // fewer bits than there are sub-buckets.
+    u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const u32 gt = __vcmpgtu4(s_cnt[tid * 8 + j], 0x01010101u) & 0x08040201u;
+      const u32 gt = __vcmpgtu4(s_cnt[j * BT + tid], 0x01010101u) & 0x08040201u;
       todo |= ((gt | (gt >> 8) | (gt >> 16) | (gt >> 24)) & 0xFu) << (4 * j);
     }
     while (todo) {
       const int i = __ffs(todo) - 1, sh = 8 * (i & 3);
       todo &= todo - 1u;
-      const u32 c4 = s_cnt[tid * 8 + (i >> 2)];
-      const u32 lo = s_base[tid * 8 + (i >> 2)] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
+      const u32 c4 = s_cnt[(i >> 2) * BT + tid];
+      const u32 lo = s_base[(i >> 2) * BT + tid] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
       const u32 k = (c4 >> sh) & 0xFFu;
       const ulonglong2 e0 = s_r[lo], e1 = s_r[lo + 1];
-      if (k == 2 && (!FOLD || ((e0.x ^ e1.x) >> ib) != 0)) {  // nearly always
-        if (e1.x < e0.x) {
-          s_r[lo] = e1;
-          s_r[lo + 1] = e0;
+      if (k == 2) {  // nearly always
+        const bool swap = e1.x < e0.x;
+        const ulonglong2 f = swap ? e1 : e0, g = swap ? e0 : e1;
+        if (FOLD) {
+          const double x = __longlong_as_double((long long)f.y), y = __longlong_as_double((long long)g.y);
+          const bool equal = ((f.x ^ g.x) >> ib) == 0;
+          u32 drop = equal ? 2u : 0u;  // bit q: position lo + q is not written
+          if (skip_zero_heads) {
+            if (x == 0.0 && !(equal && y != 0.0) && start + lo != 0) drop |= 1u;
+            if (!equal && y == 0.0) drop |= 2u;
+          }
+          if (drop & 1u) atomicAnd(&s_kept[lo >> 5], ~(1u << (lo & 31)));
+          if (drop & 2u) atomicAnd(&s_kept[(lo + 1) >> 5], ~(1u << ((lo + 1) & 31)));
+          if (equal) {
+            s_r[lo] = make_ulonglong2(f.x, (u64)__double_as_longlong(x + y));
+          } else if (swap) {
+            s_r[lo] = f;
+            s_r[lo + 1] = g;
+          }
+        } else if (swap) {
+          s_r[lo] = f;
+          s_r[lo + 1] = g;
         }
-        if (FOLD && skip_zero_heads && (__longlong_as_double((long long)e0.y) == 0.0 ||
-                                        __longlong_as_double((long long)e1.y) == 0.0))
-          fold_sub_bucket<FOLD>(s_r + lo, 2, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
       } else {
         fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
       }

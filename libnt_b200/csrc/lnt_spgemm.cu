@@ -122,29 +122,113 @@ struct Identity64 {
 };
 
 // ---- ESC engine ----------------------------------------------------------
-__global__ void expand_kernel(Lat A, Lat B, AColumns ac, const u64* __restrict__ boff, u64 P, Divider div_w,
-                              Divider div_wB, u64* __restrict__ pk, double* __restrict__ pv) {
-  const u64 h = A.rows, w = A.cols;
-  const u64 stride = (u64)gridDim.x * blockDim.x;
-  for (u64 p = (u64)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += stride) {
-    // B entry e with boff[e] <= p < boff[e+1]
-    u64 a = 0, b = B.nnz;
-    while (a < b) {
-      const u64 m = (a + b + 1) >> 1;
-      if (boff[m] <= p) a = m; else b = m - 1;
+// One CTA per 2048 consecutive products.  The B entries they belong to (found
+// by two searches for the tile, not one per product) are decoded once each
+// into shared memory; their first products are marked and a maximum scan gives
+// every product its entry.  Then a product costs its A entry's load and its
+// store.  17.4M products of 1M x 1.1M entries: 0.49 -> 0.12 ms.
+constexpr int kExpandThreads = 256;
+constexpr int kExpandTile = 2048;
+constexpr int kExpandEntries = 1024;  // decoded B entries a tile has room for
+
+// Last e in [a, b] with boff[e] <= p.
+__device__ __forceinline__ u64 entry_of(const u64* __restrict__ boff, u64 a, u64 b, u64 p) {
+  while (a < b) {
+    const u64 m = (a + b + 1) >> 1;
+    if (boff[m] <= p) a = m; else b = m - 1;
+  }
+  return a;
+}
+
+struct ExpandEntry {
+  u64 x0;      // A position of product p: x0 + p (modulo 2^64)
+  u64 kshift;  // C key = A key + kshift
+  double beta;
+};
+
+__device__ __forceinline__ ExpandEntry expand_entry(const Lat& A, const Lat& B, const AColumns& ac, u64 boff_e, u64 e,
+                                                    const Divider& div_w, const Divider& div_wB) {
+  const u64 k = B.keys[e];
+  const u64 bcol = divide(k, div_w);  // col + wB*tab
+  const u64 t = divide(bcol, div_wB);
+  const u64 acol = k - bcol * A.cols + A.cols * t;
+  u64 lo, hi;
+  ac.range(acol, lo, hi);
+  // A key = row + h*acol -> C key = row + h*(col + wB*tab)
+  return {lo - boff_e, A.rows * bcol - A.rows * acol, B.vals[e]};
+}
+
+__global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AColumns ac,
+                                                                const u64* __restrict__ boff, u64 P, Divider div_w,
+                                                                Divider div_wB, u64* __restrict__ pk,
+                                                                double* __restrict__ pv) {
+  constexpr int I = kExpandTile / kExpandThreads;
+  __shared__ ExpandEntry s_e[kExpandEntries];
+  __shared__ __align__(16) unsigned short s_ent[kExpandTile];
+  __shared__ u32 s_warp[kExpandThreads / 32];
+  __shared__ u64 s_range[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const u64 p0 = (u64)blockIdx.x * kExpandTile, p1 = min(P, p0 + kExpandTile);
+  if (tid == 0) s_range[0] = entry_of(boff, 0, B.nnz - 1, p0);
+  if (tid == 32) s_range[1] = entry_of(boff, 0, B.nnz - 1, p1 - 1);
+  reinterpret_cast<uint4*>(s_ent)[tid] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  const u64 e0 = s_range[0], ne = s_range[1] - e0 + 1;
+  if (ne > (u64)kExpandEntries) {  // many B entries without products: each product searches the tile's range
+    for (u64 p = p0 + tid; p < p1; p += kExpandThreads) {
+      const u64 e = entry_of(boff, e0, e0 + ne - 1, p);
+      const ExpandEntry q = expand_entry(A, B, ac, boff[e], e, div_w, div_wB);
+      const u64 x = q.x0 + p;
+      pk[p] = A.keys[x] + q.kshift;
+      pv[p] = A.vals[x] * q.beta;
     }
-    const u64 e = a;
-    const u64 k = B.keys[e];
-    const u64 bcol = divide(k, div_w);
-    const u64 t = divide(bcol, div_wB);
-    const u64 brow = k - bcol * w;
-    const u64 acol = brow + w * t;
-    u64 lo, hi;
-    ac.range(acol, lo, hi);
-    const u64 x = lo + (p - boff[e]);
-    const u64 arow = A.keys[x] - acol * h;
-    pk[p] = arow + h * bcol;  // row + h*(col + wB*tab): bcol already is col + wB*tab
-    pv[p] = A.vals[x] * B.vals[e];
+    return;
+  }
+  for (u32 i = tid; i < (u32)ne; i += kExpandThreads) {
+    const u64 b = boff[e0 + i];
+    // (of the entries that start at one product only the last has products)
+    if (boff[e0 + i + 1] > b) {
+      s_e[i] = expand_entry(A, B, ac, b, e0 + i, div_w, div_wB);
+      if (b > p0) s_ent[b - p0] = (unsigned short)i;  // (entry 0 covers the tile's start)
+    }
+  }
+  __syncthreads();
+  {  // maximum scan over the tile: the entry of every product
+    uint4 q = reinterpret_cast<uint4*>(s_ent)[tid];  // eight consecutive products
+    u32 w[4] = {q.x, q.y, q.z, q.w};
+    u32 run = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const u32 a0 = max(run, w[j] & 0xFFFFu), a1 = max(a0, w[j] >> 16);
+      w[j] = a0 | (a1 << 16);
+      run = a1;
+    }
+    u32 inc = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc = max(inc, t);
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    u32 before = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) before = 0;
+    __syncthreads();
+    for (int x = 0; x < warp; ++x) before = max(before, s_warp[x]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = max(w[j] & 0xFFFFu, before) | (max(w[j] >> 16, before) << 16);
+    reinterpret_cast<uint4*>(s_ent)[tid] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  __syncthreads();
+  static_assert(I == 8, "eight products per thread");
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 o = j * kExpandThreads + tid;
+    if (p0 + o < p1) {
+      const ExpandEntry q = s_e[s_ent[o]];
+      const u64 x = q.x0 + p0 + o;
+      pk[p0 + o] = A.keys[x] + q.kshift;
+      pv[p0 + o] = A.vals[x] * q.beta;
+    }
   }
 }
 
@@ -446,8 +530,8 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   double* ev = reinterpret_cast<double*>(pe + E.sort.a_bytes / 2);
   {
     ProfScope prof("spgemm_expand", cs);
-    expand_kernel<<<grid_for(products, 256), 256, 0, cs>>>(s.A, s.B, ac, boff, products, make_divider(s.w),
-                                                          make_divider(s.wB), ek, ev);
+    expand_kernel<<<(unsigned)((products + kExpandTile - 1) / kExpandTile), kExpandThreads, 0, cs>>>(
+        s.A, s.B, ac, boff, products, make_divider(s.w), make_divider(s.wB), ek, ev);
     count_launch();
   }
   const PairSource src = plain_source(ek, ev, products);
