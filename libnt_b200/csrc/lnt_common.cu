@@ -115,6 +115,7 @@ int make_rekey_params(int order, const int64_t* dims, const int32_t* cur_seq,
   if (!out) return LNT_BAD_ARG;
   out->order = 0;
   out->pow2 = 0;
+  out->narrow = 0;
   if (order <= 1) return order < 0 ? LNT_BAD_ARG : LNT_OK;
   if (order > LNT_MAX_ORDER || !dims || !cur_seq || !new_seq) return LNT_BAD_ARG;
   if (!is_permutation(order, cur_seq) || !is_permutation(order, new_seq)) return LNT_BAD_SEQ;
@@ -146,6 +147,12 @@ int make_rekey_params(int order, const int64_t* dims, const int32_t* cur_seq,
   for (int i = 0; i < order; ++i) pow2 = pow2 && ((u64)dims[i] & ((u64)dims[i] - 1)) == 0;
   out->pow2 = pow2 ? 1 : 0;
   for (int i = 0; i < LNT_MAX_ORDER; ++i) out->field[i] = 0;
+  bool short_modes = true;
+  for (int i = 0; i < order; ++i) {
+    short_modes = short_modes && dims[i] < ((int64_t)1 << 31);
+    out->inv[i] = 1.0 / (double)out->acc[i].d;
+  }
+  out->narrow = total <= ((unsigned __int128)1 << 31) ? 1 : total <= ((unsigned __int128)1 << 52) && short_modes ? 2 : 0;
   if (pow2) {
     for (int i = 0; i < order; ++i) {
       const u32 src = (u32)__builtin_ctzll(out->acc[i].d);

@@ -114,13 +114,13 @@ struct Divider {
   u64 d;      // divisor
   u64 magic;  // 0 => power of two
   u32 shift;  // log2(d) for powers of two, l-1 otherwise
-  u32 pad;
+  u32 magic32;  // the same m for 32-bit n and d < 2^32: floor(2^32 (2^l - d) / d) + 1
 };
 
 inline Divider make_divider(u64 d) {
   Divider r;
   r.d = d;
-  r.pad = 0;
+  r.magic32 = 0;
   if ((d & (d - 1)) == 0) {  // power of two (d >= 1)
     r.magic = 0;
     r.shift = (u32)__builtin_ctzll(d);
@@ -131,6 +131,7 @@ inline Divider make_divider(u64 d) {
   unsigned __int128 num = (unsigned __int128)diff << 64;
   r.magic = (u64)(num / d) + 1ull;
   r.shift = l - 1u;
+  if (d < (1ull << 32)) r.magic32 = (u32)(((diff << 32) / d) + 1ull);  // (l <= 32, diff < d)
   return r;
 }
 
@@ -148,6 +149,13 @@ __host__ __device__ __forceinline__ u64 divide(u64 n, const Divider& dv) {
   return (t + ((n - t) >> 1)) >> dv.shift;
 }
 
+// n / d for 32-bit n and a Divider with d <= 2^31.
+__device__ __forceinline__ u32 divide32(u32 n, const Divider& dv) {
+  if (dv.magic == 0) return n >> dv.shift;
+  const u32 t = __umulhi(dv.magic32, n);
+  return (t + ((n - t) >> 1)) >> dv.shift;
+}
+
 // ---------------------------------------------------------------------------
 // Re-keying (mixed-radix decode under the current sequence, encode under the
 // new one).  Same arithmetic as create_shuffle_needs + reShuffleLinearIndex
@@ -158,9 +166,11 @@ __host__ __device__ __forceinline__ u64 divide(u64 n, const Divider& dv) {
 struct RekeyParams {
   int order;        // 0 or 1 => identity
   int pow2;         // every extent a power of two: `field` holds the bit-field moves
+  int narrow;       // 1: keys below 2^31, 32-bit arithmetic; 2: keys below 2^52 and extents below 2^31, `inv`
   Divider acc[LNT_MAX_ORDER];  // cumulative extents, current order
   u64 mult[LNT_MAX_ORDER];     // new stride of the mode at current position i
   u32 field[LNT_MAX_ORDER];    // pow2: source shift | bits << 8 | destination shift << 16
+  double inv[LNT_MAX_ORDER];   // narrow == 2: 1 / acc
 };
 
 // With power-of-two extents the re-key is a permutation of bit fields: the
@@ -197,6 +207,103 @@ __host__ __device__ __forceinline__ u64 rekey(u64 k, const RekeyParams& p) {
     k -= q * p.acc[i].d;
   }
   return out + k * p.mult[0];
+}
+
+// Re-keys I keys in place (those whose bit is set in `use`): the loop over the
+// modes is outside the one over the keys, so that the code stays small
+// whatever the order.
+template <int I>
+__device__ __forceinline__ void rekey_items(u64 (&k)[I], const RekeyParams& p, u32 use) {
+  if (p.order <= 1 || use == 0u) return;
+  u64 out[I];
+#pragma unroll
+  for (int j = 0; j < I; ++j) out[j] = 0;
+  if (p.pow2) {
+#pragma unroll 1
+    for (int m = 0; m < p.order; ++m) {
+      const u32 f = p.field[m];
+      const u32 from = f & 63u, to = (f >> 16) & 63u;
+      const u64 mask = (1ull << ((f >> 8) & 63u)) - 1ull;
+#pragma unroll
+      for (int j = 0; j < I; ++j) out[j] |= ((k[j] >> from) & mask) << to;
+    }
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) k[j] = out[j];
+    return;
+  }
+  u64 high = 0;
+#pragma unroll
+  for (int j = 0; j < I; ++j) high |= use & (1u << j) ? k[j] : 0ull;
+  if (p.narrow == 1 && (high >> 32) == 0) {
+    // 32 bits: six instructions per mode and key instead of some 28
+    u32 r[I], o[I];
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      r[j] = (u32)k[j];
+      o[j] = 0;
+    }
+#pragma unroll 1
+    for (int m = p.order - 1; m >= 1; --m) {
+      const Divider dv = p.acc[m];
+      const u32 mult = (u32)p.mult[m], d = (u32)dv.d;
+#pragma unroll
+      for (int j = 0; j < I; ++j) {
+        const u32 q = divide32(r[j], dv);
+        o[j] += q * mult;
+        r[j] -= q * d;
+      }
+    }
+    const u32 m0 = (u32)p.mult[0];
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) k[j] = (u64)(o[j] + r[j] * m0);
+    return;
+  }
+  if (p.narrow == 2 && (high >> 52) == 0) {
+    // k is exact as a double and k / acc < 2^31 is at most one unit of its
+    // nearest integer away: round the product with 1 / acc, and correct
+    constexpr double kTwo52 = 4503599627370496.0;
+#pragma unroll 1
+    for (int m = p.order - 1; m >= 1; --m) {
+      const u64 d = p.acc[m].d, mult = p.mult[m];
+      const double inv = p.inv[m];
+#pragma unroll
+      for (int j = 0; j < I; ++j)
+        if (use & (1u << j)) {
+          const double x = __longlong_as_double((long long)(k[j] | 0x4330000000000000ull)) - kTwo52;
+          u32 q = (u32)__double2loint(fma(x, inv, kTwo52));
+          u64 rem = k[j] - q * d;
+          if ((long long)rem < 0) {
+            rem += d;
+            --q;
+          }
+          out[j] += q * mult;
+          k[j] = rem;
+        }
+    }
+    const u64 m0 = p.mult[0];
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) k[j] = out[j] + k[j] * m0;
+    return;
+  }
+#pragma unroll 1
+  for (int m = p.order - 1; m >= 1; --m) {
+    const Divider dv = p.acc[m];
+    const u64 mult = p.mult[m];
+#pragma unroll
+    for (int j = 0; j < I; ++j)
+      if (use & (1u << j)) {
+        const u64 q = divide(k[j], dv);
+        out[j] += q * mult;
+        k[j] -= q * dv.d;
+      }
+  }
+  const u64 m0 = p.mult[0];
+#pragma unroll
+  for (int j = 0; j < I; ++j)
+    if (use & (1u << j)) k[j] = out[j] + k[j] * m0;
 }
 
 // Builds RekeyParams; returns an lnt_status.

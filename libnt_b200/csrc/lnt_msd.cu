@@ -100,47 +100,6 @@ __device__ __forceinline__ void count16(u32* sh, u32 b, const MsdCtrl& c) {
   }
 }
 
-// Re-keys I keys in place (those whose bit is set in `use`): the loop over the
-// modes is outside the one over the keys, so that the code stays small
-// whatever the order.
-template <int I>
-__device__ __forceinline__ void rekey_items(u64 (&k)[I], const RekeyParams& p, u32 use) {
-  if (p.order <= 1 || use == 0u) return;
-  u64 out[I];
-#pragma unroll
-  for (int j = 0; j < I; ++j) out[j] = 0;
-  if (p.pow2) {
-#pragma unroll 1
-    for (int m = 0; m < p.order; ++m) {
-      const u32 f = p.field[m];
-      const u32 from = f & 63u, to = (f >> 16) & 63u;
-      const u64 mask = (1ull << ((f >> 8) & 63u)) - 1ull;
-#pragma unroll
-      for (int j = 0; j < I; ++j) out[j] |= ((k[j] >> from) & mask) << to;
-    }
-#pragma unroll
-    for (int j = 0; j < I; ++j)
-      if (use & (1u << j)) k[j] = out[j];
-    return;
-  }
-#pragma unroll 1
-  for (int m = p.order - 1; m >= 1; --m) {
-    const Divider dv = p.acc[m];
-    const u64 mult = p.mult[m];
-#pragma unroll
-    for (int j = 0; j < I; ++j)
-      if (use & (1u << j)) {
-        const u64 q = divide(k[j], dv);
-        out[j] += q * mult;
-        k[j] -= q * dv.d;
-      }
-  }
-  const u64 m0 = p.mult[0];
-#pragma unroll
-  for (int j = 0; j < I; ++j)
-    if (use & (1u << j)) k[j] = out[j] + k[j] * m0;
-}
-
 // Loads I keys at positions base + j * stride + tid (those below `end`; 0
 // beyond) of the concatenated source and re-keys them.
 template <int I>

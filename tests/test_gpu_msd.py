@@ -85,3 +85,30 @@ def test_sort_pairs_bucketed(cuda, torch, n, max_key, kind, inplace):
     np.testing.assert_array_equal(to_host(k, np.uint64), keys[at])
     np.testing.assert_array_equal(to_host(v), vals[at])
     assert cuda.device_status() == 0
+
+
+# extents whose products lie on either side of the limits of the 32-bit and
+# the double-precision re-key: 2^31, 2^52, a mode of 2^31 and more
+@pytest.mark.parametrize("dims", [[1291, 1291, 1289], [1291, 1290, 1290], [46341, 46341], [1, 2147483647, 1],
+                                  [2147483647, 2097151], [2147483648, 3, 5], [67108859, 67108859], [94906265, 94906265],
+                                  [7, 11, 13, 17, 19, 23, 29, 31, 37], [3, 5, 1 << 40]])
+def test_rekeyed_sort_limits(cuda, torch, dims):
+    import libnt_b200 as L
+    rng = np.random.default_rng(len(dims))
+    total = int(np.prod([int(d) for d in dims], dtype=object))
+    n = 6001
+    keys = rng.integers(0, total, n, dtype=np.uint64)
+    keys[:3] = 0, total - 1, total // 2
+    # keys at a mode's boundaries: quotients with remainders 0 and d - 1
+    keys[3:1000] = np.minimum(keys[3:1000] // np.uint64(dims[0]) * np.uint64(dims[0]), np.uint64(total - 1))
+    keys[1000:2000] = np.minimum(keys[1000:2000] // np.uint64(dims[0]) * np.uint64(dims[0]) + np.uint64(dims[0] - 1),
+                                 np.uint64(total - 1))
+    vals = rng.uniform(-1, 1, n)
+    order = list(range(len(dims)))
+    spec = L.RekeySpec.make(dims, order, order[::-1])
+    k, v = cuda.permute_sort(to_dev(keys, torch), to_dev(vals, torch), max_key=total, rekey=spec)
+    want = oracle.rekey(keys, dims, order, order[::-1])
+    at = np.argsort(want, kind="stable")
+    np.testing.assert_array_equal(to_host(k, np.uint64), want[at])
+    np.testing.assert_array_equal(to_host(v), vals[at])
+    assert cuda.device_status() == 0
