@@ -381,42 +381,45 @@ __global__ void __launch_bounds__(P::kThreads, P::kMinBlocks)
   }
 }
 
+__device__ __forceinline__ u64 word_of(const ulonglong2& r) { return r.x; }
+__device__ __forceinline__ u64 word_of(u64 w) { return w; }
+
 // Sorts the records s_r[0, cap) by word in place (cap = BT * ITEMS; the unused
 // ones hold ~0): ITEMS records per thread by odd-even transposition, then
 // merge rounds over doubling groups of threads, each thread finding its output
 // range by a merge-path search.
-template <class G>
-__device__ __noinline__ void bucket_merge_sort(ulonglong2* s_r) {
-  constexpr int I = G::kItems;
+template <int BT, int I, class R>
+__device__ __noinline__ void bucket_merge_sort(R* s_r) {
   const int tid = threadIdx.x;
-  ulonglong2 x[I];
+  R x[I];
 #pragma unroll
   for (int j = 0; j < I; ++j) x[j] = s_r[tid * I + j];
 #pragma unroll
   for (int r = 0; r < I; ++r)
 #pragma unroll
     for (int j = r & 1; j + 1 < I; j += 2) {
-      const ulonglong2 p = x[j], q = x[j + 1];
-      x[j] = p.x < q.x ? p : q;
-      x[j + 1] = p.x < q.x ? q : p;
+      const R p = x[j], q = x[j + 1];
+      const bool lt = word_of(p) < word_of(q);
+      x[j] = lt ? p : q;
+      x[j + 1] = lt ? q : p;
     }
 #pragma unroll
   for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
-  for (int g = 1; g < G::kBT; g <<= 1) {  // merge runs of g * I records
+  for (int g = 1; g < BT; g <<= 1) {  // merge runs of g * I records
     __syncthreads();
     const int first = (tid / (2 * g)) * 2 * g * I;
-    const ulonglong2* a = s_r + first;
-    const ulonglong2* b = a + g * I;
+    const R* a = s_r + first;
+    const R* b = a + g * I;
     const int len = g * I, d = (tid % (2 * g)) * I;
     int lo = d > len ? d - len : 0, hi = d < len ? d : len;
     while (lo < hi) {
       const int m = (lo + hi) >> 1;
-      if (a[m].x <= b[d - 1 - m].x) lo = m + 1; else hi = m;
+      if (word_of(a[m]) <= word_of(b[d - 1 - m])) lo = m + 1; else hi = m;
     }
     int ia = lo, ib = d - lo;
 #pragma unroll
     for (int j = 0; j < I; ++j) {
-      const bool ta = ib >= len || (ia < len && a[ia].x <= b[ib].x);
+      const bool ta = ib >= len || (ia < len && word_of(a[ia]) <= word_of(b[ib]));
       x[j] = ta ? a[ia] : b[ib];
       ia += ta ? 1 : 0;
       ib += ta ? 0 : 1;
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
       }
     }
   } else {
-    bucket_merge_sort<G>(s_r);
+    bucket_merge_sort<G::kBT, G::kItems>(s_r);
     if (FOLD) {
       for (u32 p = tid; p < cnt; p += BT) {
         const u64 low = s_r[p].x >> ib;
@@ -717,6 +720,339 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
   }
 }
 
+// ---- small sorts: one cluster, one launch --------------------------------------
+// Up to 20480 pairs.  Every CTA of a cluster of C reads all keys and keeps those
+// of its own range (the c-th part of [0, max_key)), so that it knows without
+// asking how many lie before; a single CTA could hold all pairs, whatever their
+// distribution.  It sorts its words (key << 15 | index) in shared memory as the
+// bucket kernel does (a merge sort when a sub-bucket is crowded), fetches their
+// values, and writes once the whole cluster has read its input (the output may
+// be the input).  FOLD exchanges the CTAs' output counts through distributed
+// shared memory.  Bound by latency (B200, replayed in a graph,
+// 20 to 41 key bits): 2048 pairs 8-10 us, 10,000 14.5, 20,000 18.6, against 20.6
+// to 22.7 us for histogram, partition, buckets and the skipped path behind them;
+// one CTA alone takes 12.5, 20.6 and 33 us.
+constexpr int kOneThreads = 1024, kOneItems = 20, kOneCap = kOneThreads * kOneItems;
+constexpr int kOneIb = 15;       // index bits (kOneCap < 2^15)
+constexpr int kOneSubBits = 15;  // 2^15 sub-buckets: 8 count words per thread
+constexpr int kOneSubWords = 1 << (kOneSubBits - 2);
+constexpr int kOneGroups = kOneCap / 32;
+constexpr size_t kOneSmem = (size_t)kOneCap * 8 + (size_t)kOneSubWords * 6 + (size_t)kOneGroups * 12 + 64 * 4;
+static_assert(kOneSubWords == 8 * kOneThreads, "eight count words per thread");
+
+__device__ __forceinline__ u32 cluster_rank() {
+  u32 r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+  cluster_arrive();
+  cluster_wait();
+}
+// *(p in the shared memory of CTA `rank`) = v
+__device__ __forceinline__ void st_cluster(u32* p, u32 rank, u32 v) {
+  u32 at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(at)
+               : "r"((u32)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+}
+
+// Exclusive sum over the CTA (kOneThreads threads); s: 32 words.
+__device__ __forceinline__ u32 one_sum(u32 v, u32* s, u32* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  u32 inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s[warp] = inc;
+  __syncthreads();
+  u32 w = s[lane];  // every warp scans the warps' sums
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 t = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += t;
+  }
+  *total = __shfl_sync(0xffffffffu, w, 31);
+  const u32 before = __shfl_sync(0xffffffffu, w, warp == 0 ? 0 : warp - 1);
+  return (warp == 0 ? 0u : before) + inc - v;
+}
+
+template <bool FOLD>
+__global__ void __launch_bounds__(kOneThreads, 1)
+    small_sort_kernel(const PairSource src, u32 n, int key_bits, u64 width, int sshift, u32 C, int skip_zero_heads,
+                      u64* out_k, double* out_v, u64* d_nout) {
+  constexpr int BT = kOneThreads, I = kOneItems, ib = kOneIb;
+  extern __shared__ __align__(16) unsigned char smem[];
+  u64* s_w = reinterpret_cast<u64*>(smem);
+  u32* s_cnt = reinterpret_cast<u32*>(s_w + kOneCap);            // sub-bucket counts, four to a word
+  unsigned short* s_base = reinterpret_cast<unsigned short*>(s_cnt + kOneSubWords);
+  u32* s_head = reinterpret_cast<u32*>(s_base + kOneSubWords);   // per 32 positions: first of their runs
+  u32* s_kept = s_head + kOneGroups;
+  u32* s_pre = s_kept + kOneGroups;
+  u32* s_misc = s_pre + kOneGroups;  // [0, 32) sums, [40] crowded, [41] kept here, [42] before, [48, 56) CTA totals
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const u32 le = lane == 31 ? ~0u : (2u << lane) - 1u;
+  const u32 rank = C > 1 ? cluster_rank() : 0u;
+  if (FOLD && C > 1) cluster_arrive();  // (this CTA runs: its shared memory may be written to)
+  const u64 kmask = (1ull << key_bits) - 1ull;
+  const u64 first_key = width * rank, end_key = rank + 1 == C ? ~0ull : first_key + width;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s_cnt[j * BT + tid] = 0;
+  if (tid >= 40 && tid < 43) s_misc[tid] = 0;
+  __syncthreads();
+  // ---- this CTA's words, in any order; how many keys lie before them ----------
+  u64 high = 0;
+  u32 before = 0;
+#pragma unroll 1
+  for (u32 base = 0; base < n; base += 5 * BT) {
+    u64 k[5];
+    source_keys<5>(src, base, (u32)BT, n, k);
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const u32 p = base + j * BT + tid;
+      high |= k[j] & ~kmask;
+      const u64 key = k[j] & kmask;
+      const bool mine = p < n && key >= first_key && key < end_key;
+      before += p < n && key < first_key ? 1u : 0u;
+      const u32 m = __ballot_sync(0xffffffffu, mine);
+      if (m == 0u) continue;
+      u32 at = 0;
+      if (lane == 0) at = atomicAdd(&s_misc[41], __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (mine) s_w[at + __popc(m & (le >> 1))] = (key << ib) | p;
+    }
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0 && before) atomicAdd(&s_misc[42], before);
+  // keys with bits above the sorted ones keep them: they are read again below
+  const bool wide = __syncthreads_or(high != 0) != 0;
+  const u32 cnt = s_misc[41], start = s_misc[42];
+  const int items = (int)((cnt + BT - 1) / BT);  // (uniform; a handful, all only when every key is here)
+  u64 w[I];
+  u32 pos[I / 2], most = 0;
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 p = j * BT + tid;
+    w[j] = p < cnt ? s_w[p] : ~0ull;
+    u32 slot = 0;
+    if (p < cnt) {
+      const u32 sub = min((u32)(((w[j] >> ib) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1));
+      const u32 sh = 8u * (sub & 3u);
+      slot = (atomicAdd(&s_cnt[sub >> 2], 1u << sh) >> sh) & 0xFFu;
+    }
+    pos[j / 2] = j & 1 ? pos[j / 2] | (slot << 16) : slot;
+    most = max(most, slot);
+  }
+  if (most >= (u32)kSubMax) s_misc[40] = 1;  // crowded: the counts may have run over, and are not used
+  __syncthreads();
+  {  // records before every count word
+    u32 c8[8], sum = 0, total;
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&s_cnt[tid * 8 + j]);
+      c8[j] = __dp4a(q.x, 0x01010101u, 0u);
+      c8[j + 1] = __dp4a(q.y, 0x01010101u, 0u);
+      c8[j + 2] = __dp4a(q.z, 0x01010101u, 0u);
+      c8[j + 3] = __dp4a(q.w, 0x01010101u, 0u);
+      sum += c8[j] + c8[j + 1] + c8[j + 2] + c8[j + 3];
+    }
+    u32 run = one_sum(sum, s_misc, &total);
+    u32 pk[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const u32 lo = run;
+      run += c8[2 * j];
+      pk[j] = (lo & 0xFFFFu) | (run << 16);
+      run += c8[2 * j + 1];
+    }
+    *reinterpret_cast<uint4*>(&s_base[tid * 8]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  }
+  __syncthreads();
+  if (s_misc[40] == 0) {
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      if (j >= items) break;
+      if (j * BT + tid < cnt) {
+        const u32 sub = min((u32)(((w[j] >> ib) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1));
+        const u32 sh = 8u * (sub & 3u), c4 = s_cnt[sub >> 2];
+        s_w[s_base[sub >> 2] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u) +
+            ((pos[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] = w[j];
+      }
+    }
+    __syncthreads();
+    u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const u32 gt = __vcmpgtu4(s_cnt[j * BT + tid], 0x01010101u) & 0x08040201u;
+      todo |= ((gt | (gt >> 8) | (gt >> 16) | (gt >> 24)) & 0xFu) << (4 * j);
+    }
+    while (todo) {  // insertion sort of a sub-bucket (mostly two words)
+      const int i = __ffs(todo) - 1, sh = 8 * (i & 3);
+      todo &= todo - 1u;
+      const u32 c4 = s_cnt[(i >> 2) * BT + tid];
+      u64* r = s_w + s_base[(i >> 2) * BT + tid] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
+      const int k = (int)((c4 >> sh) & 0xFFu);
+      for (int x = 1; x < k; ++x) {
+        const u64 a = r[x];
+        int q = x;
+        for (; q > 0; --q) {
+          const u64 y = r[q - 1];
+          if (y < a) break;
+          r[q] = y;
+        }
+        if (q != x) r[q] = a;
+      }
+    }
+  } else {
+    for (u32 p = cnt + tid; p < (u32)kOneCap; p += BT) s_w[p] = ~0ull;
+    __syncthreads();
+    bucket_merge_sort<BT, I>(s_w);
+  }
+  __syncthreads();
+  // ---- the words by position, and their values ----------------------------------
+  double v[I];
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 p = j * BT + tid;
+    w[j] = p < cnt ? s_w[p] : 0ull;
+  }
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 i = (u32)w[j] & ((1u << ib) - 1u);
+    v[j] = 0.0;
+    if (j * BT + tid < cnt) v[j] = i < src.na ? __ldcs(src.av + i) : src.bscale * __ldcs(src.bv + (i - src.na));
+  }
+  if (wide) {  // (rare) the whole keys in the words' place
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      if (j >= items) break;
+      const u32 i = (u32)w[j] & ((1u << ib) - 1u);
+      if (j * BT + tid < cnt) {
+        w[j] = i < src.na ? rekey(src.ak[i], src.ra) : rekey(src.bk[i - src.na], src.rb);
+        s_w[j * BT + tid] = w[j];
+      }
+    }
+    __syncthreads();
+  }
+  const int kshift = wide ? 0 : ib;
+  if (!FOLD) {
+    if (C > 1) cluster_sync();  // everyone has read the input, which the output may be
+    else __syncthreads();
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      if (j >= items) break;
+      const u32 p = j * BT + tid;
+      if (p < cnt) {
+        out_k[start + p] = w[j] >> kshift;
+        out_v[start + p] = v[j];
+      }
+    }
+    return;
+  }
+  // ---- fold runs of equal keys in input order: into the value of the first -------
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 p = j * BT + tid;
+    const u32 m = __ballot_sync(0xffffffffu, p < cnt && (p == 0 || (s_w[p - 1] >> kshift) != (w[j] >> kshift)));
+    if (lane == 0) s_head[j * (BT / 32) + warp] = m;
+  }
+  __syncthreads();
+  double* s_v = reinterpret_cast<double*>(s_w);  // the values in the words' place
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    if (j * BT + tid < cnt) s_v[j * BT + tid] = v[j];
+  }
+  __syncthreads();
+  const u32 groups = (u32)items * (BT / 32);
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 p = j * BT + tid, g = j * (BT / 32) + warp;
+    bool kept = false;
+    if (p < cnt && (s_head[g] >> lane & 1u)) {
+      bool anynz = v[j] != 0.0;
+      for (u32 q = p + 1; q < cnt && !(s_head[q >> 5] >> (q & 31) & 1u); ++q) {
+        const double y = s_v[q];
+        v[j] += y;
+        anynz |= y != 0.0;
+      }
+      kept = !skip_zero_heads || anynz || start + p == 0;
+    }
+    const u32 m = __ballot_sync(0xffffffffu, kept);
+    if (lane == 0) s_kept[g] = m;
+  }
+  __syncthreads();
+  u32 total;
+  const u32 at = one_sum((u32)tid < groups ? __popc(s_kept[tid]) : 0u, s_misc, &total);
+  if ((u32)tid < groups) s_pre[tid] = at;
+  u32 off = 0;
+  if (C > 1) {
+    cluster_wait();
+    if ((u32)tid < C) st_cluster(&s_misc[48 + rank], (u32)tid, total);
+    cluster_sync();
+    u32 all = 0;
+    for (u32 q = 0; q < C; ++q) {
+      off += q < rank ? s_misc[48 + q] : 0u;
+      all += s_misc[48 + q];
+    }
+    if (rank == 0 && tid == 0) *d_nout = all;
+  } else {
+    if (tid == 0) *d_nout = total;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    if (j >= items) break;
+    const u32 g = j * (BT / 32) + warp, m = s_kept[g];
+    if (m >> lane & 1u) {
+      const u32 o = off + s_pre[g] + __popc(m & (le >> 1));
+      out_k[o] = w[j] >> kshift;
+      out_v[o] = v[j];
+    }
+  }
+}
+
+template <bool FOLD>
+int launch_small_sort(const MsdPlan& p, const PairSource& src, const MsdFold* fold, u64* out_k, double* out_v,
+                      cudaStream_t s) {
+  // CTAs of about 2560 pairs
+  u32 C = 1;
+  while (C < 8 && p.n > C * 2560) C *= 2;
+  const u64 width = (p.max_key + C - 1) / C;
+  const int sshift = std::max(0, key_bits_for(width) - kOneSubBits);
+  auto kern = small_sort_kernel<FOLD>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOneSmem) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(kOneThreads);
+  cfg.dynamicSmemBytes = kOneSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  ProfScope prof(FOLD ? "small_sort_collect" : "small_sort", s);
+  if (cudaLaunchKernelEx(&cfg, kern, src, p.n, p.key_bits, width, sshift, C, FOLD ? fold->skip_zero_heads : 0, out_k,
+                         out_v, FOLD ? fold->d_nout : (u64*)nullptr) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  count_launch();
+  return launch_status();
+}
+
 template <bool FIRST>
 int launch_partition(const MsdPlan& p, const PairSource& src, const ulonglong2* in, ulonglong2* out, u32 tiles,
                      int dshift, int dbits, int nseg, const MsdCtrl& c, cudaStream_t s) {
@@ -762,8 +1098,14 @@ void top_fields(RekeyParams* r, int shift) {
 MsdPlan make_msd_plan(size_t n, u64 max_key) {
   MsdPlan p;
   p.n = (u32)n;
+  p.max_key = max_key;
   p.key_bits = key_bits_for(max_key);
-  if (n < kMinPairs || n >= (1u << 30) || getenv("LNT_NO_BUCKETS") || getenv("LNT_SORT_VARIANT")) return p;
+  if (n == 0 || n >= (1u << 30) || getenv("LNT_NO_BUCKETS") || getenv("LNT_SORT_VARIANT")) return p;
+  if (n <= (size_t)kOneCap && p.key_bits > 0 && p.key_bits + kOneIb <= 64) {
+    p.ok = p.single = true;
+    return p;
+  }
+  if (n < kMinPairs) return p;
   const char* force = getenv("LNT_BUCKET_SMALL");
   int bestT = 99;
   for (int large = 0; large < 2; ++large) {
@@ -811,6 +1153,10 @@ MsdPlan make_msd_plan(size_t n, u64 max_key) {
 }
 
 int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void* ctrl, const MsdFold* fold, u64* out_k, double* out_v, u32* gate, cudaStream_t s) {
+  if (p.single) {
+    return fold ? launch_small_sort<true>(p, src, fold, out_k, out_v, s)
+                : launch_small_sort<false>(p, src, fold, out_k, out_v, s);
+  }
   unsigned char* w = static_cast<unsigned char*>(ctrl);
   MsdCtrl c;
   c.counts = reinterpret_cast<u32*>(w + p.off_counts);
@@ -873,7 +1219,7 @@ int run_pair_sort(const PairSort& p, const PairSource& src, u64* out_k, double* 
   if (p.msd.ok) {
     gate = reinterpret_cast<u32*>(static_cast<unsigned char*>(ctrl) + p.ctrl_bytes - 256);
     const int st = run_msd_sort(p.msd, src, b, a, ctrl, nullptr, out_k, out_v, gate, s);
-    if (st != LNT_OK) return st;
+    if (st != LNT_OK || p.msd.single) return st;
   }
   u64* ak = static_cast<u64*>(a);
   double* av = reinterpret_cast<double*>(static_cast<unsigned char*>(a) + p.a_bytes / 2);

@@ -10,8 +10,10 @@ namespace lnt {
 // name the bucket, `shift` bits remain below them.
 struct MsdPlan {
   bool ok = false;   // the bucketed path applies
+  bool single = false;  // one cluster does it all (small_sort_kernel): no scratch, no gate, no path behind it
   bool large = false;  // bucket geometry: 512-thread CTAs of up to 5120 pairs, else 256 threads, 2560 pairs
   u32 n = 0;
+  u64 max_key = 0;
   int key_bits = 0;
   int shift = 0;     // key bits below the bucket bits
   int T = 0;         // bucket bits

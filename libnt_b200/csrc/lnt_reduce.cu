@@ -513,7 +513,7 @@ int lnt_sort_reduce(const uint64_t* a_keys, const double* a_vals, size_t na, con
     u32* g = reinterpret_cast<u32*>(w + L.off_gate);
     const MsdFold fold{skip_zero_heads, (u64*)d_nout};
     st = run_msd_sort(L.msd, src, k1, k0, w + L.off_ctrl, &fold, (u64*)keys_out, vals_out, g, s);
-    if (st != LNT_OK) return st;
+    if (st != LNT_OK || L.msd.single) return st;
     gate = g;
   }
   st = run_sort(L.plan, gated_source(src, gate, 1), k0, v0, k1, v1, w + L.off_ctrl, s);

@@ -717,7 +717,7 @@ int lnt_sort_pairs(const uint64_t* keys_in, const double* vals_in, uint64_t* key
     gate = reinterpret_cast<u32*>(ws + L.sort.ctrl_bytes - 256);
     const int st = run_msd_sort(L.sort.msd, src, ws + L.off_b, ws + L.off_a, ws, nullptr, (u64*)keys_out, vals_out,
                                 gate, s);
-    if (st != LNT_OK) return st;
+    if (st != LNT_OK || L.sort.msd.single) return st;
     src = gated_source(src, gate, 1);
   }
   if (lsd.passes == 0) return LNT_OK;  // all keys equal: input order is the stable order

@@ -543,7 +543,7 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
     void* x = E.sort.msd.passes == 2 ? po : nullptr;
     void* y = E.sort.msd.passes == 2 ? pe : po;
     st = run_msd_sort(E.sort.msd, src, x, y, ctrl, &fold, (u64*)c_keys, c_vals, gate, cs);
-    if (st != LNT_OK) return st;
+    if (st != LNT_OK || E.sort.msd.single) return st;
   }
   u64* k0 = reinterpret_cast<u64*>(w + E.off_a);
   double* v0 = reinterpret_cast<double*>(w + E.off_a + E.sort.a_bytes / 2);

@@ -112,3 +112,30 @@ def test_rekeyed_sort_limits(cuda, torch, dims):
     np.testing.assert_array_equal(to_host(k, np.uint64), want[at])
     np.testing.assert_array_equal(to_host(v), vals[at])
     assert cuda.device_status() == 0
+
+
+# one cluster of 1, 2, 4, 8 CTAs, and the first size beyond it
+@pytest.mark.parametrize("kind", ["uniform", "sorted", "upper", "one_key", "repeated"])
+@pytest.mark.parametrize("max_key", [7, 5000, 3 * 10 ** 6, (1 << 49) - 5])
+@pytest.mark.parametrize("n", [1, 33, 2560, 2561, 5121, 10241, 20479, 20480, 20481])
+def test_small_sorts(cuda, torch, n, max_key, kind):
+    rng = np.random.default_rng(n + max_key % 1000)
+    keys = _keys(rng, n, max_key, kind if kind in ("sorted", "upper") else "uniform")
+    if kind == "one_key":
+        keys[rng.random(n) < 0.9] = keys[0]
+    if kind == "repeated":
+        keys = keys[rng.integers(0, max(1, n // 3), n)]
+    vals = rng.uniform(-1, 1, n)
+    vals[rng.random(n) < 0.3] = 0.0
+    k, v = cuda.sort_pairs(to_dev(keys, torch), to_dev(vals, torch), max_key=max_key)
+    at = np.argsort(keys, kind="stable")
+    np.testing.assert_array_equal(to_host(k, np.uint64), keys[at])
+    np.testing.assert_array_equal(to_host(v), vals[at])
+    for skip in (True, False):
+        k, v = cuda.sort_reduce(to_dev(keys[: n // 2], torch), to_dev(vals[: n // 2], torch),
+                                to_dev(keys[n // 2:], torch), to_dev(vals[n // 2:], torch), max_key=max_key,
+                                skip_zero_heads=skip)
+        ek, ev, ea = oracle.collect_duplicates(keys[at], vals[at], skip_zero_heads=skip, with_abs=True)
+        np.testing.assert_array_equal(to_host(k, np.uint64), ek)
+        assert rel_ok(to_host(v), ev, ea)
+    assert cuda.device_status() == 0
