@@ -378,7 +378,7 @@ def lattice_mult(a_keys, a_vals, b_keys, b_vals, h: int, w: int, wB: int, d: int
     b = C.c_size_t(0)
     _check(lib().lnt_lattice_mult_plan_workspace(C.byref(A), C.byref(B), C.byref(b)), "lnt_lattice_mult_plan_workspace")
     plan = workspace(b.value, dev)
-    counts = torch.zeros(2, dtype=torch.int64, device=dev)
+    counts = torch.empty(2, dtype=torch.int64, device=dev)
     _check(lib().lnt_lattice_mult_plan(C.byref(A), C.byref(B), _ptr(plan), plan.numel(), _ptr(counts), _stream()),
            "lnt_lattice_mult_plan")
     products, cap = (int(x) for x in counts.tolist())
@@ -387,7 +387,7 @@ def lattice_mult(a_keys, a_vals, b_keys, b_vals, h: int, w: int, wB: int, d: int
     ws = workspace(b.value, dev)
     ck = torch.empty(max(cap, 1), dtype=torch.int64, device=dev)
     cv = torch.empty(max(cap, 1), dtype=torch.float64, device=dev)
-    nc = torch.zeros(1, dtype=torch.int64, device=dev)
+    nc = torch.empty(1, dtype=torch.int64, device=dev)
     _check(lib().lnt_lattice_mult(C.byref(A), C.byref(B), _ptr(plan), products, _ptr(ws), ws.numel(), _ptr(ck),
                                   _ptr(cv), _ptr(nc), _stream()), "lnt_lattice_mult")
     m = int(nc.item())

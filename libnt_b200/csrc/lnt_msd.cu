@@ -1208,6 +1208,10 @@ PairSort make_pair_sort(size_t n, u64 max_key) {
   p.msd = make_msd_plan(n, max_key);
   p.lsd = make_sort_plan(n, max_key, p.msd.ok);
   p.ctrl_bytes = align_up(std::max(p.lsd.ctrl_bytes, p.msd.ctrl_bytes), 256) + 256;
+  if (p.msd.single) {  // needs no scratch
+    p.ctrl_bytes = 256;
+    return p;
+  }
   p.a_bytes = 2 * align_up(n * 8, 256);
   p.b_bytes = p.msd.ok && p.msd.passes == 2 ? p.a_bytes : 0;
   return p;

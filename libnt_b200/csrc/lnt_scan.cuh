@@ -56,9 +56,11 @@ __global__ void __launch_bounds__(kThreads) scan_kernel(Get get, size_t n, unsig
   __shared__ u32 s_tile;
   __shared__ unsigned long long s_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(counter, 1u);
-  __syncthreads();
-  const u32 tile = s_tile;
+  if (ntiles > 1) {
+    if (tid == 0) s_tile = atomicAdd(counter, 1u);
+    __syncthreads();
+  }
+  const u32 tile = ntiles > 1 ? s_tile : 0u;  // (a single tile needs no control block)
   const size_t base = (size_t)tile * kTile + (size_t)tid * kItems;  // blocked: 8 consecutive per thread
   unsigned long long v[kItems];
   unsigned long long local = 0;
@@ -81,7 +83,8 @@ __global__ void __launch_bounds__(kThreads) scan_kernel(Get get, size_t n, unsig
     tot += s_warp[w];
   }
   if (warp == 0) {
-    if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = (tile == 0 ? kFlagPre : kFlagAgg) | tot;
+    if (lane == 0 && ntiles > 1)
+      *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = (tile == 0 ? kFlagPre : kFlagAgg) | tot;
     unsigned long long off = tile == 0 ? 0ull : warp_lookback(status, tile, kErrSpgemmLookback);
     if (lane == 0) {
       if (tile != 0) *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = kFlagPre | (off + tot);
@@ -116,7 +119,7 @@ int run(Get get, size_t n, unsigned long long* out, unsigned long long* d_total,
     if (d_total && cudaMemsetAsync(d_total, 0, 8, s) != cudaSuccess) return LNT_DEVICE_ERROR;
     return LNT_OK;
   }
-  if (cudaMemsetAsync(ws, 0, workspace_bytes(n), s) != cudaSuccess) return LNT_DEVICE_ERROR;
+  if (ntiles > 1 && cudaMemsetAsync(ws, 0, workspace_bytes(n), s) != cudaSuccess) return LNT_DEVICE_ERROR;
   unsigned char* w = static_cast<unsigned char*>(ws);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(w);
   u32* counter = reinterpret_cast<u32*>(w + align_up((size_t)ntiles * 8, 256));

@@ -61,14 +61,25 @@ struct Lat {
   u64 rows, cols, tabs;
 };
 
-// ptr[c] = first index whose column id (key / div) is >= c, for c in [0, ncol].
-__global__ void colptr_kernel(const u64* __restrict__ keys, u64 n, Divider div, u64 ncol,
-                              u64* __restrict__ ptr) {
-  const u64 stride = (u64)gridDim.x * blockDim.x;
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += stride) {
-    const long long prev = i == 0 ? -1ll : (long long)min(divide(keys[i - 1], div), ncol);
-    const u64 cur = i == n ? ncol : min(divide(keys[i], div), ncol);
-    for (long long c = prev + 1; c <= (long long)cur; ++c) ptr[c] = i;
+// ptr[c] = first index whose column id (key / div) is >= c, for c in [0, ncol],
+// of one operand, or of both (the blocks from `blocks_a` on: B).
+struct ColPtr {
+  const u64* keys;
+  u64 n;
+  Divider div;
+  u64 ncol;
+  u64* ptr;
+};
+
+__global__ void colptr_kernel(const ColPtr a, const ColPtr b, u32 blocks_a) {
+  const bool is_b = blockIdx.x >= blocks_a;
+  const ColPtr& c = is_b ? b : a;
+  const u64 block = is_b ? blockIdx.x - blocks_a : blockIdx.x, blocks = is_b ? gridDim.x - blocks_a : blocks_a;
+  const u64 stride = blocks * blockDim.x;
+  for (u64 i = block * blockDim.x + threadIdx.x; i <= c.n; i += stride) {
+    const long long prev = i == 0 ? -1ll : (long long)min(divide(c.keys[i - 1], c.div), c.ncol);
+    const u64 cur = i == c.n ? c.ncol : min(divide(c.keys[i], c.div), c.ncol);
+    for (long long x = prev + 1; x <= (long long)cur; ++x) c.ptr[x] = i;
   }
 }
 
@@ -233,64 +244,88 @@ __global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AC
 }
 
 // ---- SPA engine ----------------------------------------------------------
-template <bool NUMERIC>
+// One warp per output column; with few columns (BLOCK) one CTA per column, its
+// four warps sharing the accumulators: a column of 100 entries then takes one
+// round of dependent loads instead of four (100 columns: 10.4 -> 5.2 us numeric,
+// 7.4 -> 4.6 us symbolic).  The symbolic pass also counts the products.
+template <bool NUMERIC, bool BLOCK>
 __global__ void __launch_bounds__(kSpaWarps * 32) spa_kernel(Lat A, Lat B, AColumns ac, const u64* __restrict__ bptr,
                                                               u64 units, u64* __restrict__ ucount,
+                                                              unsigned long long* __restrict__ d_products,
                                                               const u64* __restrict__ uoff, u64* __restrict__ ck,
-                                                              double* __restrict__ cv) {
-  __shared__ u32 s_bits[kSpaWarps][kSpaMaxRows / 32];
-  __shared__ double s_acc[NUMERIC ? kSpaWarps : 1][NUMERIC ? kSpaMaxRows : 1];
+                                                              double* __restrict__ cv, u64* __restrict__ d_nc) {
+  constexpr int N = BLOCK ? 1 : kSpaWarps;
+  constexpr int T = BLOCK ? kSpaWarps * 32 : 32;  // threads per column
+  __shared__ u32 s_bits[N][kSpaMaxRows / 32];
+  __shared__ double s_acc[NUMERIC ? N : 1][NUMERIC ? kSpaMaxRows : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ct = BLOCK ? threadIdx.x : lane;
   const u64 h = A.rows, w = A.cols, wB = B.cols;
-  const int hw = (int)((h + 31) / 32);
-  u32* bits = s_bits[warp];
-  double* acc = s_acc[NUMERIC ? warp : 0];
-  const u64 nwarps = (u64)gridDim.x * kSpaWarps;
-  for (u64 u = (u64)blockIdx.x * kSpaWarps + warp; u < units; u += nwarps) {
+  const int hw = (int)((h + 31) / 32);  // at most 32
+  u32* bits = s_bits[BLOCK ? 0 : warp];
+  double* acc = s_acc[NUMERIC && !BLOCK ? warp : 0];
+  auto sync = [] {
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+  };
+  const u64 nteams = BLOCK ? gridDim.x : (u64)gridDim.x * kSpaWarps;
+  unsigned long long products = 0;
+  if (NUMERIC && blockIdx.x == 0 && threadIdx.x == 0) *d_nc = uoff[units];
+  for (u64 u = BLOCK ? blockIdx.x : (u64)blockIdx.x * kSpaWarps + warp; u < units; u += nteams) {
     const u64 e0 = bptr[u], e1 = bptr[u + 1];
     if (e0 == e1) {  // empty B column: no output rows
-      if (!NUMERIC && lane == 0) ucount[u] = 0;
+      if (!NUMERIC && ct == 0) ucount[u] = 0;
       continue;
     }
-    for (int i = lane; i < hw; i += 32) bits[i] = 0u;
+    for (int i = ct; i < hw; i += T) bits[i] = 0u;
     if (NUMERIC)
-      for (int i = lane; i < (int)h; i += 32) acc[i] = 0.0;
-    __syncwarp();
+      for (int i = ct; i < (int)h; i += T) acc[i] = 0.0;
+    sync();
     const u64 t = u / wB;
-    for (u64 e = e0 + lane; e < e1; e += 32) {
+    for (u64 e = e0 + ct; e < e1; e += T) {
       const u64 brow = B.keys[e] - w * u;  // B col id of this unit is u
       const u64 acol = brow + w * t;
       u64 lo, hi;
       ac.range(acol, lo, hi);
       const double beta = NUMERIC ? B.vals[e] : 0.0;
+      if (!NUMERIC) products += hi - lo;
       for (u64 x = lo; x < hi; ++x) {
         const u32 r = (u32)(A.keys[x] - acol * h);
         atomicOr(&bits[r >> 5], 1u << (r & 31));
         if (NUMERIC) atomicAdd(&acc[r], A.vals[x] * beta);
       }
     }
-    __syncwarp();
+    sync();
+    // rows before every word of 32 (each warp for itself)
+    const u32 mine = lane < hw ? __popc(bits[lane]) : 0u;
     if (!NUMERIC) {
-      u32 c = 0;
-      for (int i = lane; i < hw; i += 32) c += __popc(bits[i]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-      if (lane == 0) ucount[u] = c;
+      const u32 c = __reduce_add_sync(0xffffffffu, mine);
+      if (ct == 0) ucount[u] = c;
     } else {
-      u64 out = uoff[u];
+      u32 inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      const u64 out = uoff[u];
       const u64 colkey = h * u;  // h*(col + wB*tab)
-      for (int g = 0; g < hw; ++g) {
-        const u32 word = bits[g];
+      for (int g = BLOCK ? warp : 0; g < hw; g += BLOCK ? kSpaWarps : 1) {
+        const u32 word = bits[g], before = __shfl_sync(0xffffffffu, inc - mine, g);
         if (word & (1u << lane)) {
           const u32 r = (u32)g * 32 + lane;
-          const u64 o = out + __popc(word & ((1u << lane) - 1u));
+          const u64 o = out + before + __popc(word & ((1u << lane) - 1u));
           ck[o] = colkey + r;
           cv[o] = acc[r];
         }
-        out += __popc(word);
       }
     }
-    __syncwarp();
+    sync();
+  }
+  if (!NUMERIC) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) products += __shfl_xor_sync(0xffffffffu, products, o);
+    if (lane == 0 && products) atomicAdd(d_products, products);
   }
 }
 
@@ -350,6 +385,16 @@ PlanLayout plan_layout(const Shape& s) {
 
 bool spa_eligible(const Shape& s) { return s.h <= (u64)kSpaMaxRows && s.dense_a && s.dense_b; }
 
+// A CTA per output column up to this many columns (two waves of resident CTAs).
+u64 spa_block_units() { return (u64)sm_count() * 16; }
+
+// Products per B entry, summed up: boff[e] before entry e, the total to *d_total.
+int product_prefix(const Shape& s, const AColumns& ac, u64* boff, unsigned long long* d_total, void* ws,
+                   cudaStream_t cs) {
+  const ProductCount pc{ac, s.B.keys, make_divider(s.w), make_divider(s.wB), s.w};
+  return scan::run(pc, s.B.nnz, (unsigned long long*)boff, d_total, ws, cs, "spgemm_count");
+}
+
 enum class Engine { Spa, Esc, Tile };
 
 Engine choose_engine(const Shape& s, u64 products) {
@@ -367,23 +412,31 @@ Engine choose_engine(const Shape& s, u64 products) {
 // Workspace of the ESC engine: the products and the sort's other pairs (A, B).
 struct EscLayout {
   PairSort sort;
+  size_t pair_bytes;  // of A and of B: keys, then values
   size_t off_ctrl, off_a, off_b, off_coll, total;
 };
 
 EscLayout esc_layout(u64 products, u64 max_key) {
   EscLayout L;
   L.sort = make_pair_sort(products, max_key);
+  L.pair_bytes = 2 * align_up(products * 8, 256);
   size_t off = 0;
   L.off_ctrl = off;
   off += align_up(L.sort.ctrl_bytes, 256);
   L.off_a = off;
-  off += L.sort.a_bytes;
+  off += L.pair_bytes;
   L.off_b = off;
-  off += L.sort.a_bytes;
+  off += L.pair_bytes;
   L.off_coll = off;
   off += align_up(collect_workspace_bytes(products), 256);
   L.total = off;
   return L;
+}
+
+// The SPA engine's plan holds no product prefix; the ESC engine forced on such
+// a shape makes its own, behind its workspace.
+size_t esc_prefix_bytes(const Shape& s) {
+  return spa_eligible(s) ? align_up((s.B.nnz + 1) * 8, 256) + align_up(scan::workspace_bytes(s.B.nnz), 256) : 0;
 }
 
 // counts[1] = min(counts[0], dense): the output holds at most one entry per
@@ -427,28 +480,26 @@ int lnt_lattice_mult_plan(const lnt_lattice* a, const lnt_lattice* b, void* plan
   u64* boff = reinterpret_cast<u64*>(p + L.off_boff);
   u64* ucount = reinterpret_cast<u64*>(p + L.off_ucount);
   u64* uoff = reinterpret_cast<u64*>(p + L.off_uoff);
+  const bool spa = spa_eligible(s);
   if (s.dense_a) {
+    const ColPtr ca{s.A.keys, s.A.nnz, make_divider(s.h), s.w * s.d, aptr};
+    const ColPtr cb{s.B.keys, s.B.nnz, make_divider(s.w), L.units, bptr};
+    const u32 ga = (u32)grid_for(s.A.nnz + 1, 256), gb = spa ? (u32)grid_for(s.B.nnz + 1, 256) : 0u;
     ProfScope prof("spgemm_colptr", cs);
-    colptr_kernel<<<grid_for(s.A.nnz + 1, 256), 256, 0, cs>>>(s.A.keys, s.A.nnz, make_divider(s.h), s.w * s.d, aptr);
+    colptr_kernel<<<ga + gb, 256, 0, cs>>>(ca, cb, ga);
     count_launch();
   }
   AColumns ac{s.dense_a ? aptr : nullptr, s.A.keys, s.A.nnz, s.h};
-  ProductCount pc{ac, s.B.keys, make_divider(s.w), make_divider(s.wB), s.w};
-  // products per B entry -> prefix -> total products into d_counts[0]
-  st = scan::run(pc, s.B.nnz, (unsigned long long*)boff, (unsigned long long*)d_counts, p + L.off_scan, cs,
-                 "spgemm_count");
-  if (st != LNT_OK) return st;
-  if (spa_eligible(s)) {
-    {
-      ProfScope prof("spgemm_colptr", cs);
-      colptr_kernel<<<grid_for(s.B.nnz + 1, 256), 256, 0, cs>>>(s.B.keys, s.B.nnz, make_divider(s.w), L.units,
-                                                                 bptr);
-      count_launch();
-    }
+  if (spa) {
+    if (cudaMemsetAsync(d_counts, 0, 8, cs) != cudaSuccess) return LNT_DEVICE_ERROR;
     {
       ProfScope prof("spgemm_spa_symbolic", cs);
-      spa_kernel<false><<<grid_for(L.units * 32, kSpaWarps * 32), kSpaWarps * 32, 0, cs>>>(
-          s.A, s.B, ac, bptr, L.units, ucount, nullptr, nullptr, nullptr);
+      if (L.units <= spa_block_units())
+        spa_kernel<false, true><<<(unsigned)L.units, kSpaWarps * 32, 0, cs>>>(
+            s.A, s.B, ac, bptr, L.units, ucount, (unsigned long long*)d_counts, nullptr, nullptr, nullptr, nullptr);
+      else
+        spa_kernel<false, false><<<grid_for(L.units * 32, kSpaWarps * 32), kSpaWarps * 32, 0, cs>>>(
+            s.A, s.B, ac, bptr, L.units, ucount, (unsigned long long*)d_counts, nullptr, nullptr, nullptr, nullptr);
       count_launch();
     }
     // output rows per column -> prefix -> exact output count into d_counts[1]
@@ -456,6 +507,9 @@ int lnt_lattice_mult_plan(const lnt_lattice* a, const lnt_lattice* b, void* plan
                    p + L.off_scan, cs, "spgemm_scan");
     if (st != LNT_OK) return st;
   } else {
+    // products per B entry -> prefix -> total products into d_counts[0]
+    st = product_prefix(s, ac, boff, (unsigned long long*)d_counts, p + L.off_scan, cs);
+    if (st != LNT_OK) return st;
     capacity_kernel<<<1, 1, 0, cs>>>((u64*)d_counts, s.h * s.wB * s.d);
     count_launch();
   }
@@ -477,7 +531,7 @@ int lnt_lattice_mult_workspace(const lnt_lattice* a, const lnt_lattice* b, uint6
     return LNT_OK;
   }
   if (products >= (1ull << 30)) return LNT_UNSUPPORTED;
-  *bytes = esc_layout(products, s.h * s.wB * s.d).total;
+  *bytes = esc_layout(products, s.h * s.wB * s.d).total + esc_prefix_bytes(s);
   return LNT_OK;
 }
 
@@ -508,12 +562,14 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   if (eng == Engine::Spa) {
     {
       ProfScope prof("spgemm_spa_numeric", cs);
-      spa_kernel<true><<<grid_for(L.units * 32, kSpaWarps * 32), kSpaWarps * 32, 0, cs>>>(
-          s.A, s.B, ac, bptr, L.units, nullptr, uoff, (u64*)c_keys, c_vals);
+      if (L.units <= spa_block_units())
+        spa_kernel<true, true><<<(unsigned)L.units, kSpaWarps * 32, 0, cs>>>(
+            s.A, s.B, ac, bptr, L.units, nullptr, nullptr, uoff, (u64*)c_keys, c_vals, (u64*)d_nc);
+      else
+        spa_kernel<true, false><<<grid_for(L.units * 32, kSpaWarps * 32), kSpaWarps * 32, 0, cs>>>(
+            s.A, s.B, ac, bptr, L.units, nullptr, nullptr, uoff, (u64*)c_keys, c_vals, (u64*)d_nc);
       count_launch();
     }
-    if (cudaMemcpyAsync(d_nc, uoff + L.units, 8, cudaMemcpyDeviceToDevice, cs) != cudaSuccess)
-      return LNT_DEVICE_ERROR;
     return launch_status();
   }
   // ESC
@@ -521,13 +577,19 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   const EscLayout E = esc_layout(products, s.h * s.wB * s.d);
   unsigned char* w = static_cast<unsigned char*>(workspace);
   void* ctrl = w + E.off_ctrl;
+  if (spa_eligible(s)) {
+    u64* own = reinterpret_cast<u64*>(w + E.total);
+    st = product_prefix(s, ac, own, nullptr, w + E.total + align_up((s.B.nnz + 1) * 8, 256), cs);
+    if (st != LNT_OK) return st;
+    boff = own;
+  }
   // Pass p of the LSD sort writes buffer (passes-1-p)&1 (0 = A, the final
   // one); expand into the buffer its pass 0 does not write.
   const bool even = E.sort.lsd.passes % 2 == 0;
   unsigned char* pe = w + (even ? E.off_a : E.off_b);
   unsigned char* po = w + (even ? E.off_b : E.off_a);
   u64* ek = reinterpret_cast<u64*>(pe);
-  double* ev = reinterpret_cast<double*>(pe + E.sort.a_bytes / 2);
+  double* ev = reinterpret_cast<double*>(pe + E.pair_bytes / 2);
   {
     ProfScope prof("spgemm_expand", cs);
     expand_kernel<<<(unsigned)((products + kExpandTile - 1) / kExpandTile), kExpandThreads, 0, cs>>>(
@@ -546,9 +608,9 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
     if (st != LNT_OK || E.sort.msd.single) return st;
   }
   u64* k0 = reinterpret_cast<u64*>(w + E.off_a);
-  double* v0 = reinterpret_cast<double*>(w + E.off_a + E.sort.a_bytes / 2);
+  double* v0 = reinterpret_cast<double*>(w + E.off_a + E.pair_bytes / 2);
   u64* k1 = reinterpret_cast<u64*>(w + E.off_b);
-  double* v1 = reinterpret_cast<double*>(w + E.off_b + E.sort.a_bytes / 2);
+  double* v1 = reinterpret_cast<double*>(w + E.off_b + E.pair_bytes / 2);
   st = run_sort(E.sort.lsd, gated_source(src, gate, 1), k0, v0, k1, v1, ctrl, cs);
   if (st != LNT_OK) return st;
   return run_collect_gated(k0, v0, products, 0, (u64*)c_keys, c_vals, (u64*)d_nc, w + E.off_coll, cs, gate, 1);
@@ -651,7 +713,9 @@ int lnt_nolattice_mult_count(const lnt_lattice* a, const lnt_lattice* b, void* w
   u64* aptr = reinterpret_cast<u64*>(p + L.off_aptr);
   if (s.dense_a) {
     ProfScope prof("spgemm_colptr", cs);
-    colptr_kernel<<<grid_for(s.A.nnz + 1, 256), 256, 0, cs>>>(s.A.keys, s.A.nnz, make_divider(s.h), s.w * s.d, aptr);
+    const ColPtr ca{s.A.keys, s.A.nnz, make_divider(s.h), s.w * s.d, aptr};
+    const unsigned ga = (unsigned)grid_for(s.A.nnz + 1, 256);
+    colptr_kernel<<<ga, 256, 0, cs>>>(ca, ca, ga);
     count_launch();
   }
   AColumns ac{s.dense_a ? aptr : nullptr, s.A.keys, s.A.nnz, s.h};
