@@ -23,7 +23,11 @@
 // partners are read from there - global memory only when a run of equal keys
 // crosses the slice boundary.  Emitted elements keep merged order; their output
 // offsets come from a block scan plus a decoupled look-back over tiles.
-// Traffic: 16 B read per input pair + 16 B written per output pair.
+// A tile in which no key repeats inside an operand (checked on the staged keys)
+// needs none of the run bookkeeping: an A meets at most the B at hand, a B only
+// the A taken last (0.54 -> 0.46 ms).
+// Traffic: 16 B read per input pair + 16 B written per output pair; bound by the
+// latency of the tile's steps, the look-back a quarter of it (0.30 ms without).
 #include <algorithm>
 
 #include "lnt_msd.cuh"
@@ -54,13 +58,19 @@ __device__ __forceinline__ size_t merge_path(const u64* __restrict__ a, size_t n
   return lo;
 }
 
-// Same search over shared-memory slices.
-__device__ __forceinline__ int merge_path_smem(const u64* a, int na, const u64* b, int nb, int d) {
-  int lo = d > nb ? d - nb : 0;
-  int hi = d < na ? d : na;
+// Shared-memory place of slice element i: a thread's elements are 32 or 64
+// bytes from its neighbour's, so a spare word pair per 16 elements spreads a
+// warp's accesses over the banks (0.46 -> 0.41 ms on 20M + 12M pairs).
+__device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
+constexpr int kPadded = kTile + kTile / 16;
+
+// Same search over the padded slices (A, then B from la on).
+__device__ __forceinline__ int merge_path_smem(const u64* k, int la, int lb, int d) {
+  int lo = d > lb ? d - lb : 0;
+  int hi = d < la ? d : la;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (a[mid] <= b[d - 1 - mid])
+    if (k[pad(mid)] <= k[pad(la + d - 1 - mid)])
       lo = mid + 1;
     else
       hi = mid;
@@ -85,18 +95,20 @@ __global__ void merge_partition_kernel(const u64* __restrict__ a, size_t na, con
   splits[t] = merge_path(a, na, b, nb, min(na + nb, (size_t)t * kTile));
 }
 
-__global__ void __launch_bounds__(kThreads) merge_kernel(const u64* __restrict__ ak, const double* __restrict__ av,
+__global__ void __launch_bounds__(kThreads, 4) merge_kernel(const u64* __restrict__ ak, const double* __restrict__ av,
                                                          size_t na, const u64* __restrict__ bk,
                                                          const double* __restrict__ bv, size_t nb, int op,
                                                          u32 ntiles, const u64* __restrict__ splits,
                                                          unsigned long long* __restrict__ status,
                                                          u32* __restrict__ tile_counter, u64* __restrict__ ck,
                                                          double* __restrict__ cv, u64* __restrict__ d_nout) {
-  __shared__ u64 s_k[kTile];
-  __shared__ double s_v[kTile];
+  __shared__ u64 s_k[kPadded];
+  __shared__ double s_v[kPadded];
   __shared__ u32 s_warp[kThreads / 32];
   __shared__ u32 s_tile;
   __shared__ unsigned long long s_off;
+  __shared__ u64 s_edge[3];
+  __shared__ double s_edge_v;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
   __syncthreads();
@@ -107,73 +119,120 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const u64* __restrict__
   const size_t a0 = splits[tile], a1 = splits[tile + 1];
   const size_t b0 = d0 - a0, b1 = d1 - a1;
   const int la = (int)(a1 - a0), lb = (int)(b1 - b0);
+  if (warp == kThreads / 32 - 1) {  // what lies just outside the slices
+    if (lane == 0 && a0 > 0) s_edge[0] = ak[a0 - 1];
+    if (lane == 1 && b1 < nb) s_edge[1] = bk[b1];
+    if (lane == 2 && b1 < nb) s_edge_v = bv[b1];
+    if (lane == 3 && b0 > 0) s_edge[2] = bk[b0 - 1];
+  }
   // stage the tile's A slice then its B slice, keys and values, in shared memory
   for (int i = tid; i < la + lb; i += kThreads) {
     if (i < la) {
-      s_k[i] = __ldcs(ak + a0 + i);
-      s_v[i] = __ldcs(av + a0 + i);
+      s_k[pad(i)] = __ldcs(ak + a0 + i);
+      s_v[pad(i)] = __ldcs(av + a0 + i);
     } else {
-      s_k[i] = __ldcs(bk + b0 + (i - la));
-      s_v[i] = __ldcs(bv + b0 + (i - la));
+      s_k[pad(i)] = __ldcs(bk + b0 + (i - la));
+      s_v[pad(i)] = __ldcs(bv + b0 + (i - la));
     }
   }
   __syncthreads();
+  // a key repeated inside an operand (also across the slice's start)?
+  bool repeat = false;
+  for (int i = tid; i < la + lb; i += kThreads) {
+    const bool first = i == 0 || i == la;
+    repeat = repeat || (first ? (i < la ? a0 > 0 && s_k[pad(i)] == s_edge[0] : b0 > 0 && s_k[pad(i)] == s_edge[2])
+                              : s_k[pad(i)] == s_k[pad(i - 1)]);
+  }
   // each thread merges kItems consecutive merged positions
   const int dt = min(tid * kItems, la + lb);
-  int ia = merge_path_smem(s_k, la, s_k + la, lb, dt);
+  int ia = merge_path_smem(s_k, la, lb, dt);
   int ib = dt - ia;
-  bool emit[kItems];
+  u32 emit = 0;  // bit q: item q is written
   u64 ek[kItems];
   double evv[kItems];
-  u32 nemit = 0;
+  if (!__syncthreads_or(repeat)) {
+    // no: an A meets at most the B at hand, a B only the last A
+    u64 ka = ia < la ? s_k[pad(ia)] : ~0ull, kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
+    u64 last = ia > 0 ? s_k[pad(ia - 1)] : s_edge[0];
+    bool any_last = a0 + ia > 0;
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+      
+      ek[q] = 0;
+      evv[q] = 0.0;
+      if (dt + q >= la + lb) continue;
+      if (ib >= lb || (ia < la && ka <= kb)) {
+        double v = s_v[pad(ia)];
+        if (kb == ka && (ib < lb || b1 < nb)) v = apply_op(op, v, ib < lb ? s_v[pad(la + ib)] : s_edge_v);
+        emit |= 1u << q;
+        ek[q] = ka;
+        evv[q] = v;
+        last = ka;
+        any_last = true;
+        ++ia;
+        ka = ia < la ? s_k[pad(ia)] : ~0ull;
+      } else {
+        if (!any_last || last != kb) {
+          emit |= 1u << q;
+          ek[q] = kb;
+          evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
+        }
+        ++ib;
+        kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
+      }
+      
+    }
+  } else {
 #pragma unroll
   for (int q = 0; q < kItems; ++q) {
-    emit[q] = false;
+    
     ek[q] = 0;
     evv[q] = 0.0;
     const int m = dt + q;
     if (m >= la + lb) continue;
-    const bool take_a = ib >= lb || (ia < la && s_k[ia] <= s_k[la + ib]);
+    const bool take_a = ib >= lb || (ia < la && s_k[pad(ia)] <= s_k[pad(la + ib)]);
     const size_t mg = d0 + (size_t)m;  // global merged position
     if (take_a) {
       const size_t i = a0 + ia;
-      const u64 k = s_k[ia];
+      const u64 k = s_k[pad(ia)];
       const size_t lbB = mg - i;  // B elements before A_i: those with key < k
       size_t j = 0;               // occurrence of k in A before A_i
-      while ((int)j < ia && s_k[ia - 1 - j] == k) ++j;
+      while ((int)j < ia && s_k[pad(ia - 1 - j)] == k) ++j;
       if ((int)j == ia) j += run_index(ak, a0, k);
-      double v = s_v[ia];
+      double v = s_v[pad(ia)];
       const size_t pb = lbB + j;  // the partner B, if it has key k
       if (pb >= b0 && pb < b1) {
-        if (s_k[la + (int)(pb - b0)] == k) v = apply_op(op, v, s_v[la + (int)(pb - b0)]);
+        if (s_k[pad(la + (int)(pb - b0))] == k) v = apply_op(op, v, s_v[pad(la + (int)(pb - b0))]);
       } else if (pb < nb && bk[pb] == k) {
         v = apply_op(op, v, bv[pb]);
       }
-      emit[q] = true;
+      emit |= 1u << q;
       ek[q] = k;
       evv[q] = v;
       ++ia;
     } else {
       const size_t i = b0 + ib;
-      const u64 k = s_k[la + ib];
+      const u64 k = s_k[pad(la + ib)];
       const size_t ubA = mg - i;  // A elements before B_i: those with key <= k
       size_t j = 0;               // occurrence of k in B before B_i
-      while ((int)j < ib && s_k[la + ib - 1 - j] == k) ++j;
+      while ((int)j < ib && s_k[pad(la + ib - 1 - j)] == k) ++j;
       if ((int)j == ib) j += run_index(bk, b0, k);
       bool consumed = false;
       if (ubA >= j + 1) {
         const size_t pa = ubA - 1 - j;  // the A it would pair with
-        consumed = (pa >= a0 && pa < a1) ? s_k[(int)(pa - a0)] == k : ak[pa] == k;
+        consumed = (pa >= a0 && pa < a1) ? s_k[pad((int)(pa - a0))] == k : ak[pa] == k;
       }
       if (!consumed) {
-        emit[q] = true;
+        emit |= 1u << q;
         ek[q] = k;
-        evv[q] = apply_op(op, 0.0, s_v[la + ib]);
+        evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
       }
       ++ib;
     }
-    nemit += emit[q] ? 1u : 0u;
+    
   }
+  }
+  const u32 nemit = __popc(emit);
   // ---- block scan of emitted counts -------------------------------------
   u32 inc = nemit;
 #pragma unroll
@@ -227,17 +286,17 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const u64* __restrict__
   u32 r = excl;
 #pragma unroll
   for (int q = 0; q < kItems; ++q) {
-    if (emit[q]) {
-      s_k[r] = ek[q];
-      s_v[r] = evv[q];
+    if (emit & (1u << q)) {
+      s_k[pad(r)] = ek[q];
+      s_v[pad(r)] = evv[q];
       ++r;
     }
   }
   __syncthreads();
   const unsigned long long off = s_off;
   for (u32 i = tid; i < tot; i += kThreads) {
-    __stcs(ck + off + i, s_k[i]);
-    __stcs(cv + off + i, s_v[i]);
+    __stcs(ck + off + i, s_k[pad(i)]);
+    __stcs(cv + off + i, s_v[pad(i)]);
   }
 }
 
