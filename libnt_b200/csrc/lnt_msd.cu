@@ -20,11 +20,10 @@
 //      the buckets; a plain sort knows its offsets already.
 //
 // DRAM traffic: 8 B (histogram) + 32 B per pass + 16 B + 16 B per pair.
-// Measured on 2^27 pairs with 36-bit keys (B200): histogram 0.45 ms (bound by
-// issue: re-key and count), partition passes 0.81 and 0.86 ms (80% of the
-// measured copy rate), bucket kernel 1.85 ms (bound by the latency of its
-// block-wide phases and of the look-back); 4.08 ms against 5.93 ms for the
-// stable 7- and 8-bit onesweep passes (1.59 + 1.30 ms: eight ballots, a
+// Measured on 2^27 pairs with 36-bit keys (B200): histogram 0.36 ms, partition
+// passes 0.80 and 0.86 ms (80% of the measured copy rate), bucket kernel 1.9 ms
+// (bound by the latency of its block-wide phases and of the look-back); 3.95 ms
+// against 5.93 ms for the stable 7- and 8-bit onesweep passes (1.59 + 1.30 ms: eight ballots, a
 // per-warp counter and a look-back per pass) and a bucket kernel whose threads
 // each ranked ten words by looping over their sub-buckets (2.43 ms).
 #include <algorithm>
@@ -86,20 +85,6 @@ struct MsdCtrl {
   u32* gate;      // 0: every bucket fits a CTA (and no key loses bits), 1: take the LSD path
 };
 
-// Bucket counts in shared memory as 16-bit fields (two per word, 64 KB at
-// T = 15: two 1024-thread CTAs per SM).  A field keeps 15 bits; the increment
-// that takes it to 2^15 moves 2^15 to the bucket's global count and clears bit
-// 15 again, so no field carries into its neighbour (the other increments that
-// can land in between are far fewer than 2^15).
-__device__ __forceinline__ void count16(u32* sh, u32 b, const MsdCtrl& c) {
-  const u32 sh_bits = 16u * (b & 1u);
-  const u32 old = atomicAdd(&sh[b >> 1], 1u << sh_bits);
-  if (((old >> sh_bits) & 0x7FFFu) == 0x7FFFu) {  // rare: once per 2^15 keys of one bucket in one CTA
-    atomicSub(&sh[b >> 1], 0x8000u << sh_bits);
-    atomicAdd(&c.counts[b], 0x8000u);
-  }
-}
-
 // Loads I keys at positions base + j * stride + tid (those below `end`; 0
 // beyond) of the concatenated source and re-keys them.
 template <int I>
@@ -122,18 +107,21 @@ __device__ __forceinline__ void source_keys(const PairSource& s, u32 base, u32 s
   if (!all_a) rekey_items(k, s.rb, ~in_a);
 }
 
-__global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSource src, u32 n, int T, int db,
+// 32-bit counts, one CTA of 1024 threads per SM with eight keys per thread in
+// flight: 2^27 keys in 0.36 ms (0.48 with 16-bit counts, whose every increment
+// had to be checked, and two CTAs of half the registers).
+__global__ void __launch_bounds__(kHistThreads, 1) msd_hist_kernel(const PairSource src, u32 n, int T, int db,
                                                                    int shift, int key_bits, u32 cap, MsdCtrl c) {
-  extern __shared__ u32 sh[];  // 2^T 16-bit fields
+  extern __shared__ u32 sh[];  // 2^T counts
   __shared__ bool s_last;
   __shared__ u32 s_w[kHistThreads / 32], s_mx[kHistThreads / 32];
-  const int nb = 1 << T, nw = (nb + 1) >> 1;
+  const int nb = 1 << T;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < nw; i += kHistThreads) sh[i] = 0;
+  for (int i = tid; i < nb; i += kHistThreads) sh[i] = 0;
   __syncthreads();
   const u32 bmask = (u32)(nb - 1);
   u64 any = 0;
-  constexpr int U = 4;
+  constexpr int U = 8;
   for (u64 base = (u64)blockIdx.x * (kHistThreads * U); base < n; base += (u64)gridDim.x * (kHistThreads * U)) {
     const u32 end = (u32)min((u64)n, base + kHistThreads * U);
     u64 k[U];
@@ -141,7 +129,7 @@ __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSou
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if ((u32)base + u * kHistThreads + tid < end) {
-        count16(sh, (u32)(k[u] >> shift) & bmask, c);
+        atomicAdd(&sh[(u32)(k[u] >> shift) & bmask], 1u);
         any |= k[u];
       }
   }
@@ -149,7 +137,7 @@ __global__ void __launch_bounds__(kHistThreads, 2) msd_hist_kernel(const PairSou
   if (key_bits < 64 && (any >> key_bits) != 0) atomicOr(&c.misc[2], 1u);
   __syncthreads();
   for (int b = tid; b < nb; b += kHistThreads) {
-    const u32 v = (sh[b >> 1] >> (16 * (b & 1))) & 0xFFFFu;
+    const u32 v = sh[b];
     if (v) atomicAdd(&c.counts[b], v);
   }
   __threadfence();
@@ -1170,7 +1158,7 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
   if (cudaMemsetAsync(ctrl, 0, p.zero_bytes, s) != cudaSuccess) return LNT_DEVICE_ERROR;
   const u32 cap = p.large ? (u32)GeomLarge::kCap : (u32)GeomSmall::kCap;
   {
-    const size_t sh = std::max<size_t>(((size_t)1 << p.T) * 2, 4);  // 16-bit fields
+    const size_t sh = ((size_t)1 << p.T) * 4;
     if (cudaFuncSetAttribute(msd_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
       return LNT_DEVICE_ERROR;
     const u32 want = (p.n + kHistThreads * 4 - 1) / (kHistThreads * 4);
@@ -1181,7 +1169,7 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
     top_fields(&top.ra, p.shift);
     top_fields(&top.rb, p.shift);
     // (with one pass the cursors are the bucket starts: every bucket is its own segment)
-    msd_hist_kernel<<<std::min(want, (u32)sm_count() * 2), kHistThreads, sh, s>>>(
+    msd_hist_kernel<<<std::min(want, (u32)sm_count()), kHistThreads, sh, s>>>(
         top, p.n, p.T, p.passes == 1 ? 0 : p.db, p.shift, p.key_bits, cap, c);
     count_launch();
   }
