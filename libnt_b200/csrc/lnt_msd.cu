@@ -22,10 +22,11 @@
 // DRAM traffic: 8 B (histogram) + 32 B per pass + 16 B + 16 B per pair.
 // Measured on 2^27 pairs with 36-bit keys (B200): histogram 0.36 ms, partition
 // passes 0.80 and 0.86 ms (80% of the measured copy rate), bucket kernel 1.9 ms
-// (bound by the latency of its block-wide phases and of the look-back); 3.95 ms
-// against 5.93 ms for the stable 7- and 8-bit onesweep passes (1.59 + 1.30 ms: eight ballots, a
-// per-warp counter and a look-back per pass) and a bucket kernel whose threads
-// each ranked ten words by looping over their sub-buckets (2.43 ms).
+// (bound by the latency of its block-wide phases and of the look-back); 3.98 ms
+// against 5.90 ms for the stable 7- and 8-bit onesweep passes (1.59 + 1.30 ms:
+// eight ballots, a per-warp counter and a look-back per pass) and a bucket
+// kernel whose threads each ranked ten words by looping over their sub-buckets
+// (2.43 ms).
 #include <algorithm>
 #include <cstdlib>
 
