@@ -556,7 +556,8 @@ __global__ void residue_b_kernel(const double* __restrict__ B, u64 w, u64 wB, u6
 // of beta) while the estimate errs by under 2^-15; X = T - q M in limbs,
 // converted to double once (Horner from the top limb).  Each thread takes four
 // consecutive rows (one 4-byte load per modulus); grid x over rows of C, y
-// over columns.  (Unrolling the modulus loop to its compile-time bound, so
+// over columns.  Serves up to 9 and more than 16 moduli; the kernel below takes
+// the counts between.  (Unrolling the modulus loop to its compile-time bound, so
 // that the moduli tables become direct constant operands, measured slower at
 // 13 moduli: 5.35 against 4.69 ms at 16384^2.)
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
@@ -638,6 +639,170 @@ __global__ void __launch_bounds__(256) crt_kernel(const unsigned char* __restric
       C[i0 + c + h * j] = scale2(x, ea[c] + unbias(eB[j]));
     }
   }
+}
+
+// The same remaindering for 10 to 16 moduli with the limb sums on the tensor
+// cores.  The kernel above is bound by issue: 13 moduli x 4 limbs of 64-bit
+// multiply-adds, byte extractions and 64-bit carries are about 270
+// instructions per entry.  As a product of the residue bytes (entries x 16
+// moduli) with the bytes of the V_l (16 moduli x 16 bytes) the sums are two
+// m16n8k16 byte products per 16 entries, exact in 32 bits (16 x 255^2 < 2^20),
+// and what is left is byte shuffling before them, one 128-bit carry chain, the
+// subtraction of q M modulo 2^128 (|X| <= M/32 < 2^127, so the wrapped
+// difference is X) and the conversion.  The contraction is 16 deep: far too
+// thin for the tile engine of the modular products, whose accumulators would
+// have to come back through TMEM.
+//
+// A warp takes 128 rows of one column at a time.  Lane (g, t) loads 16 rows
+// (16 g ..) of moduli 4t .. 4t+3, which after a 4 x 4 byte transpose are its A
+// fragments; the columns of the B fragments are ordered so that it gets the
+// sums of bytes 4t .. 4t+3 of its rows.  The four quarters of a row meet
+// through shared memory, from where lane r takes the rows r, r + 32, ... (the
+// stores of C are whole lines).  The quarters of one row lie in two halves
+// whose 16-byte slots are permuted by the row, so that neither the writes nor
+// the reads conflict.
+struct CrtMma {
+  int n, beta;
+  u32 V[16][4];  // V_l in 32-bit words; zero from n on
+  u32 negM[4];   // 2^128 - M
+  u32 recip;     // floor(2^(32 + shift) / M), 20 or 21 bits
+  int shift;     // bit length of M less 12: T >> shift < 2^24
+};
+
+__device__ __forceinline__ void mma_u8(int (&c)[4], u32 a0, u32 a1, u32 b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+      : "r"(a0), "r"(a1), "r"(b), "r"(0));
+}
+
+constexpr int kCrtWarps = 8;
+constexpr int kCrtRows = 128;  // rows per warp and column
+
+// HIGH: the quotient's bits start in word 3 of T (else in word 2).
+template <bool HIGH>
+__global__ void __launch_bounds__(kCrtWarps * 32, 4) crt_mma_kernel(const unsigned char* __restrict__ res, u64 Mp,
+                                                                    u64 Np, u64 h, u64 wB, const CrtMma P,
+                                                                    const int* __restrict__ eA,
+                                                                    const int* __restrict__ eB,
+                                                                    double* __restrict__ C) {
+  __shared__ __align__(16) unsigned char buf[kCrtWarps][4096];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  unsigned char* sm = buf[threadIdx.x >> 5];
+  // warps over (row block, first column): row blocks fastest
+  const u32 blocks = (u32)((h + kCrtRows - 1) / kCrtRows);
+  const u32 warp = blockIdx.x * kCrtWarps + (threadIdx.x >> 5);
+  const u32 step = gridDim.x * kCrtWarps / blocks;
+  const u64 i0 = (u64)(warp % blocks) * kCrtRows;
+  u64 j = warp / blocks;
+  if (j >= step) return;
+  const u64 plane = Mp * Np;
+  res += blockIdx.z * P.n * plane;  // tabs
+  eA += blockIdx.z * h;
+  eB += blockIdx.z * wB;
+  C += blockIdx.z * h * wB;
+  u32 b[2] = {0, 0};
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    const u32 w = P.V[4 * t + kk][g >> 1] >> (8 * (g & 1));
+    b[0] |= (w & 0xffu) << (8 * kk);
+    b[1] |= ((w >> 16) & 0xffu) << (8 * kk);
+  }
+  int ea[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const u64 i = i0 + 32 * k + lane;
+    ea[k] = i < h ? unbias(eA[i]) - 2 * P.beta : 0;
+  }
+  const bool rows = i0 + 16 * g < Mp;  // Mp is a multiple of 16
+  const unsigned char* src = res + (u64)(4 * t) * plane + i0 + 16 * g;
+  for (; j < wB; j += step) {
+    uint4 x[4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+      x[kk] = rows && 4 * t + kk < P.n ? __ldcs(reinterpret_cast<const uint4*>(src + (u64)kk * plane + Mp * j))
+                                       : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // rows 4q .. 4q+3 of the lane's 16
+      const u32 w0 = (&x[0].x)[q], w1 = (&x[1].x)[q], w2 = (&x[2].x)[q], w3 = (&x[3].x)[q];
+      const u32 l01 = __byte_perm(w0, w1, 0x5140), h01 = __byte_perm(w0, w1, 0x7362);
+      const u32 l23 = __byte_perm(w2, w3, 0x5140), h23 = __byte_perm(w2, w3, 0x7362);
+      const u32 e[4] = {__byte_perm(l01, l23, 0x5410), __byte_perm(l01, l23, 0x7632), __byte_perm(h01, h23, 0x5410),
+                        __byte_perm(h01, h23, 0x7632)};
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        int c[4], d[4];
+        mma_u8(c, e[2 * m], e[2 * m + 1], b[0]);
+        mma_u8(d, e[2 * m], e[2 * m + 1], b[1]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int i = 4 * q + 2 * m + r;  // row 16 g + i: bytes 4t, 4t+1 and 4t+2, 4t+3
+          const int slot = g ^ (i & 7) ^ ((t >> 1) << 2);
+          *reinterpret_cast<uint2*>(sm + (t >> 1) * 2048 + (i * 8 + slot) * 16 + (t & 1) * 8) =
+              make_uint2((u32)c[2 * r] + ((u32)c[2 * r + 1] << 8), (u32)d[2 * r] + ((u32)d[2 * r + 1] << 8));
+        }
+      }
+    }
+    __syncwarp();
+    const int eb = unbias(eB[j]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = lane & 15, slot = (2 * k + (lane >> 4)) ^ (i & 7);
+      const uint4 p0 = *reinterpret_cast<const uint4*>(sm + (i * 8 + slot) * 16);
+      const uint4 p1 = *reinterpret_cast<const uint4*>(sm + 2048 + (i * 8 + (slot ^ 4)) * 16);
+      // T = sum_t (x_t + 2^16 y_t) 2^(32 t), 140 bits
+      u32 w0, w1, w2, w3, w4;
+      asm("add.cc.u32 %0, %5, %10;\n\taddc.cc.u32 %1, %6, %11;\n\taddc.cc.u32 %2, %7, %12;\n\t"
+          "addc.cc.u32 %3, %8, %13;\n\taddc.u32 %4, %9, %14;"
+          : "=&r"(w0), "=&r"(w1), "=&r"(w2), "=&r"(w3), "=&r"(w4)
+          : "r"(p0.x), "r"(p0.z), "r"(p1.x), "r"(p1.z), "r"(0), "r"(p0.y << 16), "r"(__byte_perm(p0.y, p0.w, 0x5432)),
+            "r"(__byte_perm(p0.w, p1.y, 0x5432)), "r"(__byte_perm(p1.y, p1.w, 0x5432)), "r"(p1.w >> 16));
+      // q = round(T / M): T / M < 2^12, from 24 bits of T and 20 of 1 / M to
+      // within 2^-7, and X / M is at most 1/32 away from an integer
+      const u32 top = HIGH ? __funnelshift_r(w3, w4, P.shift) : __funnelshift_r(w2, w3, P.shift);
+      const u32 quot = (u32)(((u64)top * P.recip + 0x80000000ull) >> 32);
+      asm("mad.lo.cc.u32 %0, %4, %5, %0;\n\tmadc.lo.cc.u32 %1, %4, %6, %1;\n\t"
+          "madc.lo.cc.u32 %2, %4, %7, %2;\n\tmadc.lo.u32 %3, %4, %8, %3;\n\t"
+          "mad.hi.cc.u32 %1, %4, %5, %1;\n\tmadc.hi.cc.u32 %2, %4, %6, %2;\n\tmadc.hi.u32 %3, %4, %7, %3;"
+          : "+&r"(w0), "+&r"(w1), "+&r"(w2), "+&r"(w3)
+          : "r"(quot), "r"(P.negM[0]), "r"(P.negM[1]), "r"(P.negM[2]), "r"(P.negM[3]));
+      // each word as a double by its bits (2^52 units of the word's weight in
+      // front), added from the top: exact until 53 bits are used up
+      constexpr double k0 = 4503599627370496.0, k1 = k0 * 4294967296.0, k2 = k1 * 4294967296.0,
+                       k3 = k2 * 4294967296.0;
+      double v = __hiloint2double(0x49300000, (int)(w3 ^ 0x80000000u)) - (k3 + k3 / 2097152.0);
+      v += __hiloint2double(0x47300000, (int)w2) - k2;
+      v += __hiloint2double(0x45300000, (int)w1) - k1;
+      v += __hiloint2double(0x43300000, (int)w0) - k0;
+      const u64 row = i0 + 32 * k + lane;
+      if (row < h) C[row + h * j] = scale2(v, ea[k] + eb);
+    }
+    __syncwarp();
+  }
+}
+
+// Host: the tables of crt_mma_kernel; false when it does not serve this count
+// of moduli (T's quotient bits would lie outside words 2 to 4, or a 17th
+// modulus does not fit the contraction).
+bool make_crt_mma(const CrtParams& P, CrtMma* q) {
+  if (P.n > 16) return false;
+  auto words = [](const u32* limbs, u32* w) {  // 27-bit limbs to 32-bit words
+    unsigned __int128 x = 0;
+    for (int b = kMaxLimbs - 1; b >= 0; --b) x = (x << kLimbBits) | limbs[b];
+    for (int k = 0; k < 4; ++k) w[k] = (u32)(x >> (32 * k));
+    return x;
+  };
+  q->n = P.n;
+  q->beta = P.beta;
+  for (int l = 0; l < 16; ++l) words(P.V[l], q->V[l]);  // zero beyond n
+  u32 m[4];
+  const unsigned __int128 M = words(P.Ml, m);
+  for (int k = 0; k < 4; ++k) q->negM[k] = (u32)((0 - M) >> (32 * k));
+  int bits = 0;
+  while (bits < 128 && (M >> bits)) ++bits;
+  q->shift = bits - 12;
+  if (q->shift < 64) return false;
+  q->recip = (u32)std::floor(std::ldexp(P.Minv, 32 + q->shift));
+  return true;
 }
 
 // ---- choosing the number of moduli ------------------------------------------
@@ -999,23 +1164,32 @@ int lnt_dense_lattice_mult_crt(const double* A, const double* B, double* C, int6
     if (st != LNT_OK) return st;
     {
       ProfScope prof("dense_crt", s);
-      const u64 rows4 = (uh + 3) / 4;
-      const unsigned gx = (unsigned)((rows4 + 255) / 256);
-      const unsigned gy = (unsigned)std::min<u64>(uwB, std::max<u64>(1, (u64)sms * 32 / gx));
-      const dim3 grid(gx, gy, n);
-      switch (P.lv) {
-        case 1:
-        case 2:
-        case 3:
-        case 4:
-          crt_kernel<4><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
-          break;
-        case 5:
-          crt_kernel<5><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
-          break;
-        default:
-          crt_kernel<6><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
-          break;
+      CrtMma Q;
+      if (make_crt_mma(P, &Q)) {
+        const u64 blocks = (uh + kCrtRows - 1) / kCrtRows;
+        const u64 most = std::max<u64>((blocks + kCrtWarps - 1) / kCrtWarps, (u64)sms * 4);
+        const dim3 grid((unsigned)std::min<u64>(most, (blocks * uwB + kCrtWarps - 1) / kCrtWarps), 1, n);
+        auto kern = Q.shift >= 96 ? crt_mma_kernel<true> : crt_mma_kernel<false>;
+        kern<<<grid, kCrtWarps * 32, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, Q, eA, eB, Ct);
+      } else {
+        const u64 rows4 = (uh + 3) / 4;
+        const unsigned gx = (unsigned)((rows4 + 255) / 256);
+        const unsigned gy = (unsigned)std::min<u64>(uwB, std::max<u64>(1, (u64)sms * 32 / gx));
+        const dim3 grid(gx, gy, n);
+        switch (P.lv) {
+          case 1:
+          case 2:
+          case 3:
+          case 4:
+            crt_kernel<4><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
+            break;
+          case 5:
+            crt_kernel<5><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
+            break;
+          default:
+            crt_kernel<6><<<grid, 256, 0, s>>>(prod, L.Mp, L.Np, uh, uwB, P, eA, eB, Ct);
+            break;
+        }
       }
       count_launch();
     }
