@@ -8,7 +8,7 @@
 // surplus A's are copied and surplus B's become op(0, b).
 //
 // GPU formulation: the stable merge of A and B (A first on ties) is split by
-// merge-path diagonals into tiles of 2048 merged elements.  In that order the
+// merge-path diagonals into tiles of 1536 merged elements.  In that order the
 // j-th A of a key run sits before every B of the run, so each element decides
 // locally (from its merged position and at most two neighbour reads) whether
 // it is emitted and with which partner:
@@ -25,9 +25,20 @@
 // offsets come from a block scan plus a decoupled look-back over tiles.
 // A tile in which no key repeats inside an operand (checked on the staged keys)
 // needs none of the run bookkeeping: an A meets at most the B at hand, a B only
-// the A taken last (0.54 -> 0.46 ms).
+// the A taken last.
+// CTAs are persistent and the look-back is off their path: a ninth warp runs it
+// while the other eight go on with the CTA's next tile, and a tile's elements
+// wait for their offset in shared memory, in one of two buffers.  (When every
+// warp waited for the offset, 40% of the stalls were at that barrier.)  Tile ids
+// are taken as late as possible: the longer a CTA sits on an id, the longer the
+// others look back.
 // Traffic: 16 B read per input pair + 16 B written per output pair; bound by the
-// latency of the tile's steps, the look-back a quarter of it (0.30 ms without).
+// latency of a tile's steps.  20M + 12M pairs 0.41 ms (0.47 before the ninth
+// warp), 2 x 2^26 pairs 1.75 ms (2.04), 2 x 2^24 with many repeats 0.57 (0.60).
+// Also measured for the first two: tiles of 2048 with three CTAs per SM 0.41 and
+// 1.85, of 1024 with four 0.44 and 1.82; the next id taken before the merge (at
+// 2048) 0.43 and 1.89; the next tile's loads held in registers across the write
+// 0.50 and 2.2.
 #include <algorithm>
 
 #include "lnt_msd.cuh"
@@ -36,7 +47,8 @@ namespace lnt {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 8;
+constexpr int kItems = 6;
+constexpr int kCtas = 4;  // per SM: 54 KB of shared memory and 56 registers a thread
 constexpr int kTile = kThreads * kItems;
 constexpr unsigned long long kFlagAgg = 1ull << 62;
 constexpr unsigned long long kFlagPre = 2ull << 62;
@@ -95,208 +107,257 @@ __global__ void merge_partition_kernel(const u64* __restrict__ a, size_t na, con
   splits[t] = merge_path(a, na, b, nb, min(na + nb, (size_t)t * kTile));
 }
 
-__global__ void __launch_bounds__(kThreads, 4) merge_kernel(const u64* __restrict__ ak, const double* __restrict__ av,
-                                                         size_t na, const u64* __restrict__ bk,
-                                                         const double* __restrict__ bv, size_t nb, int op,
-                                                         u32 ntiles, const u64* __restrict__ splits,
-                                                         unsigned long long* __restrict__ status,
-                                                         u32* __restrict__ tile_counter, u64* __restrict__ ck,
-                                                         double* __restrict__ cv, u64* __restrict__ d_nout) {
-  __shared__ u64 s_k[kPadded];
-  __shared__ double s_v[kPadded];
+// Barriers of part of a CTA (ids 1..; 0 is __syncthreads).
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ bool bar_or(int id, int threads, bool p) {
+  int r;
+  __syncwarp();
+  asm volatile("{.reg .pred p, q; setp.ne.s32 p, %3, 0; bar.red.or.pred q, %1, %2, p; selp.s32 %0, 1, 0, q;}"
+               : "=r"(r)
+               : "r"(id), "r"(threads), "r"((int)p)
+               : "memory");
+  return r != 0;
+}
+constexpr int kMainBar = 1, kReqBar = 2, kOffBar = 4;  // the last two for both buffers
+constexpr int kMergeSmem = 2 * kPadded * 16;
+
+__global__ void __launch_bounds__(kThreads + 32, kCtas)
+    merge_kernel(const u64* __restrict__ ak, const double* __restrict__ av, size_t na, const u64* __restrict__ bk,
+                 const double* __restrict__ bv, size_t nb, int op, u32 ntiles, const u64* __restrict__ splits,
+                 unsigned long long* __restrict__ status, u32* __restrict__ tile_counter, u64* __restrict__ ck,
+                 double* __restrict__ cv, u64* __restrict__ d_nout) {
+  extern __shared__ u64 smem[];
   __shared__ u32 s_warp[kThreads / 32];
-  __shared__ u32 s_tile;
-  __shared__ unsigned long long s_off;
+  __shared__ u32 s_tile, s_rt[2], s_tot[2];
+  __shared__ unsigned long long s_off[2];
   __shared__ u64 s_edge[3];
   __shared__ double s_edge_v;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
-  __syncthreads();
-  const u32 tile = s_tile;
-  const size_t total = na + nb;
-  const size_t d0 = (size_t)tile * kTile;
-  const size_t d1 = min(total, d0 + kTile);
-  const size_t a0 = splits[tile], a1 = splits[tile + 1];
-  const size_t b0 = d0 - a0, b1 = d1 - a1;
-  const int la = (int)(a1 - a0), lb = (int)(b1 - b0);
-  if (warp == kThreads / 32 - 1) {  // what lies just outside the slices
-    if (lane == 0 && a0 > 0) s_edge[0] = ak[a0 - 1];
-    if (lane == 1 && b1 < nb) s_edge[1] = bk[b1];
-    if (lane == 2 && b1 < nb) s_edge_v = bv[b1];
-    if (lane == 3 && b0 > 0) s_edge[2] = bk[b0 - 1];
-  }
-  // stage the tile's A slice then its B slice, keys and values, in shared memory
-  for (int i = tid; i < la + lb; i += kThreads) {
-    if (i < la) {
-      s_k[pad(i)] = __ldcs(ak + a0 + i);
-      s_v[pad(i)] = __ldcs(av + a0 + i);
-    } else {
-      s_k[pad(i)] = __ldcs(bk + b0 + (i - la));
-      s_v[pad(i)] = __ldcs(bv + b0 + (i - la));
+  if (warp == kThreads / 32) {
+    // ---- look-back for the tiles' output offsets ----------------------------
+    for (int buf = 0;; buf ^= 1) {
+      bar_sync(kReqBar + buf, 64);
+      const u32 tile = *(volatile u32*)&s_rt[buf], tot = *(volatile u32*)&s_tot[buf];
+      if (tile >= ntiles) return;
+      unsigned long long off = 0;
+      if (tile != 0) {
+        int base = (int)tile - 1;
+        u32 spins = 0;
+        while (base >= 0) {
+          const int p = base - lane;
+          const unsigned long long w =
+              p >= 0 ? *reinterpret_cast<const volatile unsigned long long*>(status + p) : kFlagPre;
+          const unsigned long long f = w & kFlagMask;
+          const u32 notready = __ballot_sync(0xffffffffu, f == 0);
+          const u32 pre = __ballot_sync(0xffffffffu, f == kFlagPre);
+          const int first_nr = notready ? __ffs(notready) - 1 : 32;
+          const int first_pre = pre ? __ffs(pre) - 1 : 32;
+          const int take = first_pre < first_nr ? first_pre + 1 : first_nr;
+          unsigned long long v = lane < take ? (w & kValMask) : 0ull;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          off += v;
+          if (first_pre < first_nr) break;
+          base -= first_nr;
+          if (first_nr < 32 && ++spins > spin_limit()) {
+            latch_error(kErrMergeLookback);
+            break;
+          }
+        }
+        if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = kFlagPre | (off + tot);
+      }
+      if (lane == 0) {
+        s_off[buf] = off;
+        if (tile == ntiles - 1) *d_nout = off + tot;
+      }
+      __syncwarp();
+      bar_arrive(kOffBar + buf, kThreads + 32);
     }
   }
-  __syncthreads();
-  // a key repeated inside an operand (also across the slice's start)?
-  bool repeat = false;
-  for (int i = tid; i < la + lb; i += kThreads) {
-    const bool first = i == 0 || i == la;
-    repeat = repeat || (first ? (i < la ? a0 > 0 && s_k[pad(i)] == s_edge[0] : b0 > 0 && s_k[pad(i)] == s_edge[2])
-                              : s_k[pad(i)] == s_k[pad(i - 1)]);
-  }
-  // each thread merges kItems consecutive merged positions
-  const int dt = min(tid * kItems, la + lb);
-  int ia = merge_path_smem(s_k, la, lb, dt);
-  int ib = dt - ia;
-  u32 emit = 0;  // bit q: item q is written
-  u64 ek[kItems];
-  double evv[kItems];
-  if (!__syncthreads_or(repeat)) {
-    // no: an A meets at most the B at hand, a B only the last A
-    u64 ka = ia < la ? s_k[pad(ia)] : ~0ull, kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
-    u64 last = ia > 0 ? s_k[pad(ia - 1)] : s_edge[0];
-    bool any_last = a0 + ia > 0;
+  const size_t total = na + nb;
+  u32 held = 0;  // elements of the previous tile, still to be written
+  auto write_held = [&](int b) {
+    const u64* h_k = smem + b * 2 * kPadded;
+    const double* h_v = reinterpret_cast<const double*>(h_k + kPadded);
+    bar_sync(kOffBar + b, kThreads + 32);
+    const unsigned long long off = *(volatile unsigned long long*)&s_off[b];
+    for (u32 i = tid; i < held; i += kThreads) {
+      __stcs(ck + off + i, h_k[pad(i)]);
+      __stcs(cv + off + i, h_v[pad(i)]);
+    }
+  };
+  for (int n = 0;; ++n) {
+    const int buf = n & 1;
+    u64* s_k = smem + buf * 2 * kPadded;
+    double* s_v = reinterpret_cast<double*>(s_k + kPadded);
+    if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
+    bar_sync(kMainBar, kThreads);  // also: the buffer's last tile is written
+    const u32 tile = s_tile;
+    if (tile >= ntiles) {
+      if (warp == 0) {  // ends the look-back warp
+        if (lane == 0) s_rt[buf] = tile;
+        bar_arrive(kReqBar + buf, 64);
+      }
+      if (n > 0) write_held(buf ^ 1);
+      return;
+    }
+    const size_t d0 = (size_t)tile * kTile;
+    const size_t d1 = min(total, d0 + kTile);
+    const size_t a0 = splits[tile], a1 = splits[tile + 1];
+    const size_t b0 = d0 - a0, b1 = d1 - a1;
+    const int la = (int)(a1 - a0), lb = (int)(b1 - b0);
+    if (warp == kThreads / 32 - 1) {  // what lies just outside the slices
+      if (lane == 0 && a0 > 0) s_edge[0] = ak[a0 - 1];
+      if (lane == 1 && b1 < nb) s_edge[1] = bk[b1];
+      if (lane == 2 && b1 < nb) s_edge_v = bv[b1];
+      if (lane == 3 && b0 > 0) s_edge[2] = bk[b0 - 1];
+    }
+    // stage the tile's A slice then its B slice, keys and values, in shared memory
+    for (int i = tid; i < la + lb; i += kThreads) {
+      if (i < la) {
+        s_k[pad(i)] = __ldcs(ak + a0 + i);
+        s_v[pad(i)] = __ldcs(av + a0 + i);
+      } else {
+        s_k[pad(i)] = __ldcs(bk + b0 + (i - la));
+        s_v[pad(i)] = __ldcs(bv + b0 + (i - la));
+      }
+    }
+    bar_sync(kMainBar, kThreads);
+    // a key repeated inside an operand (also across the slice's start)?
+    bool repeat = false;
+    for (int i = tid; i < la + lb; i += kThreads) {
+      const bool first = i == 0 || i == la;
+      repeat = repeat || (first ? (i < la ? a0 > 0 && s_k[pad(i)] == s_edge[0] : b0 > 0 && s_k[pad(i)] == s_edge[2])
+                                : s_k[pad(i)] == s_k[pad(i - 1)]);
+    }
+    // each thread merges kItems consecutive merged positions
+    const int dt = min(tid * kItems, la + lb);
+    int ia = merge_path_smem(s_k, la, lb, dt);
+    int ib = dt - ia;
+    u32 emit = 0;  // bit q: item q is written
+    u64 ek[kItems];
+    double evv[kItems];
+    if (!bar_or(kMainBar, kThreads, repeat)) {
+      // no: an A meets at most the B at hand, a B only the last A
+      u64 ka = ia < la ? s_k[pad(ia)] : ~0ull, kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
+      u64 last = ia > 0 ? s_k[pad(ia - 1)] : s_edge[0];
+      bool any_last = a0 + ia > 0;
+#pragma unroll
+      for (int q = 0; q < kItems; ++q) {
+        ek[q] = 0;
+        evv[q] = 0.0;
+        if (dt + q >= la + lb) continue;
+        if (ib >= lb || (ia < la && ka <= kb)) {
+          double v = s_v[pad(ia)];
+          if (kb == ka && (ib < lb || b1 < nb)) v = apply_op(op, v, ib < lb ? s_v[pad(la + ib)] : s_edge_v);
+          emit |= 1u << q;
+          ek[q] = ka;
+          evv[q] = v;
+          last = ka;
+          any_last = true;
+          ++ia;
+          ka = ia < la ? s_k[pad(ia)] : ~0ull;
+        } else {
+          if (!any_last || last != kb) {
+            emit |= 1u << q;
+            ek[q] = kb;
+            evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
+          }
+          ++ib;
+          kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < kItems; ++q) {
+        ek[q] = 0;
+        evv[q] = 0.0;
+        const int m = dt + q;
+        if (m >= la + lb) continue;
+        const bool take_a = ib >= lb || (ia < la && s_k[pad(ia)] <= s_k[pad(la + ib)]);
+        const size_t mg = d0 + (size_t)m;  // global merged position
+        if (take_a) {
+          const size_t i = a0 + ia;
+          const u64 k = s_k[pad(ia)];
+          const size_t lbB = mg - i;  // B elements before A_i: those with key < k
+          size_t j = 0;               // occurrence of k in A before A_i
+          while ((int)j < ia && s_k[pad(ia - 1 - j)] == k) ++j;
+          if ((int)j == ia) j += run_index(ak, a0, k);
+          double v = s_v[pad(ia)];
+          const size_t pb = lbB + j;  // the partner B, if it has key k
+          if (pb >= b0 && pb < b1) {
+            if (s_k[pad(la + (int)(pb - b0))] == k) v = apply_op(op, v, s_v[pad(la + (int)(pb - b0))]);
+          } else if (pb < nb && bk[pb] == k) {
+            v = apply_op(op, v, bv[pb]);
+          }
+          emit |= 1u << q;
+          ek[q] = k;
+          evv[q] = v;
+          ++ia;
+        } else {
+          const size_t i = b0 + ib;
+          const u64 k = s_k[pad(la + ib)];
+          const size_t ubA = mg - i;  // A elements before B_i: those with key <= k
+          size_t j = 0;               // occurrence of k in B before B_i
+          while ((int)j < ib && s_k[pad(la + ib - 1 - j)] == k) ++j;
+          if ((int)j == ib) j += run_index(bk, b0, k);
+          bool consumed = false;
+          if (ubA >= j + 1) {
+            const size_t pa = ubA - 1 - j;  // the A it would pair with
+            consumed = (pa >= a0 && pa < a1) ? s_k[pad((int)(pa - a0))] == k : ak[pa] == k;
+          }
+          if (!consumed) {
+            emit |= 1u << q;
+            ek[q] = k;
+            evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
+          }
+          ++ib;
+        }
+      }
+    }
+    const u32 nemit = __popc(emit);
+    // ---- block scan of emitted counts -------------------------------------
+    u32 inc = nemit;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    bar_sync(kMainBar, kThreads);
+    u32 excl = inc - nemit, tot = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) excl += s_warp[w];
+      tot += s_warp[w];
+    }
+    if (tid == 0)
+      *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = (tile == 0 ? kFlagPre : kFlagAgg) | tot;
+    // the emitted elements to the front (every thread is past its reads)
+    u32 r = excl;
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-      
-      ek[q] = 0;
-      evv[q] = 0.0;
-      if (dt + q >= la + lb) continue;
-      if (ib >= lb || (ia < la && ka <= kb)) {
-        double v = s_v[pad(ia)];
-        if (kb == ka && (ib < lb || b1 < nb)) v = apply_op(op, v, ib < lb ? s_v[pad(la + ib)] : s_edge_v);
-        emit |= 1u << q;
-        ek[q] = ka;
-        evv[q] = v;
-        last = ka;
-        any_last = true;
-        ++ia;
-        ka = ia < la ? s_k[pad(ia)] : ~0ull;
-      } else {
-        if (!any_last || last != kb) {
-          emit |= 1u << q;
-          ek[q] = kb;
-          evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
-        }
-        ++ib;
-        kb = ib < lb ? s_k[pad(la + ib)] : s_edge[1];
+      if (emit & (1u << q)) {
+        s_k[pad(r)] = ek[q];
+        s_v[pad(r)] = evv[q];
+        ++r;
       }
-      
     }
-  } else {
-#pragma unroll
-  for (int q = 0; q < kItems; ++q) {
-    
-    ek[q] = 0;
-    evv[q] = 0.0;
-    const int m = dt + q;
-    if (m >= la + lb) continue;
-    const bool take_a = ib >= lb || (ia < la && s_k[pad(ia)] <= s_k[pad(la + ib)]);
-    const size_t mg = d0 + (size_t)m;  // global merged position
-    if (take_a) {
-      const size_t i = a0 + ia;
-      const u64 k = s_k[pad(ia)];
-      const size_t lbB = mg - i;  // B elements before A_i: those with key < k
-      size_t j = 0;               // occurrence of k in A before A_i
-      while ((int)j < ia && s_k[pad(ia - 1 - j)] == k) ++j;
-      if ((int)j == ia) j += run_index(ak, a0, k);
-      double v = s_v[pad(ia)];
-      const size_t pb = lbB + j;  // the partner B, if it has key k
-      if (pb >= b0 && pb < b1) {
-        if (s_k[pad(la + (int)(pb - b0))] == k) v = apply_op(op, v, s_v[pad(la + (int)(pb - b0))]);
-      } else if (pb < nb && bk[pb] == k) {
-        v = apply_op(op, v, bv[pb]);
+    if (warp == 0) {  // hand the tile to the look-back warp
+      if (lane == 0) {
+        s_rt[buf] = tile;
+        s_tot[buf] = tot;
       }
-      emit |= 1u << q;
-      ek[q] = k;
-      evv[q] = v;
-      ++ia;
-    } else {
-      const size_t i = b0 + ib;
-      const u64 k = s_k[pad(la + ib)];
-      const size_t ubA = mg - i;  // A elements before B_i: those with key <= k
-      size_t j = 0;               // occurrence of k in B before B_i
-      while ((int)j < ib && s_k[pad(la + ib - 1 - j)] == k) ++j;
-      if ((int)j == ib) j += run_index(bk, b0, k);
-      bool consumed = false;
-      if (ubA >= j + 1) {
-        const size_t pa = ubA - 1 - j;  // the A it would pair with
-        consumed = (pa >= a0 && pa < a1) ? s_k[pad((int)(pa - a0))] == k : ak[pa] == k;
-      }
-      if (!consumed) {
-        emit |= 1u << q;
-        ek[q] = k;
-        evv[q] = apply_op(op, 0.0, s_v[pad(la + ib)]);
-      }
-      ++ib;
+      bar_arrive(kReqBar + buf, 64);
     }
-    
-  }
-  }
-  const u32 nemit = __popc(emit);
-  // ---- block scan of emitted counts -------------------------------------
-  u32 inc = nemit;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) s_warp[warp] = inc;
-  __syncthreads();
-  u32 excl = inc - nemit, tot = 0;
-  for (int w = 0; w < kThreads / 32; ++w) {
-    if (w < warp) excl += s_warp[w];
-    tot += s_warp[w];
-  }
-  // ---- look-back for the tile's output offset (warp 0) --------------------
-  if (warp == 0) {
-    if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = (tile == 0 ? kFlagPre : kFlagAgg) | tot;
-    unsigned long long off = 0;
-    if (tile != 0) {
-      int base = (int)tile - 1;
-      u32 spins = 0;
-      while (base >= 0) {
-        const int p = base - lane;
-        const unsigned long long w =
-            p >= 0 ? *reinterpret_cast<const volatile unsigned long long*>(status + p) : kFlagPre;
-        const unsigned long long f = w & kFlagMask;
-        const u32 notready = __ballot_sync(0xffffffffu, f == 0);
-        const u32 pre = __ballot_sync(0xffffffffu, f == kFlagPre);
-        const int first_nr = notready ? __ffs(notready) - 1 : 32;
-        const int first_pre = pre ? __ffs(pre) - 1 : 32;
-        const int take = first_pre < first_nr ? first_pre + 1 : first_nr;
-        unsigned long long v = lane < take ? (w & kValMask) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        off += v;
-        if (first_pre < first_nr) break;
-        base -= first_nr;
-        if (first_nr < 32 && ++spins > spin_limit()) {
-          latch_error(kErrMergeLookback);
-          break;
-        }
-      }
-      if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&status[tile]) = kFlagPre | (off + tot);
-    }
-    if (lane == 0) {
-      s_off = off;
-      if (tile == ntiles - 1) *d_nout = off + tot;
-    }
-  }
-  __syncthreads();  // s_k reads done; s_off ready
-  u32 r = excl;
-#pragma unroll
-  for (int q = 0; q < kItems; ++q) {
-    if (emit & (1u << q)) {
-      s_k[pad(r)] = ek[q];
-      s_v[pad(r)] = evv[q];
-      ++r;
-    }
-  }
-  __syncthreads();
-  const unsigned long long off = s_off;
-  for (u32 i = tid; i < tot; i += kThreads) {
-    __stcs(ck + off + i, s_k[pad(i)]);
-    __stcs(cv + off + i, s_v[pad(i)]);
+    if (n > 0) write_held(buf ^ 1);
+    held = tot;
   }
 }
 
@@ -367,7 +428,10 @@ int lnt_merge_sorted(const uint64_t* a_keys, const double* a_vals, size_t na, co
     ProfScope prof("merge", s);
     merge_partition_kernel<<<(L.ntiles + 1 + 255) / 256, 256, 0, s>>>((const u64*)a_keys, na, (const u64*)b_keys, nb,
                                                                        L.ntiles, splits);
-    merge_kernel<<<L.ntiles, kThreads, 0, s>>>((const u64*)a_keys, a_vals, na, (const u64*)b_keys, b_vals, nb, op,
+    if (cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMergeSmem) != cudaSuccess)
+      return LNT_DEVICE_ERROR;
+    const u32 grid = std::min<u32>(L.ntiles, (u32)kCtas * (u32)sm_count());
+    merge_kernel<<<grid, kThreads + 32, kMergeSmem, s>>>((const u64*)a_keys, a_vals, na, (const u64*)b_keys, b_vals, nb, op,
                                                L.ntiles, splits, reinterpret_cast<unsigned long long*>(w + L.off_status),
                                                reinterpret_cast<u32*>(w + L.off_counter), (u64*)c_keys, c_vals,
                                                (u64*)d_nout);

@@ -35,3 +35,23 @@ def test_pairs_on_tile_boundaries(cuda, torch, n, repeat, shift, op):
     np.testing.assert_array_equal(to_host(k, np.uint64), ek)
     np.testing.assert_array_equal(to_host(v), ev)
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("op", [0, 1])
+@pytest.mark.parametrize("n", [1, 767, 768, 769, 1536, 4608, 460000, 2500000])
+def test_tiles_of_1536_and_several_per_cta(cuda, torch, n, op):
+    """Tiles of 1536 merged elements, taken in turn by persistent CTAs: one tile,
+    two, fewer than there are CTAs, one more each, and several.  Runs of equal
+    keys at every second boundary, and outputs that shrink from tile to tile."""
+    rng = np.random.default_rng(n)
+    ak = np.arange(n, dtype=np.uint64) * np.uint64(2)
+    for at in range(766, n - 4, 1536):
+        ak[at:at + 4] = ak[at]
+    bk = np.where(rng.random(n) < np.linspace(0.0, 1.0, n), ak, ak + np.uint64(1))
+    bk.sort()
+    av, bv = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    k, v = cuda.merge_sorted(to_dev(ak, torch), to_dev(av, torch), to_dev(bk, torch), to_dev(bv, torch), op=op)
+    ek, ev = oracle.merge_sorted(ak, av, bk, bv, op)[:2]
+    np.testing.assert_array_equal(to_host(k, np.uint64), ek)
+    np.testing.assert_array_equal(to_host(v), ev)
+    assert cuda.device_status() == 0
