@@ -387,9 +387,9 @@ struct PermuteSortLayout {
   PairSort sort;
   size_t off_ctrl, off_a, off_b, total;
 };
-PermuteSortLayout permute_sort_layout(size_t n, u64 max_key) {
+PermuteSortLayout permute_sort_layout(size_t n, u64 max_key, bool buckets = true) {
   PermuteSortLayout L;
-  L.sort = make_pair_sort(n, max_key);
+  L.sort = make_pair_sort(n, max_key, buckets);
   size_t off = 0;
   L.off_ctrl = off;
   off += align_up(L.sort.ctrl_bytes, 256);
@@ -456,6 +456,7 @@ int lnt_permute_sort(const uint64_t* keys_in, const double* vals_in, size_t n, c
     return LNT_BAD_ARG;  // out of place only
   if (n >= (1u << 30)) return LNT_UNSUPPORTED;
   PermuteSortLayout L = permute_sort_layout(n, max_key);
+  if (workspace_bytes < L.total) L = permute_sort_layout(n, max_key, false);  // the digit passes may need less
   if (!workspace || workspace_bytes < L.total) return LNT_WORKSPACE;
   if ((uintptr_t)workspace % 256) return LNT_BAD_ARG;
   PairSource src = plain_source((const u64*)keys_in, vals_in, n);

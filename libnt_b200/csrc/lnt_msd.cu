@@ -1192,11 +1192,11 @@ int run_msd_sort(const MsdPlan& p, const PairSource& src, void* x, void* y, void
                  : launch_bucket_sort<GeomSmall>(p, ry, c, fold, out_k, out_v, s);
 }
 
-PairSort make_pair_sort(size_t n, u64 max_key) {
+PairSort make_pair_sort(size_t n, u64 max_key, bool buckets) {
   PairSort p;
-  p.msd = make_msd_plan(n, max_key);
+  if (buckets) p.msd = make_msd_plan(n, max_key);
   p.lsd = make_sort_plan(n, max_key, p.msd.ok);
-  p.ctrl_bytes = align_up(std::max(p.lsd.ctrl_bytes, p.msd.ctrl_bytes), 256) + 256;
+  p.ctrl_bytes = align_up(std::max(p.lsd.ctrl_bytes, p.msd.ctrl_bytes), 256) + (p.msd.ok ? 256 : 0);
   if (p.msd.single) {  // needs no scratch
     p.ctrl_bytes = 256;
     return p;

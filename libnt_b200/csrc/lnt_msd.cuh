@@ -49,7 +49,7 @@ struct PairSort {
   size_t ctrl_bytes = 0;  // control block: either path's, then the gate word
   size_t a_bytes = 0, b_bytes = 0;  // scratch (b: 0 when not needed)
 };
-PairSort make_pair_sort(size_t n, u64 max_key);
+PairSort make_pair_sort(size_t n, u64 max_key, bool buckets = true);
 // out must not overlap the source; a, b, ctrl: 256-byte aligned.
 int run_pair_sort(const PairSort& p, const PairSource& src, u64* out_k, double* out_v, void* a, void* b, void* ctrl,
                   cudaStream_t s);

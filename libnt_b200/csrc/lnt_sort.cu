@@ -660,9 +660,9 @@ struct SortPairsLayout {
   size_t off_a, off_b, total;
 };
 
-SortPairsLayout sort_pairs_layout(size_t n, u64 max_key) {
+SortPairsLayout sort_pairs_layout(size_t n, u64 max_key, bool buckets = true) {
   SortPairsLayout L;
-  L.sort = make_pair_sort(n, max_key);
+  L.sort = make_pair_sort(n, max_key, buckets);
   size_t off = align_up(L.sort.ctrl_bytes, 256);
   L.off_a = off;
   off += L.sort.a_bytes;
@@ -700,6 +700,7 @@ int lnt_sort_pairs(const uint64_t* keys_in, const double* vals_in, uint64_t* key
   if (!keys_in || !vals_in || !keys_out || !vals_out) return LNT_BAD_ARG;
   if (n >= (1u << 30)) return LNT_UNSUPPORTED;
   SortPairsLayout L = sort_pairs_layout(n, max_key);
+  if (workspace_bytes < L.total) L = sort_pairs_layout(n, max_key, false);  // the digit passes may need less
   if (!workspace || workspace_bytes < L.total) return LNT_WORKSPACE;
   if ((uintptr_t)workspace % 256) return LNT_BAD_ARG;
   cudaStream_t s = as_stream(stream);

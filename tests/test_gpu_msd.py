@@ -139,3 +139,39 @@ def test_small_sorts(cuda, torch, n, max_key, kind):
         np.testing.assert_array_equal(to_host(k, np.uint64), ek)
         assert rel_ok(to_host(v), ev, ea)
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("entry", ["lnt_sort_pairs", "lnt_permute_sort"])
+@pytest.mark.parametrize("n,bits", [(40000, 36), (1 << 20, 20), ((1 << 21) + 3, 36)])
+def test_scratch_of_the_digit_passes_is_enough(cuda, torch, rng, monkeypatch, entry, n, bits):
+    """With room for the digit passes but not for the bucketed path the sort
+    takes the digit passes; with less it is refused."""
+    import ctypes as C
+    import libnt_b200 as L
+    need, have = C.c_size_t(0), C.c_size_t(0)
+    query = getattr(L.lib(), entry + "_workspace")
+    monkeypatch.setenv("LNT_NO_BUCKETS", "1")
+    assert query(n, 1 << bits, C.byref(need)) == 0
+    monkeypatch.delenv("LNT_NO_BUCKETS")
+    assert query(n, 1 << bits, C.byref(have)) == 0
+    keys = rng.integers(0, 1 << bits, n).astype(np.uint64)
+    vals = rng.uniform(-1, 1, n)
+    k, v = to_dev(keys, torch), to_dev(vals, torch)
+    ok, ov = torch.empty_like(k), torch.empty_like(v)
+    ws = L.workspace(max(need.value, have.value))
+
+    def call(nbytes):
+        p = [C.c_void_p(x.data_ptr()) for x in (k, v, ok, ov, ws)]
+        if entry == "lnt_sort_pairs":
+            return L.lib().lnt_sort_pairs(p[0], p[1], p[2], p[3], n, 1 << bits, p[4], nbytes, None)
+        return L.lib().lnt_permute_sort(p[0], p[1], n, None, p[2], p[3], 1 << bits, p[4], nbytes, None)
+
+    order = np.argsort(keys, kind="stable")
+    for nbytes in (need.value, have.value):
+        ok.zero_(), ov.zero_()
+        assert call(nbytes) == 0
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(to_host(ok, np.uint64), keys[order])
+        np.testing.assert_array_equal(to_host(ov), vals[order])
+    assert call(min(need.value, have.value) - 1) == 5  # LNT_WORKSPACE
+    assert cuda.device_status() == 0
