@@ -41,8 +41,8 @@
 // The work is cut into tasks of one operand of one problem (at most 64 K
 // entries, less when the batch is small), largest first.
 // 4096 problems of 100 to 10^5 entries (1.18e8 pairs, 4.4e7 products), B200:
-// mark 0.33, rank 0.03, filter 0.57, base 0.02, place 0.52, symbolic 0.43,
-// numeric 0.66, the call 2.6 ms (11.7 ms when the batch was sorted: compose 0.61,
+// mark 0.33, rank 0.03, filter 0.57, base 0.02, place 0.51, symbolic 0.45,
+// numeric 0.61, the call 2.57 ms (11.7 ms when the batch was sorted: compose 0.61,
 // histogram 0.50, five digit passes 5.9, column pointers 1.3, symbolic 1.3,
 // numeric 2.05).  2.7e7 entries and 6.7e6 of 3.7e7 indices have a partner.
 // Batches with taller problems sort instead: one kernel re-keys every pair into
@@ -440,7 +440,7 @@ struct GroupArgs {
   uint4* kept;   // kept entries, at their task's place: (group, row or index, value)
   u32* kept_n;   // per task
   ulonglong2* arec;  // (row, value) grouped by index
-  ulonglong2* brec;  // (index, value) grouped by output column
+  ulonglong2* brec;  // (index, later its (end, count) in arec; value) grouped by output column
   u32* counters;     // [0] numbered indices, [1], [2] next free arec, brec
 };
 
@@ -724,7 +724,11 @@ __global__ void __launch_bounds__(kGroupThreads) group_place_kernel(const GroupA
 // end or behind another (in the batch's order a grab of 4 columns took 1.16 ms
 // in the numeric pass and one of 16 3.5 ms); after `singles` columns kGrab at a
 // time, which saves most of the latency of the queue and the tables.  Lanes take entries of B; an index with many
-// entries of A is walked by the whole warp.
+// entries of A is walked by the whole warp.  The symbolic pass leaves an index's
+// (end, count) in the entry of B, which saves the numeric pass one of its three
+// dependent loads (0.66 -> 0.61 ms; the symbolic pass 0.43 -> 0.45).  Reading the
+// next column's entries ahead of the accumulation gained nothing: the loads of A
+// are 16 scattered bytes per product, 3 TB/s from the L2.
 template <bool NUMERIC>
 __global__ void __launch_bounds__(kWarps * 32, 8) group_spa_kernel(const GroupArgs a, const uint2* __restrict__ order,
                                                                  u64 singles, u32* __restrict__ queue,
@@ -767,14 +771,19 @@ __global__ void __launch_bounds__(kWarps * 32, 8) group_spa_kernel(const GroupAr
       if (NUMERIC)
         for (u32 i = lane; i < h; i += 32) acc[i] = 0.0;
       __syncwarp();
-      const ulonglong2* b = a.brec + (bc.x - bc.y);
+      ulonglong2* b = a.brec + (bc.x - bc.y);
       for (u32 e0 = 0; e0 < bc.y; e0 += 32) {
         uint2 ac = make_uint2(0u, 0u);
         double beta = 0.0;
         if (e0 + lane < bc.y) {
-          const ulonglong2 rb = b[e0 + lane];
-          ac = a.acol[(u32)rb.x];  // (end, count)
-          beta = __longlong_as_double((long long)rb.y);
+          if (NUMERIC) {
+            const ulonglong2 rb = b[e0 + lane];
+            ac = make_uint2((u32)rb.x, (u32)(rb.x >> 32));
+            beta = __longlong_as_double((long long)rb.y);
+          } else {
+            ac = a.acol[(u32)b[e0 + lane].x];  // (end, count)
+            b[e0 + lane].x = (u64)ac.x | ((u64)ac.y << 32);
+          }
         }
         u32 many = __ballot_sync(0xffffffffu, ac.y >= kLong);
         while (many) {
