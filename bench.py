@@ -1642,8 +1642,8 @@ def measure_skewed(args):
     L.profile_enable(False)
     ms = max_over_ranks(e0.elapsed_time(e1) / args.steps, world)
     launches = L.launch_count() - launches0
-    names = ("spgemm_colptr", "spgemm_count", "sort_hist", "sort_onesweep", "collect", "tile_rowptr", "tile_bprep",
-             "tile_cbits", "tile_count", "tile_scan", "tile_numeric")
+    names = ("spgemm_colptr", "spgemm_count", "sort_hist", "sort_partition", "bucket_sort", "sort_onesweep", "collect",
+             "tile_rowptr", "tile_bprep", "tile_cbits", "tile_count", "tile_scan", "tile_numeric")
     kernels = {k: L.profile_query(k)[0] / args.steps for k in names}
     if rank != 0:
         return None

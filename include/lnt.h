@@ -100,8 +100,8 @@ LNT_API int lnt_profile_enable(int on);
 /* Clears all timing records. */
 LNT_API int lnt_profile_reset(void);
 /* Synchronises the recorded events and returns, for kernels of the given name
- * ("rekey", "sort_hist", "sort_onesweep", "sort_copy", "collect_lead",
- * "collect", ...), the summed device time in milliseconds and the launch
+ * ("rekey", "sort_hist", "sort_partition", "bucket_sort", "sort_onesweep",
+ * "sort_fallback", "collect", ...), the summed device time in milliseconds and the launch
  * count since the last reset. */
 LNT_API int lnt_profile_query(const char* kernel, double* total_ms, uint64_t* launches);
 
@@ -131,10 +131,11 @@ LNT_API int lnt_sort_pairs(const uint64_t* keys_in, const double* vals_in,
                    uint64_t* keys_out, double* vals_out, size_t n, uint64_t max_key,
                    void* workspace, size_t workspace_bytes, void* stream);
 
-/* Kernel variants of the sort compiled into this library (digit width, CTA
- * threads, keys per thread, look-back window); the autotuner times each one.
- * The variant used is the tuned choice, or LNT_SORT_VARIANT=<index> from the
- * environment. */
+/* Kernel variants of the digit-pass sort compiled into this library (digit
+ * width, CTA threads, keys per thread, look-back window); the autotuner times
+ * each one.  It serves the sorts that the bucketed path does not take; there the
+ * variant is the tuned choice.  LNT_SORT_VARIANT=<index> in the environment makes
+ * every sort use that variant. */
 LNT_API int lnt_sort_variant_count(void);
 LNT_API int lnt_sort_variant(int index, int* bits, int* threads, int* items, int* window);
 
@@ -337,8 +338,8 @@ LNT_API int lnt_contract_attract(const uint64_t* keys, const double* vals, size_
  * tables, including the problem of every output column, into the workspace,
  * synchronously), then lnt_batched_lattice_mult, which only enqueues kernels
  * and memsets on `stream` and can therefore be captured into a CUDA graph and
- * replayed.  Chunk size of the work queue: LNT_BATCH_CHUNK from the
- * environment, else the autotuned value (1 column). */
+ * replayed.  Chunk size of the work queue of lnt_batched_lattice_mult:
+ * LNT_BATCH_CHUNK from the environment, else the autotuned value (1 column). */
 LNT_API int lnt_batched_workspace(int count, const int64_t* dims_host, const uint64_t* a_off_host,
                                   const uint64_t* b_off_host, size_t* bytes, uint64_t* c_capacity);
 LNT_API int lnt_batched_prepare(int count, const int64_t* dims_host, const uint64_t* a_off_host,
@@ -354,11 +355,12 @@ LNT_API int lnt_batched_lattice_mult(int count, const int64_t* dims_host, const 
  * key linearised in its tensor's own mode order.  Problem p's A keys are
  * re-keyed by a_rekey_host[p] and its B keys by b_rekey_host[p] into lattice
  * order (order 0 = already in lattice order; NULL array = all order 0), and
- * both are sorted inside the call -- the per-product toLatticeSort of the
- * reference (SparseMIABase.h:1457-1586; for c(i,l) = a(i,j,k) * b(k,l,j): A
- * as it is, B to the mode order {2,0,1}, SparseMIABase.h:1527-1586) done for
- * the whole batch by one radix sort over keys prefixed with the problem index
- * -- then multiplied as lnt_batched_lattice_mult does.  Keys must lie below
+ * both are put in lattice order inside the call -- what the per-product
+ * toLatticeSort of the reference does (SparseMIABase.h:1457-1586; for c(i,l) =
+ * a(i,j,k) * b(k,l,j): A as it is, B to the mode order {2,0,1},
+ * SparseMIABase.h:1527-1586), here for the whole batch, by grouping the entries
+ * that have a partner, or by one sort of all pairs when a problem has more than
+ * 512 rows -- then multiplied.  Keys must lie below
  * their lattice's size (rows x cols x tabs).  a_off_host[0] and b_off_host[0]
  * must be 0, and the batch holds fewer than 2^30 pairs.  Call
  * lnt_batched_contract_prepare once per batch layout (synchronous uploads),
