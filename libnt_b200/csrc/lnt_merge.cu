@@ -100,11 +100,14 @@ __device__ __forceinline__ size_t run_index(const u64* __restrict__ x, size_t i,
 __device__ __forceinline__ double apply_op(int op, double a, double b) { return op == 0 ? a + b : a - b; }
 
 // splits[t] = A elements among the first min(t * kTile, na + nb) of the merge.
+// (Split: 32 bits for fewer than 2^32 pairs, which keeps the scratch at 12 bytes
+// per tile.)
+template <class Split>
 __global__ void merge_partition_kernel(const u64* __restrict__ a, size_t na, const u64* __restrict__ b, size_t nb,
-                                       u32 ntiles, u64* __restrict__ splits) {
+                                       u32 ntiles, Split* __restrict__ splits) {
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t > ntiles) return;
-  splits[t] = merge_path(a, na, b, nb, min(na + nb, (size_t)t * kTile));
+  splits[t] = (Split)merge_path(a, na, b, nb, min(na + nb, (size_t)t * kTile));
 }
 
 // Barriers of part of a CTA (ids 1..; 0 is __syncthreads).
@@ -128,9 +131,10 @@ __device__ __forceinline__ bool bar_or(int id, int threads, bool p) {
 constexpr int kMainBar = 1, kReqBar = 2, kOffBar = 4;  // the last two for both buffers
 constexpr int kMergeSmem = 2 * kPadded * 16;
 
+template <class Split>
 __global__ void __launch_bounds__(kThreads + 32, kCtas)
     merge_kernel(const u64* __restrict__ ak, const double* __restrict__ av, size_t na, const u64* __restrict__ bk,
-                 const double* __restrict__ bv, size_t nb, int op, u32 ntiles, const u64* __restrict__ splits,
+                 const double* __restrict__ bv, size_t nb, int op, u32 ntiles, const Split* __restrict__ splits,
                  unsigned long long* __restrict__ status, u32* __restrict__ tile_counter, u64* __restrict__ ck,
                  double* __restrict__ cv, u64* __restrict__ d_nout) {
   extern __shared__ u64 smem[];
@@ -372,10 +376,27 @@ static MergeLayout merge_layout(size_t n) {
   MergeLayout L;
   L.ntiles = (u32)((n + kTile - 1) / kTile);
   L.off_status = 0;
-  L.off_counter = align_up((size_t)std::max<u32>(L.ntiles, 1) * 8, 256);
-  L.off_splits = L.off_counter + 256;
-  L.total = L.off_splits + align_up(((size_t)L.ntiles + 1) * 8, 256);
+  L.off_counter = (size_t)std::max<u32>(L.ntiles, 1) * 8;
+  L.off_splits = L.off_counter + 8;
+  L.total = align_up(L.off_splits + ((size_t)L.ntiles + 1) * (n >> 32 ? 8 : 4), 256);
   return L;
+}
+
+template <class Split>
+static int run_merge(const MergeLayout& L, const u64* ak, const double* av, size_t na, const u64* bk, const double* bv,
+                     size_t nb, int op, u64* ck, double* cv, u64* d_nout, unsigned char* w, cudaStream_t s) {
+  Split* splits = reinterpret_cast<Split*>(w + L.off_splits);
+  if (cudaMemsetAsync(w, 0, L.off_splits, s) != cudaSuccess) return LNT_DEVICE_ERROR;
+  if (cudaFuncSetAttribute(merge_kernel<Split>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMergeSmem) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  ProfScope prof("merge", s);
+  merge_partition_kernel<Split><<<(L.ntiles + 1 + 255) / 256, 256, 0, s>>>(ak, na, bk, nb, L.ntiles, splits);
+  const u32 grid = std::min<u32>(L.ntiles, (u32)kCtas * (u32)sm_count());
+  merge_kernel<Split><<<grid, kThreads + 32, kMergeSmem, s>>>(
+      ak, av, na, bk, bv, nb, op, L.ntiles, splits, reinterpret_cast<unsigned long long*>(w + L.off_status),
+      reinterpret_cast<u32*>(w + L.off_counter), ck, cv, d_nout);
+  count_launch(2);
+  return launch_status();
 }
 
 }  // namespace lnt
@@ -421,23 +442,9 @@ int lnt_merge_sorted(const uint64_t* a_keys, const double* a_vals, size_t na, co
   if (!c_keys || !c_vals) return LNT_BAD_ARG;
   MergeLayout L = merge_layout(n);
   if (!workspace || workspace_bytes < L.total) return LNT_WORKSPACE;
-  if (cudaMemsetAsync(workspace, 0, L.off_splits, s) != cudaSuccess) return LNT_DEVICE_ERROR;
-  unsigned char* w = static_cast<unsigned char*>(workspace);
-  u64* splits = reinterpret_cast<u64*>(w + L.off_splits);
-  {
-    ProfScope prof("merge", s);
-    merge_partition_kernel<<<(L.ntiles + 1 + 255) / 256, 256, 0, s>>>((const u64*)a_keys, na, (const u64*)b_keys, nb,
-                                                                       L.ntiles, splits);
-    if (cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMergeSmem) != cudaSuccess)
-      return LNT_DEVICE_ERROR;
-    const u32 grid = std::min<u32>(L.ntiles, (u32)kCtas * (u32)sm_count());
-    merge_kernel<<<grid, kThreads + 32, kMergeSmem, s>>>((const u64*)a_keys, a_vals, na, (const u64*)b_keys, b_vals, nb, op,
-                                               L.ntiles, splits, reinterpret_cast<unsigned long long*>(w + L.off_status),
-                                               reinterpret_cast<u32*>(w + L.off_counter), (u64*)c_keys, c_vals,
-                                               (u64*)d_nout);
-  }
-  count_launch(2);
-  return launch_status();
+  auto run = n >> 32 ? run_merge<u64> : run_merge<u32>;
+  return run(L, (const u64*)a_keys, a_vals, na, (const u64*)b_keys, b_vals, nb, op, (u64*)c_keys, c_vals, (u64*)d_nout,
+             static_cast<unsigned char*>(workspace), s);
 }
 
 int lnt_permute_sort_workspace(size_t n, uint64_t max_key, size_t* bytes) {

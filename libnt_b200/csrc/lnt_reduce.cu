@@ -413,9 +413,9 @@ struct SortReduceLayout {
   size_t off_ctrl, off_k0, off_v0, off_k1, off_v1, off_coll, off_gate, total;
 };
 
-SortReduceLayout sort_reduce_layout(size_t n, u64 max_key) {
+SortReduceLayout sort_reduce_layout(size_t n, u64 max_key, bool buckets = true) {
   SortReduceLayout L;
-  L.msd = make_msd_plan(n, max_key);
+  if (buckets) L.msd = make_msd_plan(n, max_key);
   L.plan = make_sort_plan(n, max_key, L.msd.ok);
   size_t off = 0;
   L.off_ctrl = off;
@@ -482,6 +482,7 @@ int lnt_sort_reduce(const uint64_t* a_keys, const double* a_vals, size_t na, con
   cudaStream_t s = as_stream(stream);
   if (n == 0) return run_collect(nullptr, nullptr, 0, skip_zero_heads, nullptr, nullptr, (u64*)d_nout, nullptr, s);
   SortReduceLayout L = sort_reduce_layout(n, max_key);
+  if (workspace_bytes < L.total) L = sort_reduce_layout(n, max_key, false);  // the digit passes may need less
   if (!workspace || workspace_bytes < L.total) return LNT_WORKSPACE;
   if ((uintptr_t)workspace % 256) return LNT_BAD_ARG;
   PairSource src;

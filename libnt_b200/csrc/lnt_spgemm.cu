@@ -42,7 +42,7 @@ int run_collect(const u64* keys, const double* vals, size_t n, int skip_zero_hea
                 u64* d_nout, void* ws, cudaStream_t s);
 size_t collect_workspace_bytes(size_t n);
 bool tile_shape_ok(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb);
-size_t tile_workspace_bytes(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb);
+size_t tile_workspace_bytes(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb, bool buckets);
 int run_tile_mult(const u64* akeys, const double* avals, u64 na, const u64* bkeys, const double* bvals, u64 nb,
                   u64 h, u64 w, u64 wB, u64 d, void* ws, size_t ws_bytes, u64* ck, double* cv, u64* d_nc,
                   cudaStream_t s);
@@ -416,9 +416,9 @@ struct EscLayout {
   size_t off_ctrl, off_a, off_b, off_coll, total;
 };
 
-EscLayout esc_layout(u64 products, u64 max_key) {
+EscLayout esc_layout(u64 products, u64 max_key, bool buckets = true) {
   EscLayout L;
-  L.sort = make_pair_sort(products, max_key);
+  L.sort = make_pair_sort(products, max_key, buckets);
   L.pair_bytes = 2 * align_up(products * 8, 256);
   size_t off = 0;
   L.off_ctrl = off;
@@ -527,7 +527,7 @@ int lnt_lattice_mult_workspace(const lnt_lattice* a, const lnt_lattice* b, uint6
     return LNT_OK;
   }
   if (eng == Engine::Tile) {
-    *bytes = tile_workspace_bytes(s.h, s.w, s.wB, s.d, s.A.nnz, s.B.nnz);
+    *bytes = tile_workspace_bytes(s.h, s.w, s.wB, s.d, s.A.nnz, s.B.nnz, true);
     return LNT_OK;
   }
   if (products >= (1ull << 30)) return LNT_UNSUPPORTED;
@@ -553,9 +553,13 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   size_t need = 0;
   st = lnt_lattice_mult_workspace(a, b, products, &need);
   if (st != LNT_OK) return st;
+  const Engine eng = choose_engine(s, products);
+  const bool buckets = workspace_bytes >= need;  // else sort by digit passes, which may need less
+  if (!buckets && eng == Engine::Esc) need = esc_layout(products, s.h * s.wB * s.d, false).total + esc_prefix_bytes(s);
+  if (!buckets && eng == Engine::Tile)
+    need = tile_workspace_bytes(s.h, s.w, s.wB, s.d, s.A.nnz, s.B.nnz, false);
   if (workspace_bytes < need || (need > 256 && !workspace)) return LNT_WORKSPACE;
   if (products && (!c_keys || !c_vals)) return LNT_BAD_ARG;
-  const Engine eng = choose_engine(s, products);
   if (eng == Engine::Tile)
     return run_tile_mult(s.A.keys, s.A.vals, s.A.nnz, s.B.keys, s.B.vals, s.B.nnz, s.h, s.w, s.wB, s.d, workspace,
                          workspace_bytes, (u64*)c_keys, c_vals, (u64*)d_nc, cs);
@@ -574,7 +578,7 @@ int lnt_lattice_mult(const lnt_lattice* a, const lnt_lattice* b, const void* pla
   }
   // ESC
   if (products == 0) return cudaMemsetAsync(d_nc, 0, 8, cs) == cudaSuccess ? LNT_OK : LNT_DEVICE_ERROR;
-  const EscLayout E = esc_layout(products, s.h * s.wB * s.d);
+  const EscLayout E = esc_layout(products, s.h * s.wB * s.d, buckets);
   unsigned char* w = static_cast<unsigned char*>(workspace);
   void* ctrl = w + E.off_ctrl;
   if (spa_eligible(s)) {

@@ -115,9 +115,9 @@ struct TileLayout {
   SortPlan pb;   // B's have the skewed contracted index on top: LSD
 };
 
-TileLayout tile_layout(const TileDims& t, u64 na, u64 nb) {
+TileLayout tile_layout(const TileDims& t, u64 na, u64 nb, bool buckets = true) {
   TileLayout L;
-  L.pa = make_pair_sort(na, t.h * t.w * t.d);
+  L.pa = make_pair_sort(na, t.h * t.w * t.d, buckets);
   L.pb = make_sort_plan(nb, t.w * t.wB * t.d);
   const u64 ncnt = t.d * t.wB * t.np;
   const u64 nmax = std::max(na, nb);
@@ -546,15 +546,16 @@ bool tile_shape_ok(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb) {
   return cb <= kMaxBitmapBytes && bb <= kMaxBitmapBytes && cn <= kMaxBitmapBytes;
 }
 
-size_t tile_workspace_bytes(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb) {
-  return tile_layout(tile_dims(h, w, wB, d, nb), na, nb).total;
+size_t tile_workspace_bytes(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb, bool buckets) {
+  return tile_layout(tile_dims(h, w, wB, d, nb), na, nb, buckets).total;
 }
 
 int run_tile_mult(const u64* akeys, const double* avals, u64 na, const u64* bkeys, const double* bvals, u64 nb,
                   u64 h, u64 w, u64 wB, u64 d, void* ws, size_t ws_bytes, u64* ck, double* cv, u64* d_nc,
                   cudaStream_t s) {
   const TileDims t = tile_dims(h, w, wB, d, nb);
-  const TileLayout L = tile_layout(t, na, nb);
+  TileLayout L = tile_layout(t, na, nb);
+  if (ws_bytes < L.total) L = tile_layout(t, na, nb, false);  // A by digit passes needs less
   if (!ws || ws_bytes < L.total || (uintptr_t)ws % 256) return LNT_WORKSPACE;
   unsigned char* W = static_cast<unsigned char*>(ws);
   auto at = [&](size_t off) { return static_cast<void*>(W + off); };

@@ -175,3 +175,73 @@ def test_scratch_of_the_digit_passes_is_enough(cuda, torch, rng, monkeypatch, en
         np.testing.assert_array_equal(to_host(ov), vals[order])
     assert call(min(need.value, have.value) - 1) == 5  # LNT_WORKSPACE
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("engine", ["esc", "tile"])
+def test_products_with_the_scratch_of_the_digit_passes(cuda, torch, rng, monkeypatch, engine):
+    """The lattice product's engines likewise: the same C from either scratch."""
+    import ctypes as C
+    import libnt_b200 as L
+    h, w, wB, d = 1500, 60, 40, 2
+    ak = np.sort(rng.choice(h * w * d, 60000, replace=False)).astype(np.uint64)
+    bk = np.sort(rng.choice(w * wB * d, 1500, replace=False)).astype(np.uint64)
+    av, bv = rng.uniform(-1, 1, ak.size), rng.uniform(-1, 1, bk.size)
+    da, dav, db, dbv = (to_dev(x, torch) for x in (ak, av, bk, bv))
+    monkeypatch.setenv("LNT_SPGEMM_ENGINE", engine)
+    A, B = L.Lattice.of(da, dav, h, w, d), L.Lattice.of(db, dbv, w, wB, d)
+    n = C.c_size_t(0)
+    assert L.lib().lnt_lattice_mult_plan_workspace(C.byref(A), C.byref(B), C.byref(n)) == 0
+    plan = L.workspace(n.value)
+    counts = torch.empty(2, dtype=torch.int64, device="cuda")
+    assert L.lib().lnt_lattice_mult_plan(C.byref(A), C.byref(B), C.c_void_p(plan.data_ptr()), plan.numel(),
+                                         C.c_void_p(counts.data_ptr()), None) == 0
+    torch.cuda.synchronize()
+    products, cap = (int(x) for x in counts.tolist())
+    monkeypatch.setenv("LNT_NO_BUCKETS", "1")
+    need = C.c_size_t(0)
+    assert L.lib().lnt_lattice_mult_workspace(C.byref(A), C.byref(B), products, C.byref(need)) == 0
+    monkeypatch.delenv("LNT_NO_BUCKETS")
+    have = C.c_size_t(0)
+    assert L.lib().lnt_lattice_mult_workspace(C.byref(A), C.byref(B), products, C.byref(have)) == 0
+    ek, ev, ea = oracle.lattice_mult(ak, av, h, w, d, bk, bv, wB, with_abs=True)
+    for nbytes in (need.value, have.value):
+        ws = L.workspace(nbytes)
+        ck = torch.empty(cap, dtype=torch.int64, device="cuda")
+        cv = torch.empty(cap, dtype=torch.float64, device="cuda")
+        nc = torch.empty(1, dtype=torch.int64, device="cuda")
+        assert L.lib().lnt_lattice_mult(C.byref(A), C.byref(B), C.c_void_p(plan.data_ptr()), products,
+                                        C.c_void_p(ws.data_ptr()), nbytes, C.c_void_p(ck.data_ptr()),
+                                        C.c_void_p(cv.data_ptr()), C.c_void_p(nc.data_ptr()), None) == 0
+        m = int(nc.item())
+        np.testing.assert_array_equal(to_host(ck[:m], np.uint64), ek)
+        assert rel_ok(to_host(cv[:m]), ev, ea)
+    assert cuda.device_status() == 0
+
+
+def test_sort_reduce_with_the_scratch_of_the_digit_passes(cuda, torch, rng, monkeypatch):
+    import ctypes as C
+    import libnt_b200 as L
+    n, bits = 1 << 20, 36
+    keys = rng.integers(0, 1 << bits, n).astype(np.uint64)
+    keys[: n // 8] = keys[n // 8: n // 4]
+    vals = rng.uniform(-1, 1, n)
+    monkeypatch.setenv("LNT_NO_BUCKETS", "1")
+    need = L.sort_reduce_workspace(n, 0, 1 << bits)
+    monkeypatch.delenv("LNT_NO_BUCKETS")
+    k, v = to_dev(keys, torch), to_dev(vals, torch)
+    got = []
+    for nbytes in (need, max(need, L.sort_reduce_workspace(n, 0, 1 << bits))):
+        ws = L.workspace(nbytes)
+        ok, ov = torch.empty_like(k), torch.empty_like(v)
+        cnt = torch.zeros(1, dtype=torch.int64, device="cuda")
+        assert L.lib().lnt_sort_reduce(C.c_void_p(k.data_ptr()), C.c_void_p(v.data_ptr()), n, None, None, None, 0, None,
+                                       1.0, 1 << bits, 1, C.c_void_p(ok.data_ptr()), C.c_void_p(ov.data_ptr()),
+                                       C.c_void_p(cnt.data_ptr()), C.c_void_p(ws.data_ptr()), nbytes, None) == 0
+        m = int(cnt.item())
+        got.append((to_host(ok[:m], np.uint64), to_host(ov[:m])))
+    sk, sv = oracle.sort_pairs(keys, vals)
+    ek, ev = oracle.collect_duplicates(sk, sv)[:2]
+    for gk, gv in got:
+        np.testing.assert_array_equal(gk, ek)
+        np.testing.assert_array_equal(gv, ev)
+    assert cuda.device_status() == 0
