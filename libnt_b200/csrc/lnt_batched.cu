@@ -1249,13 +1249,15 @@ int lnt_batched_contract_prepare(int count, const int64_t* dims_host, const uint
     if (c.bytes && cudaMemcpy(w + c.off, c.src, c.bytes, cudaMemcpyHostToDevice) != cudaSuccess)
       return LNT_DEVICE_ERROR;
   if (C.grouped) {
-    group_order_kernel<<<(unsigned)count, 128, 0, s>>>(reinterpret_cast<const ProbDesc*>(w + L.off_prob),
-                                                       reinterpret_cast<const uint2*>(w + C.off_porder),
-                                                       reinterpret_cast<uint2*>(w + C.off_order));
+    // on the stream of the copies, behind them
+    group_order_kernel<<<(unsigned)count, 128, 0, cudaStreamLegacy>>>(
+        reinterpret_cast<const ProbDesc*>(w + L.off_prob), reinterpret_cast<const uint2*>(w + C.off_porder),
+        reinterpret_cast<uint2*>(w + C.off_order));
     count_launch();
-    return launch_status();
+    if (launch_status() != LNT_OK) return LNT_DEVICE_ERROR;
   }
-  return LNT_OK;
+  // the tables are complete when the call returns, for whichever stream runs the batch
+  return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? LNT_OK : LNT_DEVICE_ERROR;
 }
 
 int lnt_batched_contract(int count, const int64_t* dims_host, const uint64_t* a_off_host, const uint64_t* b_off_host,
