@@ -407,23 +407,26 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
 // (zero the control block, histogram, the tiles of every pass) in order from a
 // queue; a task waits until the step before is complete, whose tasks all
 // belong to running CTAs.  gate[1]: queue, gate[2 + step]: tasks done; zeroed
-// by whoever writes the gate.
+// by whoever writes the gate.  A CTA whose wait ran out waits no more (there
+// may be hundreds of tasks left) and goes on: the error is latched, and every
+// write stays inside the output whatever the histogram holds (see the clamp in
+// onesweep_tile).
 constexpr int kQBits = 8, kQItems = 16, kQWindow = 16;
 using QueueShape = OnesweepShape<kQBits, kThreads, kQItems>;
 
-__device__ __forceinline__ void queue_wait(const u32* done, u32 want) {
+// True when the wait ran out.
+__device__ __forceinline__ bool queue_wait(const u32* done, u32 want) {
+  bool expired = false;
   if (threadIdx.x == 0) {
     u32 spins = 0;
-    while (ld_volatile(done) < want) {
+    while (!expired && ld_volatile(done) < want) {
       __nanosleep(100);
-      if (++spins > spin_limit()) {
-        latch_error(kErrSortLookback);
-        break;
-      }
+      expired = ++spins > spin_limit();
     }
+    if (expired) latch_error(kErrSortLookback);
     __threadfence();
   }
-  __syncthreads();
+  return __syncthreads_or(expired) != 0;
 }
 __device__ __forceinline__ void queue_done(u32* done) {
   __threadfence();
@@ -445,6 +448,7 @@ __global__ void __launch_bounds__(kThreads, QueueShape::MINB)
   u32* bstart = reinterpret_cast<u32*>(ctrl + plan.off_bstart);
   u32* status = reinterpret_cast<u32*>(ctrl + plan.off_status);
   u32* counters = reinterpret_cast<u32*>(ctrl + plan.off_counters);
+  bool expired = false;  // (the same in all threads)
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_task = atomicAdd(&gate[1], 1u);
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, QueueShape::MINB)
     }
     t -= nz;
     if (t < nh) {
-      queue_wait(&gate[2], nz);
+      if (!expired) expired = queue_wait(&gate[2], nz);
       hist_block<kQBits>(src, plan.n, plan.passes, plan.key_bits, ghist, bstart, counters + plan.passes,
                          reinterpret_cast<u32*>(smem), t, nh);
       queue_done(&gate[3]);
@@ -468,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, QueueShape::MINB)
     t -= nh;
     const int p = (int)(t / plan.ntiles);
     if (p >= plan.passes) return;
-    queue_wait(&gate[3 + p], p == 0 ? nh : plan.ntiles);
+    if (!expired) expired = queue_wait(&gate[3 + p], p == 0 ? nh : plan.ntiles);
     const int which = (plan.passes - 1 - p) & 1, shift = p * kQBits;
     const u32 mask = (1u << min(kQBits, plan.key_bits - shift)) - 1u;
     u64* ok = which ? buf1_k : buf0_k;
