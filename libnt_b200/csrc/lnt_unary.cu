@@ -169,17 +169,20 @@ struct CountOf {
 };
 
 // Chunk i's partial sums (at i * chunk) to pos[i] (one warp per chunk).
+// (counts, not pos[i + 1] - pos[i]: after an expired look-back of the scan that
+// difference could be negative.)
 __global__ void __launch_bounds__(256) unary_gather_kernel(const u64* __restrict__ gk, const double* __restrict__ gv,
-                                                           u32 chunk, u32 nchunks,
+                                                           const u32* __restrict__ counts, u32 chunk, u32 nchunks,
                                                            const unsigned long long* __restrict__ pos,
                                                            u64* __restrict__ ck, double* __restrict__ cv) {
   const int lane = threadIdx.x & 31;
   const u32 ci = (u32)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   if (ci >= nchunks) return;
-  const u64 to = pos[ci], cnt = pos[ci + 1] - to;
+  const u64 to = pos[ci];
+  const u32 cnt = counts[ci];
   const size_t from = (size_t)ci * chunk;
 #pragma unroll 4
-  for (u64 j = lane; j < cnt; j += 32) {
+  for (u32 j = lane; j < cnt; j += 32) {
     ck[to + j] = gk[from + j];
     cv[to + j] = gv[from + j];
   }
@@ -340,7 +343,7 @@ int lnt_contract_attract(const uint64_t* keys, const double* vals, size_t n, int
   if (st != LNT_OK) return st;
   {
     ProfScope prof("unary_gather", s);
-    unary_gather_kernel<<<blocks, 256, 0, s>>>(gk, gv, L.chunk, L.nchunks, pos, ck, cv);
+    unary_gather_kernel<<<blocks, 256, 0, s>>>(gk, gv, counts, L.chunk, L.nchunks, pos, ck, cv);
     count_launch();
   }
   st = collect::run(ck, cv, (const u64*)(pos + L.nchunks), n, UnaryGroups{P}, (u64*)out_keys, out_vals, (u64*)d_nout,
