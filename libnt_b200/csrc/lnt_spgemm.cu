@@ -137,7 +137,10 @@ struct Identity64 {
 // by two searches for the tile, not one per product) are decoded once each
 // into shared memory; their first products are marked and a maximum scan gives
 // every product its entry.  Then a product costs its A entry's load and its
-// store.  17.4M products of 1M x 1.1M entries: 0.49 -> 0.12 ms.
+// store.  17.4M products of 1M x 1.1M entries: 0.49 -> 0.12 ms.  The bounds on a
+// mark and on an A position change nothing in a correct run; they keep the
+// accesses inside when the prefix is not ascending because a look-back of its
+// scan gave up.
 constexpr int kExpandThreads = 256;
 constexpr int kExpandTile = 2048;
 constexpr int kExpandEntries = 1024;  // decoded B entries a tile has room for
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AC
     for (u64 p = p0 + tid; p < p1; p += kExpandThreads) {
       const u64 e = entry_of(boff, e0, e0 + ne - 1, p);
       const ExpandEntry q = expand_entry(A, B, ac, boff[e], e, div_w, div_wB);
-      const u64 x = q.x0 + p;
+      const u64 x = min(q.x0 + p, A.nnz - 1);
       pk[p] = A.keys[x] + q.kshift;
       pv[p] = A.vals[x] * q.beta;
     }
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AC
     // (of the entries that start at one product only the last has products)
     if (boff[e0 + i + 1] > b) {
       s_e[i] = expand_entry(A, B, ac, b, e0 + i, div_w, div_wB);
-      if (b > p0) s_ent[b - p0] = (unsigned short)i;  // (entry 0 covers the tile's start)
+      if (b > p0 && b < p1) s_ent[b - p0] = (unsigned short)i;  // (entry 0 covers the tile's start)
     }
   }
   __syncthreads();
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AC
     const u32 o = j * kExpandThreads + tid;
     if (p0 + o < p1) {
       const ExpandEntry q = s_e[s_ent[o]];
-      const u64 x = q.x0 + p0 + o;
+      const u64 x = min(q.x0 + p0 + o, A.nnz - 1);
       pk[p0 + o] = A.keys[x] + q.kshift;
       pv[p0 + o] = A.vals[x] * q.beta;
     }
