@@ -374,9 +374,10 @@ __device__ __forceinline__ u64 word_of(const ulonglong2& r) { return r.x; }
 __device__ __forceinline__ u64 word_of(u64 w) { return w; }
 
 // Sorts the records s_r[0, cap) by word in place (cap = BT * ITEMS; the unused
-// ones hold ~0): ITEMS records per thread by odd-even transposition, then
-// merge rounds over doubling groups of threads, each thread finding its output
-// range by a merge-path search.
+// ones, behind the others, hold ~0): ITEMS records per thread by odd-even
+// transposition, then merge rounds over doubling groups of threads, each thread
+// finding its output range by a merge-path search.  Stable throughout: a record
+// whose word is ~0 too stays in front of the unused ones.
 template <int BT, int I, class R>
 __device__ __noinline__ void bucket_merge_sort(R* s_r) {
   const int tid = threadIdx.x;
@@ -388,9 +389,9 @@ __device__ __noinline__ void bucket_merge_sort(R* s_r) {
 #pragma unroll
     for (int j = r & 1; j + 1 < I; j += 2) {
       const R p = x[j], q = x[j + 1];
-      const bool lt = word_of(p) < word_of(q);
-      x[j] = lt ? p : q;
-      x[j + 1] = lt ? q : p;
+      const bool keep = word_of(p) <= word_of(q);
+      x[j] = keep ? p : q;
+      x[j + 1] = keep ? q : p;
     }
 #pragma unroll
   for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
