@@ -116,6 +116,7 @@ int make_rekey_params(int order, const int64_t* dims, const int32_t* cur_seq,
   out->order = 0;
   out->pow2 = 0;
   out->narrow = 0;
+  out->narrow_bits = 0;
   if (order <= 1) return order < 0 ? LNT_BAD_ARG : LNT_OK;
   if (order > LNT_MAX_ORDER || !dims || !cur_seq || !new_seq) return LNT_BAD_ARG;
   if (!is_permutation(order, cur_seq) || !is_permutation(order, new_seq)) return LNT_BAD_SEQ;
@@ -152,7 +153,28 @@ int make_rekey_params(int order, const int64_t* dims, const int32_t* cur_seq,
     short_modes = short_modes && dims[i] < ((int64_t)1 << 31);
     out->inv[i] = 1.0 / (double)out->acc[i].d;
   }
-  out->narrow = total <= ((unsigned __int128)1 << 31) ? 1 : total <= ((unsigned __int128)1 << 52) && short_modes ? 2 : 0;
+  // The shorter arithmetics take keys below 2^narrow_bits, which every key
+  // of the tensor is, and beyond the tensor only as far as the quotient by the
+  // last cumulative extent (the one digit that its extent does not bound)
+  // and the result fit them; larger keys are re-keyed in 64 bits as before.
+  out->narrow = 0;
+  out->narrow_bits = 0;
+  const u64 top = out->acc[order - 1].d, top_mult = out->mult[order - 1];
+  unsigned __int128 others = 0;  // the largest contribution of the other modes
+  for (int i = 0; i + 1 < order; ++i) others += (unsigned __int128)(dims[cur_seq[i]] - 1) * out->mult[i];
+  auto widest = [&](int most, auto fits) {
+    for (int b = most; b >= 0 && ((unsigned __int128)1 << b) >= total; --b)
+      if (fits((((u64)1 << b) - 1) / top)) return b;
+    return 0;
+  };
+  if (total <= ((unsigned __int128)1 << 31)) {
+    out->narrow_bits = widest(32, [&](u64 q) { return ((others + (unsigned __int128)q * top_mult) >> 32) == 0; });
+    out->narrow = out->narrow_bits ? 1 : 0;
+  }
+  if (!out->narrow && total <= ((unsigned __int128)1 << 52) && short_modes) {
+    out->narrow_bits = widest(52, [&](u64 q) { return q < 0xFFFFFFFFull; });
+    out->narrow = out->narrow_bits ? 2 : 0;
+  }
   if (pow2) {
     for (int i = 0; i < order; ++i) {
       const u32 src = (u32)__builtin_ctzll(out->acc[i].d);

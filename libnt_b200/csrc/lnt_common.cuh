@@ -166,7 +166,8 @@ __device__ __forceinline__ u32 divide32(u32 n, const Divider& dv) {
 struct RekeyParams {
   int order;        // 0 or 1 => identity
   int pow2;         // every extent a power of two: `field` holds the bit-field moves
-  int narrow;       // 1: keys below 2^31, 32-bit arithmetic; 2: keys below 2^52 and extents below 2^31, `inv`
+  int narrow;       // for keys below 2^narrow_bits: 1: 32-bit arithmetic; 2: extents below 2^31, `inv`
+  int narrow_bits;  // (1: at most 32, 2: at most 52)
   Divider acc[LNT_MAX_ORDER];  // cumulative extents, current order
   u64 mult[LNT_MAX_ORDER];     // new stride of the mode at current position i
   u32 field[LNT_MAX_ORDER];    // pow2: source shift | bits << 8 | destination shift << 16
@@ -235,7 +236,7 @@ __device__ __forceinline__ void rekey_items(u64 (&k)[I], const RekeyParams& p, u
   u64 high = 0;
 #pragma unroll
   for (int j = 0; j < I; ++j) high |= use & (1u << j) ? k[j] : 0ull;
-  if (p.narrow == 1 && (high >> 32) == 0) {
+  if (p.narrow == 1 && (high >> p.narrow_bits) == 0) {
     // 32 bits: six instructions per mode and key instead of some 28
     u32 r[I], o[I];
 #pragma unroll
@@ -260,8 +261,8 @@ __device__ __forceinline__ void rekey_items(u64 (&k)[I], const RekeyParams& p, u
       if (use & (1u << j)) k[j] = (u64)(o[j] + r[j] * m0);
     return;
   }
-  if (p.narrow == 2 && (high >> 52) == 0) {
-    // k is exact as a double and k / acc < 2^31 is at most one unit of its
+  if (p.narrow == 2 && (high >> p.narrow_bits) == 0) {
+    // k is exact as a double and k / acc < 2^32 is at most one unit of its
     // nearest integer away: round the product with 1 / acc, and correct
     constexpr double kTwo52 = 4503599627370496.0;
 #pragma unroll 1
