@@ -845,15 +845,18 @@ __global__ void __launch_bounds__(256) abs_stat_kernel(const double* __restrict_
   }
 }
 
-// max / mean over the rows (rows of all tabs).
+// max / mean over the rows (rows of all tabs).  Compared by bits, like the
+// columns': a row with an infinity has the ratio NaN, which is above every
+// number either way.
 __global__ void row_ratio_kernel(const unsigned long long* __restrict__ rmax, const double* __restrict__ rsum, u64 rows,
                                  u64 w, unsigned long long* __restrict__ out) {
   const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  double r = 0.0;
-  if (i < rows && rsum[i] > 0.0) r = __longlong_as_double((long long)rmax[i]) * (double)w / rsum[i];
+  unsigned long long r = 0;
+  if (i < rows && rsum[i] > 0.0)
+    r = (unsigned long long)__double_as_longlong(__longlong_as_double((long long)rmax[i]) * (double)w / rsum[i]);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
-  if ((threadIdx.x & 31) == 0 && r > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(r));
+  for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+  if ((threadIdx.x & 31) == 0 && r) atomicMax(out, r);
 }
 
 struct CrtLayout {
