@@ -247,10 +247,13 @@ __global__ void __launch_bounds__(kExpandThreads) expand_kernel(Lat A, Lat B, AC
 }
 
 // ---- SPA engine ----------------------------------------------------------
-// One warp per output column; with few columns (BLOCK) one CTA per column, its
-// four warps sharing the accumulators: a column of 100 entries then takes one
-// round of dependent loads instead of four (100 columns: 10.4 -> 5.2 us numeric,
-// 7.4 -> 4.6 us symbolic).  The symbolic pass also counts the products.
+// One warp per output column; with few columns (BLOCK) one CTA per column: a
+// column of 100 entries then takes one round of dependent loads of its four
+// warps instead of four of one (100 columns: 10.4 -> 5.2 us numeric, 7.4 -> 4.6 us
+// symbolic).  Every warp has accumulators of its own, added up in the warps'
+// order at the end, so that a result does not depend on which warp was faster
+// (one set for all four took the same time).  The symbolic pass also counts the
+// products.
 template <bool NUMERIC, bool BLOCK>
 __global__ void __launch_bounds__(kSpaWarps * 32) spa_kernel(Lat A, Lat B, AColumns ac, const u64* __restrict__ bptr,
                                                               u64 units, u64* __restrict__ ucount,
@@ -260,13 +263,13 @@ __global__ void __launch_bounds__(kSpaWarps * 32) spa_kernel(Lat A, Lat B, AColu
   constexpr int N = BLOCK ? 1 : kSpaWarps;
   constexpr int T = BLOCK ? kSpaWarps * 32 : 32;  // threads per column
   __shared__ u32 s_bits[N][kSpaMaxRows / 32];
-  __shared__ double s_acc[NUMERIC ? N : 1][NUMERIC ? kSpaMaxRows : 1];
+  __shared__ double s_acc[NUMERIC ? kSpaWarps : 1][NUMERIC ? kSpaMaxRows : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ct = BLOCK ? threadIdx.x : lane;
   const u64 h = A.rows, w = A.cols, wB = B.cols;
   const int hw = (int)((h + 31) / 32);  // at most 32
   u32* bits = s_bits[BLOCK ? 0 : warp];
-  double* acc = s_acc[NUMERIC && !BLOCK ? warp : 0];
+  double* acc = s_acc[NUMERIC ? warp : 0];
   auto sync = [] {
     if (BLOCK) __syncthreads();
     else __syncwarp();
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(kSpaWarps * 32) spa_kernel(Lat A, Lat B, AColu
     }
     for (int i = ct; i < hw; i += T) bits[i] = 0u;
     if (NUMERIC)
-      for (int i = ct; i < (int)h; i += T) acc[i] = 0.0;
+      for (int i = lane; i < (int)h; i += 32) acc[i] = 0.0;
     sync();
     const u64 t = u / wB;
     for (u64 e = e0 + ct; e < e1; e += T) {
@@ -318,8 +321,14 @@ __global__ void __launch_bounds__(kSpaWarps * 32) spa_kernel(Lat A, Lat B, AColu
         if (word & (1u << lane)) {
           const u32 r = (u32)g * 32 + lane;
           const u64 o = out + before + __popc(word & ((1u << lane) - 1u));
+          double v = acc[r];
+          if (BLOCK) {
+            v = s_acc[0][r];
+#pragma unroll
+            for (int q = 1; q < (NUMERIC ? kSpaWarps : 1); ++q) v += s_acc[q][r];
+          }
           ck[o] = colkey + r;
-          cv[o] = acc[r];
+          cv[o] = v;
         }
       }
     }
