@@ -360,7 +360,12 @@ LNT_API int lnt_batched_lattice_mult(int count, const int64_t* dims_host, const 
  * a(i,j,k) * b(k,l,j): A as it is, B to the mode order {2,0,1},
  * SparseMIABase.h:1527-1586), here for the whole batch, by grouping the entries
  * that have a partner, or by one sort of all pairs when a problem has more than
- * 512 rows -- then multiplied.  Keys must lie below
+ * 512 rows (one such problem sorts the whole batch, about four times the time)
+ * -- then multiplied.  Grouped entries are added up in an order that differs
+ * from run to run, and with it the last bits of the sums: where the same bits
+ * are wanted on every run, sort the operands once and call
+ * lnt_batched_lattice_mult.  (That call, a batch with a taller problem, and
+ * every other call that returns sums add up in a fixed order.)  Keys must lie below
  * their lattice's size (rows x cols x tabs).  a_off_host[0] and b_off_host[0]
  * must be 0, and the batch holds fewer than 2^30 pairs.  Call
  * lnt_batched_contract_prepare once per batch layout (synchronous uploads),

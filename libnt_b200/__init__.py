@@ -476,7 +476,8 @@ class Batch:
     Without re-key specs the operands are key-sorted lattices
     (lnt_batched_lattice_mult); with a_rekey / b_rekey (a sequence of count
     RekeySpec, or None for "already in lattice order") they are unsorted tensors
-    that the call re-keys and sorts (lnt_batched_contract)."""
+    that the call re-keys and groups (lnt_batched_contract); the last bits of its
+    sums may differ from run to run."""
 
     def __init__(self, dims, a_off, b_off, a_keys, a_vals, b_keys, b_vals, a_rekey=None, b_rekey=None):
         torch = _torch()

@@ -35,8 +35,12 @@
 //   filter: a second read keeps the entries with a partner (their values are
 //           read only now), counts A's per contracted index and B's per output
 //           column;
-//   base, place: room for every group, and the entries into their groups (in any
-//           order: the sums are accumulated by atomics anyway);
+//   base, place: room for every group, and the entries into their groups, in the
+//           order in which their atomics come: the products then add up in an
+//           order that differs from run to run (the sorted operands of
+//           lnt_batched_lattice_mult add up in a fixed one).  Sorting the groups
+//           to fix the order was measured at 0.7 ms on the batch below, a quarter
+//           of the call;
 //   then spa<symbolic>, scan, spa<numeric> and coff as above on the groups.
 // The work is cut into tasks of one operand of one problem (at most 64 K
 // entries, less when the batch is small), largest first.
