@@ -41,6 +41,7 @@ constexpr int kMaxT = 15;
 // fallback behind it takes 18-21 us against 33-57 us for the digit passes (20
 // to 50 key bits); below, the histogram and one CTA are all there is to gain.
 constexpr size_t kMinPairs = 2048;
+constexpr double kMaxPerKey = 24.0;
 constexpr int kMaxDigits = 256;
 // Partition tile: 256 threads x 8 records, four CTAs per SM at 64 registers.
 // What matters is that nothing spills: 12 records per thread ran the same
@@ -74,6 +75,7 @@ using GeomSmall = BucketGeom<256, 10, 13>;
 // largest expected bucket (uniform keys): four fifths of the capacity
 constexpr double kAvgLarge = 4096.0, kAvgSmall = 2048.0;
 constexpr int kSubMax = 48;  // largest sub-bucket ranked by comparing its words
+constexpr int kSubThread = 8;  // largest one sorted (and folded) by a single thread
 
 struct MsdCtrl {
   u32* counts;    // 2^T
@@ -379,7 +381,7 @@ __device__ __forceinline__ u64 word_of(u64 w) { return w; }
 // finding its output range by a merge-path search.  Stable throughout: a record
 // whose word is ~0 too stays in front of the unused ones.
 template <int BT, int I, class R>
-__device__ __noinline__ void bucket_merge_sort(R* s_r) {
+__device__ __forceinline__ void bucket_merge_sort(R* s_r) {
   const int tid = threadIdx.x;
   R x[I];
 #pragma unroll
@@ -407,12 +409,20 @@ __device__ __noinline__ void bucket_merge_sort(R* s_r) {
       if (word_of(a[m]) <= word_of(b[d - 1 - m])) lo = m + 1; else hi = m;
     }
     int ia = lo, ib = d - lo;
+    R p = s_r[first], q = p;  // the runs' next records (one load per step)
+    if (ia < len) p = a[ia];
+    if (ib < len) q = b[ib];
 #pragma unroll
     for (int j = 0; j < I; ++j) {
-      const bool ta = ib >= len || (ia < len && word_of(a[ia]) <= word_of(b[ib]));
-      x[j] = ta ? a[ia] : b[ib];
+      const bool ta = ib >= len || (ia < len && word_of(p) <= word_of(q));
+      x[j] = ta ? p : q;
       ia += ta ? 1 : 0;
       ib += ta ? 0 : 1;
+      const R* next = ta ? a + ia : b + ib;
+      if ((ta ? ia : ib) < len) {
+        if (ta) p = *next;
+        else q = *next;
+      }
     }
     __syncthreads();
 #pragma unroll
@@ -421,13 +431,160 @@ __device__ __noinline__ void bucket_merge_sort(R* s_r) {
   __syncthreads();
 }
 
-// Sorts the k records of one sub-bucket by word (one thread); FOLD adds up its
+// Sub-buckets of more than kSubThread records, which a single thread would sort
+// for long (20 equal keys per sub-bucket: 2000 pairs 69 us, 27 like this): every
+// record of theirs counts the smaller words of its sub-bucket and goes to its
+// rank.  sub_of(word): the word's sub-bucket.
+template <int BT, int I, class R, class SubOf>
+__device__ __forceinline__ void rank_sub_buckets(R* s_r, const u32* s_cnt, const unsigned short* s_base, u32 cnt,
+                                              const SubOf sub_of) {
+  const int tid = threadIdx.x;
+  R x[I];
+  u32 to[(I + 1) / 2];  // 16 bits per item
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 p = j * BT + tid;
+    u32 at = p;
+    if (p < cnt) {
+      x[j] = s_r[p];
+      const u64 w = word_of(x[j]);
+      const u32 sub = sub_of(w), sh = 8u * (sub & 3u), c4 = s_cnt[sub >> 2], k = (c4 >> sh) & 0xFFu;
+      if (k > (u32)kSubThread) {
+        const u32 lo = s_base[sub >> 2] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
+        u32 rank = 0;
+        for (u32 q = 0; q < k; ++q) rank += word_of(s_r[lo + q]) < w ? 1u : 0u;
+        at = lo + rank;
+      }
+    }
+    to[j / 2] = j & 1 ? to[j / 2] | (at << 16) : at;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < I; ++j) {
+    const u32 p = j * BT + tid, at = (to[j / 2] >> (16 * (j & 1))) & 0xFFFFu;
+    if (p < cnt && at != p) s_r[at] = x[j];
+  }
+  __syncthreads();
+}
+
+// Sorts the sub-buckets that are too long for a thread, or the whole bucket when
+// it is crowded.  (A function of its own: these paths are rare, and their
+// registers would be taken from the others.)
+template <class G>
+__device__ __noinline__ void sort_long(ulonglong2* s_r, const u32* s_cnt, const unsigned short* s_base, u32 cnt,
+                                       int sshift, bool crowded) {
+  if (crowded) bucket_merge_sort<G::kBT, G::kItems>(s_r);
+  else rank_sub_buckets<G::kBT, G::kItems>(s_r, s_cnt, s_base, cnt, [=](u64 w) { return (u32)(w >> sshift); });
+}
+
+// The run of equal keys that starts at each head of row g (32 sorted positions,
+// one warp): adds the rest of the run to the head's sum, and sets anynz when
+// something in it is not zero.  heads: the rows' head masks (valid positions
+// only), rows of them, cnt positions.  A run that ends in its own row or the
+// next is added up in input order by the head's lane; a longer one, which only
+// the row's last head can have, by the whole warp, lane by lane over the rows
+// and then over the lanes (one key 20,000 times: 1470 us by one lane).
+template <class Val>
+__device__ __forceinline__ void fold_row(const u32* heads, u32 rows, u32 g, u32 cnt, bool head, double& sum,
+                                         bool& anynz, const Val& val) {
+  constexpr u32 FULL = 0xffffffffu;
+  const u32 lane = threadIdx.x & 31, p = g * 32 + lane;
+  bool far = false;
+  if (head) {
+    const u32 later = lane == 31 ? 0u : heads[g] >> (lane + 1);
+    u32 end = cnt;
+    if (later) {
+      end = p + __ffs(later);
+    } else if (g + 1 < rows) {
+      const u32 next = heads[g + 1];
+      far = next == 0u;
+      if (next) end = (g + 1) * 32 + __ffs(next) - 1;
+    }
+    if (!far) {
+      for (u32 q = p + 1; q < end; ++q) {
+        const double y = val(q);
+        sum += y;
+        anynz |= y != 0.0;
+      }
+    }
+  }
+  const u32 who = __ballot_sync(FULL, far);
+  if (who == 0u) return;
+  const u32 from = __ffs(who) - 1;
+  double part = -0.0;  // the additive identity that keeps the sign of a zero
+  bool nz = false;
+  auto add = [&](u32 q) {
+    const double y = val(q);
+    part += y;
+    nz |= y != 0.0;
+  };
+  if (lane > from && p < cnt) add(p);
+  for (u32 r0 = g + 1; r0 < rows; r0 += 32) {
+    const u32 mine = r0 + lane < rows ? heads[r0 + lane] : 0u;
+    const u32 some = __ballot_sync(FULL, mine != 0u);
+    const u32 whole = min(some ? __ffs(some) - 1u : 32u, rows - r0);  // rows without a head
+    u32 r = r0;
+    for (; r + 4 <= r0 + whole && (r + 4) * 32 <= cnt; r += 4) {
+      double y[4];
+#pragma unroll
+      for (u32 u = 0; u < 4; ++u) y[u] = val((r + u) * 32 + lane);
+#pragma unroll
+      for (u32 u = 0; u < 4; ++u) {
+        part += y[u];
+        nz |= y[u] != 0.0;
+      }
+    }
+    for (; r < r0 + whole; ++r)
+      if (r * 32 + lane < cnt) add(r * 32 + lane);
+    if (some) {
+      const u32 last = __shfl_sync(FULL, mine, whole);  // the run ends before this row's first head
+      if (lane < __ffs(last) - 1u) add((r0 + whole) * 32 + lane);
+      break;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
+  nz = __any_sync(FULL, nz);
+  if (lane == from) {
+    sum += part;
+    anynz |= nz;
+  }
+}
+
+// Folds the cnt sorted records of a whole bucket: every head's value becomes the
+// sum of its run, and s_kept the mask of the heads that are written.  s_head:
+// room for a mask per 32 positions; first: the bucket begins the sorted array.
+template <int BT>
+__device__ __noinline__ void fold_bucket(ulonglong2* s_r, u32* s_head, u32* s_kept, u32 cnt, int ib,
+                                         int skip_zero_heads, bool first) {
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rows = (cnt + 31) / 32;
+  for (u32 g = warp; g < rows; g += BT / 32) {
+    const u32 p = g * 32 + lane;
+    const u32 m =
+        __ballot_sync(0xffffffffu, p < cnt && (p == 0 || ((s_r[p > 0 ? p - 1 : 0].x ^ s_r[p].x) >> ib) != 0));
+    if (lane == 0) s_head[g] = m;
+  }
+  __syncthreads();
+  for (u32 g = warp; g < rows; g += BT / 32) {
+    const u32 p = g * 32 + lane;
+    const bool head = (s_head[g] >> lane & 1u) != 0u;
+    double sum = head ? __longlong_as_double((long long)s_r[p].y) : 0.0;
+    bool anynz = sum != 0.0;
+    fold_row(s_head, rows, g, cnt, head, sum, anynz,
+             [&](u32 q) { return __longlong_as_double((long long)s_r[q].y); });
+    if (head) s_r[p].y = (u64)__double_as_longlong(sum);  // (nobody else reads a head's value)
+    const u32 kept = __ballot_sync(0xffffffffu, head && (!skip_zero_heads || anynz || (first && p == 0)));
+    if (lane == 0) s_kept[g] = kept;
+  }
+}
+
+// Sorts the k records of one sub-bucket by word (one thread); fold adds up its
 // runs of equal keys in that (input) order into their first record and clears
 // the kept bits of the others and of the dropped ones.  `at`: the position of
 // r[0] in the bucket; first: it is the first of the whole sorted array.
 template <bool FOLD>
 __device__ __forceinline__ void fold_sub_bucket(ulonglong2* r, int k, int ib, int skip_zero_heads, bool first, u32 at,
-                                                u32* kept) {
+                                                u32* kept, bool fold) {
   for (int i = 1; i < k; ++i) {  // insertion sort
     const ulonglong2 x = r[i];
     int q = i;
@@ -438,7 +595,7 @@ __device__ __forceinline__ void fold_sub_bucket(ulonglong2* r, int k, int ib, in
     }
     if (q != i) r[q] = x;
   }
-  if (!FOLD) return;
+  if (!FOLD || !fold) return;
   for (int i = 0; i < k;) {
     const u64 low = r[i].x >> ib;
     double sum = __longlong_as_double((long long)r[i].y);
@@ -477,7 +634,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
   if (FOLD && tid == 0) s_misc[0] = atomicAdd(&c.misc[1], 1u);
 #pragma unroll
   for (int j = 0; j < G::kSubPer; ++j) s_cnt[j * BT + tid] = 0;
-  if (tid == 0) s_misc[1] = 0;
+  if (tid == 0) s_misc[1] = s_misc[4] = 0;
   __syncthreads();
   const u32 b = FOLD ? s_misc[0] : blockIdx.x;  // FOLD: in order of arrival, for the look-back
   const u32 start = c.start[b];
@@ -508,8 +665,10 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
     u32 most = 0;
 #pragma unroll
     for (int j = 0; j < P2; ++j) most = __vmaxu2(most, pos[j]);
+    most = max(most & 0xFFFFu, most >> 16);
+    if (most >= (u32)kSubThread) s_misc[4] = 1;  // some sub-bucket is too long for a thread
     // crowded (some slot at the limit): the counts may have run over, and are not used
-    if (max(most & 0xFFFFu, most >> 16) >= (u32)kSubMax) s_misc[1] = 1;
+    if (most >= (u32)kSubMax) s_misc[1] = 1;
   }
   __syncthreads();
   {  // records before every count word
@@ -546,7 +705,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
     *reinterpret_cast<uint4*>(&s_base[tid * 8]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   }
   __syncthreads();
-  const bool ranked = s_misc[1] == 0;
+  const bool ranked = s_misc[1] == 0, by_rows = s_misc[4] != 0;
 #pragma unroll
   for (int j = 0; j < I; ++j) {  // place every record in its sub-bucket (crowded: as they are, to be sorted)
     const u32 p = j * BT + tid;
@@ -563,11 +722,13 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
     s_r[q] = r[j];
   }
   __syncthreads();
+  if (by_rows) sort_long<G>(s_r, s_cnt, s_base, cnt, sshift, !ranked);
   if (ranked) {
-    // sort (and fold) the sub-buckets of more than one record, each by one
-    // thread: about one per thread, of two records.  Count words go to the
-    // threads in turn, so that each gets its share also when the key has
-    // fewer bits than there are sub-buckets.
+    // sort (and fold, unless the bucket is folded as a whole) the sub-buckets
+    // of two to kSubThread records, each by one thread: about one per thread, of
+    // two records.  Count words go to the threads in turn, so that each gets its
+    // share also when the key has fewer bits than there are sub-buckets.
+    const bool fold_here = FOLD && !by_rows;
     u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -584,7 +745,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
       if (k == 2) {  // nearly always
         const bool swap = e1.x < e0.x;
         const ulonglong2 f = swap ? e1 : e0, g = swap ? e0 : e1;
-        if (FOLD) {
+        if (fold_here) {
           const double x = __longlong_as_double((long long)f.y), y = __longlong_as_double((long long)g.y);
           const bool equal = ((f.x ^ g.x) >> ib) == 0;
           u32 drop = equal ? 2u : 0u;  // bit q: position lo + q is not written
@@ -604,31 +765,14 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
           s_r[lo] = f;
           s_r[lo + 1] = g;
         }
-      } else {
-        fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
+      } else if (k <= (u32)kSubThread) {
+        fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept, fold_here);
       }
     }
-  } else {
-    bucket_merge_sort<G::kBT, G::kItems>(s_r);
-    if (FOLD) {
-      for (u32 p = tid; p < cnt; p += BT) {
-        const u64 low = s_r[p].x >> ib;
-        bool kept = false;
-        if (p == 0 || (s_r[p - 1].x >> ib) != low) {  // the first of its run
-          double sum = __longlong_as_double((long long)s_r[p].y);
-          bool anynz = sum != 0.0;
-          u32 q = p + 1;
-          for (; q < cnt && (s_r[q].x >> ib) == low; ++q) {
-            const double y = __longlong_as_double((long long)s_r[q].y);
-            sum += y;
-            anynz |= y != 0.0;
-          }
-          if (q > p + 1) s_r[p].y = (u64)__double_as_longlong(sum);  // (nobody else reads a head's value)
-          kept = !skip_zero_heads || anynz || start + p == 0;
-        }
-        if (!kept) atomicAnd(&s_kept[p >> 5], ~(1u << (p & 31)));
-      }
-    }
+  }
+  if (FOLD && by_rows) {
+    __syncthreads();
+    fold_bucket<G::kBT>(s_r, s_pre, s_kept, cnt, ib, skip_zero_heads, start == 0);
   }
   __syncthreads();
   const u64 prefix = (u64)b << shift;
@@ -772,6 +916,93 @@ __device__ __forceinline__ u32 one_sum(u32 v, u32* s, u32* total) {
   return (warp == 0 ? 0u : before) + inc - v;
 }
 
+// As sort_long.  A crowded CTA sorts its words by digits of eight bits, from the
+// lowest up, without those in which no two words differ, stably: a warp takes
+// consecutive words, matches its digits and counts per warp and digit.  The counts
+// of the sub-buckets are free then.  (20,000 pairs of ten keys in a range of 2^30,
+// sorted: 48 us, 140 by a merge sort of all the CTA has room for; 2000 pairs of one
+// key 18 and 130.)
+__device__ __noinline__ void small_sort_long(u64* s_w, u32* s_cnt, unsigned short* s_base, u32 n, u32 cnt,
+                                             u64 first_key, int sshift, bool crowded) {
+  constexpr int BT = kOneThreads, W = BT / 32, I = kOneItems;
+  constexpr u32 FULL = 0xffffffffu;
+  if (!crowded) {
+    rank_sub_buckets<BT, I>(s_w, s_cnt, s_base, cnt, [=](u64 x) {
+      return min((u32)(((x >> kOneIb) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1));
+    });
+    return;
+  }
+  static_assert(W * 256 == kOneSubWords, "the counts of the sub-buckets hold one per warp and digit");
+  u32* s_sum = reinterpret_cast<u32*>(s_base);                  // 32 words
+  unsigned long long* s_diff = reinterpret_cast<unsigned long long*>(s_base) + 16;  // bits in which words differ
+  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const u32 items = (cnt + BT - 1) / BT, from = warp * items * 32;
+  u32* mine = s_cnt + warp * 256;
+  __syncthreads();
+  if (tid == 0) *s_diff = 0ull;
+  __syncthreads();
+  const u64 w0 = s_w[0];
+  u64 diff = 0;
+  for (u32 p = tid; p < cnt; p += BT) diff |= s_w[p] ^ w0;
+  const u32 lo = __reduce_or_sync(FULL, (u32)diff), hi = __reduce_or_sync(FULL, (u32)(diff >> 32));
+  if (lane == 0) atomicOr(s_diff, (unsigned long long)hi << 32 | lo);
+  __syncthreads();
+  diff = *s_diff;
+  if (cnt == n && (diff >> kOneIb) == 0ull) {  // one key throughout: the input order
+    for (u32 p = tid; p < cnt; p += BT) s_w[p] = (w0 >> kOneIb << kOneIb) | p;
+    __syncthreads();
+    return;
+  }
+  for (int shift = 0; shift < 64; shift += 8) {
+    if (((diff >> shift) & 0xFFull) == 0ull) continue;
+    u64 w[I];
+    u32 pos[I / 2];
+    for (u32 d = lane; d < 256; d += 32) mine[d] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      if (j >= (int)items) break;
+      const u32 p = from + j * 32 + lane;
+      const bool valid = p < cnt;
+      w[j] = valid ? s_w[p] : 0ull;
+      const u32 d = (u32)(w[j] >> shift) & 0xFFu;
+      u32 peers = __ballot_sync(FULL, valid);  // the lanes with the same digit
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const u32 m = __ballot_sync(FULL, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? m : ~m;
+      }
+      u32 at = 0;
+      if (valid) at = mine[d];
+      __syncwarp();
+      if (valid && lane == (u32)__ffs(peers) - 1u) mine[d] = at + __popc(peers);
+      __syncwarp();
+      at += __popc(peers & ((1u << lane) - 1u));
+      pos[j / 2] = j & 1 ? pos[j / 2] | (at << 16) : at;
+    }
+    __syncthreads();
+    u32 run = 0;
+    if (tid < 256)
+      for (int q = 0; q < W; ++q) {  // words of this digit in the warps before
+        const u32 c = s_cnt[q * 256 + tid];
+        s_cnt[q * 256 + tid] = run;
+        run += c;
+      }
+    u32 total;
+    const u32 start = one_sum(run, s_sum, &total);  // and those of the digits before
+    if (tid < 256)
+      for (int q = 0; q < W; ++q) s_cnt[q * 256 + tid] += start;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+      if (j >= (int)items) break;
+      if (from + j * 32 + lane < cnt)
+        s_w[mine[(u32)(w[j] >> shift) & 0xFFu] + ((pos[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] = w[j];
+    }
+    __syncthreads();
+  }
+}
+
 template <bool FOLD>
 __global__ void __launch_bounds__(kOneThreads, 1)
     small_sort_kernel(const PairSource src, u32 n, int key_bits, u64 width, int sshift, u32 C, int skip_zero_heads,
@@ -784,7 +1015,8 @@ __global__ void __launch_bounds__(kOneThreads, 1)
   u32* s_head = reinterpret_cast<u32*>(s_base + kOneSubWords);   // per 32 positions: first of their runs
   u32* s_kept = s_head + kOneGroups;
   u32* s_pre = s_kept + kOneGroups;
-  u32* s_misc = s_pre + kOneGroups;  // [0, 32) sums, [40] crowded, [41] kept here, [42] before, [48, 56) CTA totals
+  u32* s_misc = s_pre + kOneGroups;  // [0, 32) sums, [40] crowded, [41] kept here, [42] before, [43] long
+                                     // sub-buckets, [48, 56) CTA totals
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const u32 le = lane == 31 ? ~0u : (2u << lane) - 1u;
   const u32 rank = C > 1 ? cluster_rank() : 0u;
@@ -793,7 +1025,7 @@ __global__ void __launch_bounds__(kOneThreads, 1)
   const u64 first_key = width * rank, end_key = rank + 1 == C ? ~0ull : first_key + width;
 #pragma unroll
   for (int j = 0; j < 8; ++j) s_cnt[j * BT + tid] = 0;
-  if (tid >= 40 && tid < 43) s_misc[tid] = 0;
+  if (tid >= 40 && tid < 44) s_misc[tid] = 0;
   __syncthreads();
   // ---- this CTA's words, in any order; how many keys lie before them ----------
   u64 high = 0;
@@ -831,14 +1063,21 @@ __global__ void __launch_bounds__(kOneThreads, 1)
     const u32 p = j * BT + tid;
     w[j] = p < cnt ? s_w[p] : ~0ull;
     u32 slot = 0;
-    if (p < cnt) {
-      const u32 sub = min((u32)(((w[j] >> ib) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1));
-      const u32 sh = 8u * (sub & 3u);
+    const u32 sub =
+        p < cnt ? min((u32)(((w[j] >> ib) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1)) : ~0u;
+    const u32 sh = 8u * (sub & 3u);
+    // (keys that gather in one CTA may gather in one sub-bucket: one atomic per warp)
+    const u32 sub0 = __shfl_sync(0xffffffffu, sub, 0);
+    if (__all_sync(0xffffffffu, items > 5 && sub != ~0u && sub == sub0)) {
+      if (lane == 0) slot = (atomicAdd(&s_cnt[sub >> 2], 32u << sh) >> sh) & 0xFFu;
+      slot = __shfl_sync(0xffffffffu, slot, 0) + lane;
+    } else if (p < cnt) {
       slot = (atomicAdd(&s_cnt[sub >> 2], 1u << sh) >> sh) & 0xFFu;
     }
     pos[j / 2] = j & 1 ? pos[j / 2] | (slot << 16) : slot;
     most = max(most, slot);
   }
+  if (most >= (u32)kSubThread) s_misc[43] = 1;
   if (most >= (u32)kSubMax) s_misc[40] = 1;  // crowded: the counts may have run over, and are not used
   __syncthreads();
   {  // records before every count word
@@ -864,7 +1103,8 @@ __global__ void __launch_bounds__(kOneThreads, 1)
     *reinterpret_cast<uint4*>(&s_base[tid * 8]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   }
   __syncthreads();
-  if (s_misc[40] == 0) {
+  const bool ranked = s_misc[40] == 0;
+  if (ranked) {
 #pragma unroll
     for (int j = 0; j < I; ++j) {
       if (j >= items) break;
@@ -876,6 +1116,9 @@ __global__ void __launch_bounds__(kOneThreads, 1)
       }
     }
     __syncthreads();
+  }
+  if (s_misc[43]) small_sort_long(s_w, s_cnt, s_base, n, cnt, first_key, sshift, !ranked);
+  if (ranked) {
     u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -888,6 +1131,7 @@ __global__ void __launch_bounds__(kOneThreads, 1)
       const u32 c4 = s_cnt[(i >> 2) * BT + tid];
       u64* r = s_w + s_base[(i >> 2) * BT + tid] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
       const int k = (int)((c4 >> sh) & 0xFFu);
+      if (k > kSubThread) continue;
       for (int x = 1; x < k; ++x) {
         const u64 a = r[x];
         int q = x;
@@ -899,10 +1143,6 @@ __global__ void __launch_bounds__(kOneThreads, 1)
         if (q != x) r[q] = a;
       }
     }
-  } else {
-    for (u32 p = cnt + tid; p < (u32)kOneCap; p += BT) s_w[p] = ~0ull;
-    __syncthreads();
-    bucket_merge_sort<BT, I>(s_w);
   }
   __syncthreads();
   // ---- the words by position, and their values ----------------------------------
@@ -965,21 +1205,15 @@ __global__ void __launch_bounds__(kOneThreads, 1)
   }
   __syncthreads();
   const u32 groups = (u32)items * (BT / 32);
-#pragma unroll
-  for (int j = 0; j < I; ++j) {
-    if (j >= items) break;
+#pragma unroll 1
+  for (int j = 0; j < items; ++j) {  // (a head's value becomes its run's sum: nobody else reads it)
     const u32 p = j * BT + tid, g = j * (BT / 32) + warp;
-    bool kept = false;
-    if (p < cnt && (s_head[g] >> lane & 1u)) {
-      bool anynz = v[j] != 0.0;
-      for (u32 q = p + 1; q < cnt && !(s_head[q >> 5] >> (q & 31) & 1u); ++q) {
-        const double y = s_v[q];
-        v[j] += y;
-        anynz |= y != 0.0;
-      }
-      kept = !skip_zero_heads || anynz || start + p == 0;
-    }
-    const u32 m = __ballot_sync(0xffffffffu, kept);
+    const bool head = p < cnt && (s_head[g] >> lane & 1u);
+    double sum = head ? s_v[p] : 0.0;
+    bool anynz = sum != 0.0;
+    fold_row(s_head, groups, g, cnt, head, sum, anynz, [&](u32 q) { return s_v[q]; });
+    if (head) s_v[p] = sum;
+    const u32 m = __ballot_sync(0xffffffffu, head && (!skip_zero_heads || anynz || start + p == 0));
     if (lane == 0) s_kept[g] = m;
   }
   __syncthreads();
@@ -1008,7 +1242,7 @@ __global__ void __launch_bounds__(kOneThreads, 1)
     if (m >> lane & 1u) {
       const u32 o = off + s_pre[g] + __popc(m & (le >> 1));
       out_k[o] = w[j] >> kshift;
-      out_v[o] = v[j];
+      out_v[o] = s_v[j * BT + tid];
     }
   }
 }
@@ -1096,6 +1330,11 @@ MsdPlan make_msd_plan(size_t n, u64 max_key) {
     return p;
   }
   if (n < kMinPairs) return p;
+  // More pairs per key than a thread's or a warp's share of a sub-bucket: the
+  // digit passes and their collect are ahead from 32 pairs per key on (2^20 pairs
+  // of 2^15 keys: fold 133 us by buckets, 80 by digits; 2^26 of 2^21: 4.2 and 2.9
+  // ms), the buckets up to 16 (79 and 81 us; 2.7 and 2.9 ms).
+  if ((double)n > kMaxPerKey * (double)max_key) return p;
   const char* force = getenv("LNT_BUCKET_SMALL");
   int bestT = 99;
   for (int large = 0; large < 2; ++large) {
