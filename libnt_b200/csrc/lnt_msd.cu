@@ -14,10 +14,10 @@
 //      each first-pass segment for itself.
 //   3. bucket_sort_kernel: one CTA per bucket sorts its words (low key bits,
 //      then index: the stable order) in shared memory: the words are counted
-//      into sub-buckets, placed, and ranked within their sub-bucket (a merge
-//      sort instead when a sub-bucket is crowded).  FOLD adds up runs of
-//      equal keys in input order and writes at offsets from a look-back over
-//      the buckets; a plain sort knows its offsets already.
+//      into sub-buckets, placed, and ranked within their sub-bucket (or sorted
+//      by digits when a sub-bucket is crowded).  FOLD adds up runs of equal
+//      keys, in input order unless they are long, and writes at offsets from a
+//      look-back over the buckets; a plain sort knows its offsets already.
 //
 // DRAM traffic: 8 B (histogram) + 32 B per pass + 16 B + 16 B per pair.
 // Measured on 2^27 pairs with 36-bit keys (B200): histogram 0.36 ms, partition
@@ -37,9 +37,10 @@ namespace {
 
 constexpr int kHistThreads = 1024;
 constexpr int kMaxT = 15;
-// Smallest sort taken.  Down to 2048 pairs the bucketed path with the skipped
-// fallback behind it takes 18-21 us against 33-57 us for the digit passes (20
-// to 50 key bits); below, the histogram and one CTA are all there is to gain.
+// Smallest sort taken, where one cluster does not do it all (more than 49 key
+// bits).  Down to 2048 pairs the bucketed path with the skipped fallback behind it
+// takes 18-21 us against 33-57 us for the digit passes; below, the histogram and
+// one CTA are all there is to gain.
 constexpr size_t kMinPairs = 2048;
 constexpr double kMaxPerKey = 24.0;
 constexpr int kMaxDigits = 256;
@@ -83,7 +84,7 @@ struct MsdCtrl {
   u32* cur1;      // first pass cursors (up to 256)
   u32* cur2;      // second pass cursors (2^T)
   u32* segtile;   // second pass: first tile of every segment (up to 257)
-  u32* misc;      // [0] histogram CTAs done, [1] bucket counter, [2] a key has bits above the sorted ones
+  u32* misc;      // [0] histogram CTAs done, [1] bucket counter, [2] the gate closes, whatever the counts say
   unsigned long long* status;  // 2^T look-back words (FOLD)
   u32* gate;      // 0: every bucket fits a CTA (and no key loses bits), 1: take the LSD path
 };
@@ -125,6 +126,12 @@ __global__ void __launch_bounds__(kHistThreads, 1) msd_hist_kernel(const PairSou
   const u32 bmask = (u32)(nb - 1);
   u64 any = 0;
   constexpr int U = 8;
+  // Clustered keys: once a CTA has counted more of one bucket than fits, the rest
+  // need not be read.  Looked for after 2, 4, 8 .. rounds, while at least as many
+  // are left.
+  u32 round = 0, next_look = 2;
+  bool closed = false;
+  const u32 rounds = (u32)(n / ((u64)gridDim.x * (kHistThreads * U)));
   for (u64 base = (u64)blockIdx.x * (kHistThreads * U); base < n; base += (u64)gridDim.x * (kHistThreads * U)) {
     const u32 end = (u32)min((u64)n, base + kHistThreads * U);
     u64 k[U];
@@ -135,11 +142,20 @@ __global__ void __launch_bounds__(kHistThreads, 1) msd_hist_kernel(const PairSou
         atomicAdd(&sh[(u32)(k[u] >> shift) & bmask], 1u);
         any |= k[u];
       }
+    if (++round == next_look && 2 * round <= rounds) {
+      next_look *= 2;
+      __syncthreads();
+      u32 most = 0;
+      for (int i = tid; i < nb; i += kHistThreads) most = max(most, sh[i]);
+      closed = __syncthreads_or(most > cap) != 0;
+      if (closed) break;
+    }
   }
+  if (closed && tid == 0) atomicOr(&c.misc[2], 1u);
   // bits above the sorted ones (a key >= max_key): the records would lose them
   if (key_bits < 64 && (any >> key_bits) != 0) atomicOr(&c.misc[2], 1u);
   __syncthreads();
-  for (int b = tid; b < nb; b += kHistThreads) {
+  for (int b = tid; b < nb && !closed; b += kHistThreads) {
     const u32 v = sh[b];
     if (v) atomicAdd(&c.counts[b], v);
   }
@@ -375,60 +391,87 @@ __global__ void __launch_bounds__(P::kThreads, P::kMinBlocks)
 __device__ __forceinline__ u64 word_of(const ulonglong2& r) { return r.x; }
 __device__ __forceinline__ u64 word_of(u64 w) { return w; }
 
-// Sorts the records s_r[0, cap) by word in place (cap = BT * ITEMS; the unused
-// ones, behind the others, hold ~0): ITEMS records per thread by odd-even
-// transposition, then merge rounds over doubling groups of threads, each thread
-// finding its output range by a merge-path search.  Stable throughout: a record
-// whose word is ~0 too stays in front of the unused ones.
+// Sorts the cnt records s_r by word, by digits of eight bits from the lowest up,
+// without those in which no two words differ.  Stably: a warp takes consecutive
+// records, matches their digits and counts per warp and digit.  s_cnt: a word per
+// warp and digit; s_tmp: 36 words.  (2^21 pairs, 95% of them of 2^12 keys: 152 us
+// in all, 209 with a merge sort, whose rounds search in shared memory.)
 template <int BT, int I, class R>
-__device__ __forceinline__ void bucket_merge_sort(R* s_r) {
-  const int tid = threadIdx.x;
-  R x[I];
-#pragma unroll
-  for (int j = 0; j < I; ++j) x[j] = s_r[tid * I + j];
-#pragma unroll
-  for (int r = 0; r < I; ++r)
-#pragma unroll
-    for (int j = r & 1; j + 1 < I; j += 2) {
-      const R p = x[j], q = x[j + 1];
-      const bool keep = word_of(p) <= word_of(q);
-      x[j] = keep ? p : q;
-      x[j + 1] = keep ? q : p;
-    }
-#pragma unroll
-  for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
-  for (int g = 1; g < BT; g <<= 1) {  // merge runs of g * I records
-    __syncthreads();
-    const int first = (tid / (2 * g)) * 2 * g * I;
-    const R* a = s_r + first;
-    const R* b = a + g * I;
-    const int len = g * I, d = (tid % (2 * g)) * I;
-    int lo = d > len ? d - len : 0, hi = d < len ? d : len;
-    while (lo < hi) {
-      const int m = (lo + hi) >> 1;
-      if (word_of(a[m]) <= word_of(b[d - 1 - m])) lo = m + 1; else hi = m;
-    }
-    int ia = lo, ib = d - lo;
-    R p = s_r[first], q = p;  // the runs' next records (one load per step)
-    if (ia < len) p = a[ia];
-    if (ib < len) q = b[ib];
+__device__ __forceinline__ void sort_by_digits(R* s_r, u32* s_cnt, u32* s_tmp, u32 cnt) {
+  constexpr int W = BT / 32;
+  constexpr u32 FULL = 0xffffffffu;
+  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const u32 items = (cnt + BT - 1) / BT, from = warp * items * 32;
+  u32* mine = s_cnt + warp * 256;
+  unsigned long long* s_diff = reinterpret_cast<unsigned long long*>(s_tmp + 32);
+  __syncthreads();
+  if (tid == 0) *s_diff = 0ull;
+  __syncthreads();
+  const u64 w0 = word_of(s_r[0]);
+  u64 diff = 0;
+  for (u32 p = tid; p < cnt; p += BT) diff |= word_of(s_r[p]) ^ w0;
+  const u32 lo = __reduce_or_sync(FULL, (u32)diff), hi = __reduce_or_sync(FULL, (u32)(diff >> 32));
+  if (lane == 0) atomicOr(s_diff, (unsigned long long)hi << 32 | lo);
+  __syncthreads();
+  diff = *s_diff;
+  for (int shift = 0; shift < 64; shift += 8) {
+    if (((diff >> shift) & 0xFFull) == 0ull) continue;
+    R x[I];
+    u32 pos[(I + 1) / 2];  // 16 bits per item
+    for (u32 d = lane; d < 256; d += 32) mine[d] = 0u;
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < I; ++j) {
-      const bool ta = ib >= len || (ia < len && word_of(p) <= word_of(q));
-      x[j] = ta ? p : q;
-      ia += ta ? 1 : 0;
-      ib += ta ? 0 : 1;
-      const R* next = ta ? a + ia : b + ib;
-      if ((ta ? ia : ib) < len) {
-        if (ta) p = *next;
-        else q = *next;
+      if (j >= (int)items) break;
+      const u32 p = from + j * 32 + lane;
+      const bool valid = p < cnt;
+      if (valid) x[j] = s_r[p];
+      const u32 d = valid ? (u32)(word_of(x[j]) >> shift) & 0xFFu : 0u;
+      u32 peers = __ballot_sync(FULL, valid);  // the lanes with the same digit
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const u32 m = __ballot_sync(FULL, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? m : ~m;
       }
+      u32 at = 0;
+      if (valid) at = mine[d];
+      __syncwarp();
+      if (valid && lane == (u32)__ffs(peers) - 1u) mine[d] = at + __popc(peers);
+      __syncwarp();
+      at += __popc(peers & ((1u << lane) - 1u));
+      pos[j / 2] = j & 1 ? pos[j / 2] | (at << 16) : at;
+    }
+    __syncthreads();
+    u32 run = 0, inc = 0;
+    if (tid < 256) {
+      for (int q = 0; q < W; ++q) {  // records of this digit in the warps before
+        const u32 c = s_cnt[q * 256 + tid];
+        s_cnt[q * 256 + tid] = run;
+        run += c;
+      }
+      inc = run;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (u32)o) inc += t;
+      }
+      if (lane == 31) s_tmp[warp] = inc;
+    }
+    __syncthreads();
+    if (tid < 256) {  // and those of the digits before
+      u32 start = inc - run;
+      for (u32 q = 0; q < warp; ++q) start += s_tmp[q];
+      for (int q = 0; q < W; ++q) s_cnt[q * 256 + tid] += start;
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < I; ++j) s_r[tid * I + j] = x[j];
+    for (int j = 0; j < I; ++j) {
+      if (j >= (int)items) break;
+      if (from + j * 32 + lane < cnt)
+        s_r[mine[(u32)(word_of(x[j]) >> shift) & 0xFFu] + ((pos[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] = x[j];
+    }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // Sub-buckets of more than kSubThread records, which a single thread would sort
@@ -471,9 +514,10 @@ __device__ __forceinline__ void rank_sub_buckets(R* s_r, const u32* s_cnt, const
 // it is crowded.  (A function of its own: these paths are rare, and their
 // registers would be taken from the others.)
 template <class G>
-__device__ __noinline__ void sort_long(ulonglong2* s_r, const u32* s_cnt, const unsigned short* s_base, u32 cnt,
-                                       int sshift, bool crowded) {
-  if (crowded) bucket_merge_sort<G::kBT, G::kItems>(s_r);
+__device__ __noinline__ void sort_long(ulonglong2* s_r, u32* s_cnt, unsigned short* s_base, u32 cnt, int sshift,
+                                       bool crowded) {
+  static_assert(G::kWarps * 256 <= G::kSubWords, "the counts of the sub-buckets hold one per warp and digit");
+  if (crowded) sort_by_digits<G::kBT, G::kItems>(s_r, s_cnt, reinterpret_cast<u32*>(s_base), cnt);
   else rank_sub_buckets<G::kBT, G::kItems>(s_r, s_cnt, s_base, cnt, [=](u64 w) { return (u32)(w >> sshift); });
 }
 
@@ -859,13 +903,13 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
 // of its own range (the c-th part of [0, max_key)), so that it knows without
 // asking how many lie before; a single CTA could hold all pairs, whatever their
 // distribution.  It sorts its words (key << 15 | index) in shared memory as the
-// bucket kernel does (a merge sort when a sub-bucket is crowded), fetches their
-// values, and writes once the whole cluster has read its input (the output may
-// be the input).  FOLD exchanges the CTAs' output counts through distributed
+// bucket kernel does, fetches their values, and writes once the whole cluster has
+// read its input (the output may be the input).  FOLD exchanges the CTAs' output counts through distributed
 // shared memory.  Bound by latency (B200, replayed in a graph,
-// 20 to 41 key bits): 2048 pairs 8-10 us, 10,000 14.5, 20,000 18.6, against 20.6
-// to 22.7 us for histogram, partition, buckets and the skipped path behind them;
-// one CTA alone takes 12.5, 20.6 and 33 us.
+// 20 to 41 key bits, evenly spread): 2048 pairs 8-10 us, 10,000 14.5, 20,000 18.6,
+// against 20.6 to 22.7 us for histogram, partition, buckets and the skipped path
+// behind them; one CTA alone takes 12.5, 20.6 and 33 us.  (Enqueued one by one,
+// sort_reduce of 20,000 pairs: distinct keys 26 us, 100 keys 51, one key 56.)
 constexpr int kOneThreads = 1024, kOneItems = 20, kOneCap = kOneThreads * kOneItems;
 constexpr int kOneIb = 15;       // index bits (kOneCap < 2^15)
 constexpr int kOneSubBits = 15;  // 2^15 sub-buckets: 8 count words per thread
@@ -916,90 +960,26 @@ __device__ __forceinline__ u32 one_sum(u32 v, u32* s, u32* total) {
   return (warp == 0 ? 0u : before) + inc - v;
 }
 
-// As sort_long.  A crowded CTA sorts its words by digits of eight bits, from the
-// lowest up, without those in which no two words differ, stably: a warp takes
-// consecutive words, matches its digits and counts per warp and digit.  The counts
-// of the sub-buckets are free then.  (20,000 pairs of ten keys in a range of 2^30,
-// sorted: 48 us, 140 by a merge sort of all the CTA has room for; 2000 pairs of one
-// key 18 and 130.)
+// As sort_long; a crowded CTA with one key throughout, and all of its pairs, has
+// them in input order.
 __device__ __noinline__ void small_sort_long(u64* s_w, u32* s_cnt, unsigned short* s_base, u32 n, u32 cnt,
                                              u64 first_key, int sshift, bool crowded) {
-  constexpr int BT = kOneThreads, W = BT / 32, I = kOneItems;
-  constexpr u32 FULL = 0xffffffffu;
+  constexpr int BT = kOneThreads;
+  static_assert(BT / 32 * 256 <= kOneSubWords, "the counts of the sub-buckets hold one per warp and digit");
   if (!crowded) {
-    rank_sub_buckets<BT, I>(s_w, s_cnt, s_base, cnt, [=](u64 x) {
+    rank_sub_buckets<BT, kOneItems>(s_w, s_cnt, s_base, cnt, [=](u64 x) {
       return min((u32)(((x >> kOneIb) - first_key) >> sshift), (u32)(4 * kOneSubWords - 1));
     });
     return;
   }
-  static_assert(W * 256 == kOneSubWords, "the counts of the sub-buckets hold one per warp and digit");
-  u32* s_sum = reinterpret_cast<u32*>(s_base);                  // 32 words
-  unsigned long long* s_diff = reinterpret_cast<unsigned long long*>(s_base) + 16;  // bits in which words differ
-  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const u32 items = (cnt + BT - 1) / BT, from = warp * items * 32;
-  u32* mine = s_cnt + warp * 256;
-  __syncthreads();
-  if (tid == 0) *s_diff = 0ull;
-  __syncthreads();
-  const u64 w0 = s_w[0];
-  u64 diff = 0;
-  for (u32 p = tid; p < cnt; p += BT) diff |= s_w[p] ^ w0;
-  const u32 lo = __reduce_or_sync(FULL, (u32)diff), hi = __reduce_or_sync(FULL, (u32)(diff >> 32));
-  if (lane == 0) atomicOr(s_diff, (unsigned long long)hi << 32 | lo);
-  __syncthreads();
-  diff = *s_diff;
-  if (cnt == n && (diff >> kOneIb) == 0ull) {  // one key throughout: the input order
-    for (u32 p = tid; p < cnt; p += BT) s_w[p] = (w0 >> kOneIb << kOneIb) | p;
+  const u64 key = s_w[0] >> kOneIb;
+  bool other = false;
+  for (u32 p = threadIdx.x; p < cnt; p += BT) other = other || s_w[p] >> kOneIb != key;
+  if (__syncthreads_or(other) == 0 && cnt == n) {
+    for (u32 p = threadIdx.x; p < cnt; p += BT) s_w[p] = key << kOneIb | p;
     __syncthreads();
-    return;
-  }
-  for (int shift = 0; shift < 64; shift += 8) {
-    if (((diff >> shift) & 0xFFull) == 0ull) continue;
-    u64 w[I];
-    u32 pos[I / 2];
-    for (u32 d = lane; d < 256; d += 32) mine[d] = 0u;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < I; ++j) {
-      if (j >= (int)items) break;
-      const u32 p = from + j * 32 + lane;
-      const bool valid = p < cnt;
-      w[j] = valid ? s_w[p] : 0ull;
-      const u32 d = (u32)(w[j] >> shift) & 0xFFu;
-      u32 peers = __ballot_sync(FULL, valid);  // the lanes with the same digit
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const u32 m = __ballot_sync(FULL, (d >> b) & 1u);
-        peers &= (d >> b) & 1u ? m : ~m;
-      }
-      u32 at = 0;
-      if (valid) at = mine[d];
-      __syncwarp();
-      if (valid && lane == (u32)__ffs(peers) - 1u) mine[d] = at + __popc(peers);
-      __syncwarp();
-      at += __popc(peers & ((1u << lane) - 1u));
-      pos[j / 2] = j & 1 ? pos[j / 2] | (at << 16) : at;
-    }
-    __syncthreads();
-    u32 run = 0;
-    if (tid < 256)
-      for (int q = 0; q < W; ++q) {  // words of this digit in the warps before
-        const u32 c = s_cnt[q * 256 + tid];
-        s_cnt[q * 256 + tid] = run;
-        run += c;
-      }
-    u32 total;
-    const u32 start = one_sum(run, s_sum, &total);  // and those of the digits before
-    if (tid < 256)
-      for (int q = 0; q < W; ++q) s_cnt[q * 256 + tid] += start;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < I; ++j) {
-      if (j >= (int)items) break;
-      if (from + j * 32 + lane < cnt)
-        s_w[mine[(u32)(w[j] >> shift) & 0xFFu] + ((pos[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] = w[j];
-    }
-    __syncthreads();
+  } else {
+    sort_by_digits<BT, kOneItems>(s_w, s_cnt, reinterpret_cast<u32*>(s_base), cnt);
   }
 }
 

@@ -44,17 +44,17 @@ __device__ __forceinline__ double load_val(const PairSource& s, size_t i) {
 // ---------------------------------------------------------------------------
 // Histogram of every pass's digits in one read of the keys.
 // ---------------------------------------------------------------------------
-// Block `block` of `nblocks` (kThreads threads); sh_hist: passes * RADIX words.
-template <int BITS>
+// Block `block` of `nblocks` (THREADS threads); sh_hist: passes * RADIX words.
+template <int BITS, int THREADS>
 __device__ __forceinline__ void hist_block(const PairSource& src, u32 n, int passes, int key_bits, u32* ghist,
                                            u32* bstart, u32* done, u32* sh_hist, u32 block, u32 nblocks) {
   constexpr int RADIX = 1 << BITS;
   __shared__ bool s_last;
-  for (int i = threadIdx.x; i < passes * RADIX; i += kThreads) sh_hist[i] = 0;
+  for (int i = threadIdx.x; i < passes * RADIX; i += THREADS) sh_hist[i] = 0;
   __syncthreads();
-  const u32 stride = nblocks * kThreads;
+  const u32 stride = nblocks * THREADS;
   constexpr int U = 8;  // independent loads in flight per thread
-  u32 i = block * kThreads + threadIdx.x;
+  u32 i = block * THREADS + threadIdx.x;
   for (; i + (U - 1) * stride < n; i += U * stride) {
     u64 k[U];
 #pragma unroll
@@ -77,7 +77,7 @@ __device__ __forceinline__ void hist_block(const PairSource& src, u32 n, int pas
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < passes * RADIX; i += kThreads) {
+  for (int i = threadIdx.x; i < passes * RADIX; i += THREADS) {
     u32 c = sh_hist[i];
     if (c) atomicAdd(&ghist[i], c);
   }
@@ -88,8 +88,8 @@ __device__ __forceinline__ void hist_block(const PairSource& src, u32 n, int pas
   if (!s_last) return;
   __threadfence();
   // Last block: exclusive scan of each pass's histogram into bin starts.
-  __shared__ u32 s_warp[kWarps];
-  constexpr int DPT = (RADIX + kThreads - 1) / kThreads;
+  __shared__ u32 s_warp[THREADS / 32];
+  constexpr int DPT = (RADIX + THREADS - 1) / THREADS;
   for (int p = 0; p < passes; ++p) {
     u32 c[DPT];
     u32 local = 0;
@@ -125,7 +125,7 @@ template <int BITS>
 __global__ void __launch_bounds__(kThreads) hist_kernel(const PairSource src, u32 n, int passes, int key_bits,
                                                         u32* ghist, u32* bstart, u32* done) {
   extern __shared__ u32 sh_hist[];
-  hist_block<BITS>(src, n, passes, key_bits, ghist, bstart, done, sh_hist, blockIdx.x, gridDim.x);
+  hist_block<BITS, kThreads>(src, n, passes, key_bits, ghist, bstart, done, sh_hist, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -170,11 +170,21 @@ __device__ __forceinline__ u32 match_digit(u32 d) {
 }
 
 // One tile of a digit pass.  Tiles are handed out in order, so every
-// predecessor a look-back waits on belongs to a running CTA.
-template <int BITS, int THREADS, int ITEMS, int W, bool FIRST>
+// predecessor a look-back waits on belongs to a running CTA.  QUEUE: part of
+// lsd_queue_kernel.
+struct QueueState {
+  u32 task;
+  u32 step;   // the step this CTA is in
+  u32 count;  // its finished tasks of that step, not yet reported
+  u32 taken;  // `task` is the next one already
+  u32 expired;  // a wait ran out
+};
+
+template <int BITS, int THREADS, int ITEMS, int W, bool FIRST, bool QUEUE = false>
 __device__ __forceinline__ void onesweep_tile(const PairSource& src, u64* out_k, double* out_v, u32 n, u32 shift,
                                               u32 mask, const u32* bstart, u32* status, u32 tile,
-                                              unsigned char* smem) {
+                                              unsigned char* smem, QueueState* q = nullptr,
+                                              u32* gate = nullptr) {
   using S = OnesweepShape<BITS, THREADS, ITEMS>;
   constexpr int RADIX = S::RADIX;
   constexpr int WARPS = S::WARPS;
@@ -353,6 +363,10 @@ __device__ __forceinline__ void onesweep_tile(const PairSource& src, u64* out_k,
       s_glob[d] = excl[j] - tstart[j];
     }
   }
+  if (QUEUE && tid == 0) {
+    q->task = atomicAdd(&gate[1], 1u);  // (arrives while the tile is written)
+    q->taken = 1u;
+  }
   __syncthreads();
 
   // ---- scatter keys (digit runs -> contiguous destination ranges) ---------
@@ -404,15 +418,21 @@ __global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>:
 // The whole sort in one launch, for the path behind a gate: it is nearly
 // always skipped, and a skipped launch costs 1.6 us in the stream (seven to
 // ten of them when every step was a kernel of its own).  CTAs take the tasks
-// (zero the control block, histogram, the tiles of every pass) in order from a
-// queue; a task waits until the step before is complete, whose tasks all
-// belong to running CTAs.  gate[1]: queue, gate[2 + step]: tasks done; zeroed
-// by whoever writes the gate.  A CTA whose wait ran out waits no more (there
-// may be hundreds of tasks left) and goes on: the error is latched, and every
-// write stays inside the output whatever the histogram holds (see the clamp in
-// onesweep_tile).
-constexpr int kQBits = 8, kQItems = 16, kQWindow = 16;
-using QueueShape = OnesweepShape<kQBits, kThreads, kQItems>;
+// (zero the counts, histogram, the tiles of every pass) in order from a queue; at
+// its first task of a step a CTA waits until the step before is complete, whose
+// tasks all belong to running CTAs.  gate[1]: queue, gate[2 + step]: tasks done;
+// zeroed by whoever writes the gate.  A CTA reports its tasks when it leaves a
+// step, all at once (a report per tile, whose fence waits for the tile's scattered
+// stores: 2^25 pairs of 36 bits 2.05 ms in all, 1.97 like this), and a pass's
+// look-back words are zeroed by the step before instead of all of them first.  A
+// CTA whose wait ran out waits no more (there may be hundreds of tasks left) and
+// goes on: the error is latched, and every write stays inside the output whatever
+// the histogram holds (see the clamp in onesweep_tile).
+// Sorts behind a closed gate (95% of the keys in 1/4096 of the range), all told,
+// against the digit passes alone: 2^17 pairs of 36 bits 92 and 70 us, 2^21 212 and
+// 177, 2^25 1.96 and 1.82 ms.  The difference is the bucket histogram, the three
+// skipped launches and the waits between the steps; evenly spread keys gain 41, 87
+// us and 0.83 ms against the same figures.
 
 // True when the wait ran out.
 __device__ __forceinline__ bool queue_wait(const u32* done, u32 want) {
@@ -428,68 +448,84 @@ __device__ __forceinline__ bool queue_wait(const u32* done, u32 want) {
   }
   return __syncthreads_or(expired) != 0;
 }
-__device__ __forceinline__ void queue_done(u32* done) {
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(done, 1u);
-}
 
-__global__ void __launch_bounds__(kThreads, QueueShape::MINB)
+template <int BITS, int THREADS, int ITEMS, int W>
+__global__ void __launch_bounds__(THREADS, (OnesweepShape<BITS, THREADS, ITEMS>::MINB))
     lsd_queue_kernel(const PairSource src, const SortPlan plan, u64* buf0_k, double* buf0_v, u64* buf1_k,
                      double* buf1_v, unsigned char* ctrl, u32* gate) {
   if (gated_off(src.gate, src.gate_run)) return;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ u32 s_task;
-  constexpr int RADIX = 1 << kQBits;
-  constexpr size_t kZero = 1u << 16;  // bytes zeroed per task
-  const u32 nz = (u32)((plan.ctrl_bytes + kZero - 1) / kZero);
-  const u32 nh = min((plan.n + kThreads * 16 - 1) / (kThreads * 16), gridDim.x);
+  __shared__ QueueState s_q;
+  constexpr int RADIX = 1 << BITS;
+  const u32 nh = min((plan.n + THREADS * 16 - 1) / (THREADS * 16), gridDim.x);
   u32* ghist = reinterpret_cast<u32*>(ctrl + plan.off_ghist);
   u32* bstart = reinterpret_cast<u32*>(ctrl + plan.off_bstart);
   u32* status = reinterpret_cast<u32*>(ctrl + plan.off_status);
   u32* counters = reinterpret_cast<u32*>(ctrl + plan.off_counters);
-  bool expired = false;  // (the same in all threads)
+  if (threadIdx.x == 0) s_q = {0u, 0u, 0u, 0u, 0u};
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_task = atomicAdd(&gate[1], 1u);
+    if (threadIdx.x == 0 && !s_q.taken) s_q.task = atomicAdd(&gate[1], 1u);
     __syncthreads();
-    u32 t = s_task;
-    if (t < nz) {
-      uint4* z = reinterpret_cast<uint4*>(ctrl + (size_t)t * kZero);
-      const size_t words = min(kZero, plan.ctrl_bytes - (size_t)t * kZero) / 16;
-      for (size_t i = threadIdx.x; i < words; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-      queue_done(&gate[2]);
-      continue;
+    // steps: 0 zero the counts (one task), 1 histogram, 2 + p pass p, the last:
+    // nothing left.  The look-back words of a pass are zeroed in the step before.
+    u32 t = s_q.task, step = 0;
+    if (t >= 1) {
+      t -= 1;
+      step = 1;
+      if (t >= nh) {
+        t -= nh;
+        step = 2 + min(t / plan.ntiles, (u32)plan.passes);
+        t -= (step - 2) * plan.ntiles;
+      }
     }
-    t -= nz;
-    if (t < nh) {
-      if (!expired) expired = queue_wait(&gate[2], nz);
-      hist_block<kQBits>(src, plan.n, plan.passes, plan.key_bits, ghist, bstart, counters + plan.passes,
-                         reinterpret_cast<u32*>(smem), t, nh);
-      queue_done(&gate[3]);
-      continue;
+    if (step != s_q.step) {
+      if (threadIdx.x == 0 && s_q.count) {  // (behind the barriers above: for the whole CTA)
+        __threadfence();
+        atomicAdd(&gate[2 + s_q.step], s_q.count);
+      }
+      if (step == 2 + (u32)plan.passes) return;
+      bool expired = s_q.expired != 0u;
+      if (!expired) expired = queue_wait(&gate[1 + step], step == 1 ? 1 : step == 2 ? nh : plan.ntiles);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        s_q.step = step;
+        s_q.count = 0u;
+        s_q.expired = expired;
+      }
     }
-    t -= nh;
-    const int p = (int)(t / plan.ntiles);
-    if (p >= plan.passes) return;
-    if (!expired) expired = queue_wait(&gate[3 + p], p == 0 ? nh : plan.ntiles);
-    const int which = (plan.passes - 1 - p) & 1, shift = p * kQBits;
-    const u32 mask = (1u << min(kQBits, plan.key_bits - shift)) - 1u;
-    u64* ok = which ? buf1_k : buf0_k;
-    double* ov = which ? buf1_v : buf0_v;
-    u32* st = status + (size_t)p * plan.ntiles * RADIX;
-    t -= (u32)p * plan.ntiles;
-    if (p == 0) {
-      onesweep_tile<kQBits, kThreads, kQItems, kQWindow, true>(src, ok, ov, plan.n, (u32)shift, mask, bstart, st, t,
-                                                               smem);
+    if (step == 0) {
+      u32* z = reinterpret_cast<u32*>(ctrl);
+      for (size_t i = threadIdx.x; i < plan.off_status / 4; i += THREADS) z[i] = 0u;
+      for (size_t i = plan.off_counters / 4 + threadIdx.x; i < plan.ctrl_bytes / 4; i += THREADS) z[i] = 0u;
+    } else if (step == 1) {
+      uint4* z = reinterpret_cast<uint4*>(status);
+      for (size_t i = (size_t)t * THREADS + threadIdx.x; i < (size_t)plan.ntiles * (RADIX / 4); i += (size_t)nh * THREADS)
+        z[i] = make_uint4(0u, 0u, 0u, 0u);
+      hist_block<BITS, THREADS>(src, plan.n, plan.passes, plan.key_bits, ghist, bstart, counters + plan.passes,
+                                reinterpret_cast<u32*>(smem), t, nh);
     } else {
-      PairSource in = src;
-      in.ak = which ? buf0_k : buf1_k;
-      in.av = which ? buf0_v : buf1_v;
-      onesweep_tile<kQBits, kThreads, kQItems, kQWindow, false>(in, ok, ov, plan.n, (u32)shift, mask,
-                                                                bstart + p * RADIX, st, t, smem);
+      const int p = (int)step - 2, which = (plan.passes - 1 - p) & 1, shift = p * BITS;
+      const u32 mask = (1u << min(BITS, plan.key_bits - shift)) - 1u;
+      u64* ok = which ? buf1_k : buf0_k;
+      double* ov = which ? buf1_v : buf0_v;
+      u32* st = status + (size_t)(p & 1) * plan.ntiles * RADIX;
+      if (p + 1 < plan.passes) {
+        u32* after = status + ((size_t)(~p & 1) * plan.ntiles + t) * RADIX;
+        for (int d = threadIdx.x; d < RADIX; d += THREADS) after[d] = 0u;
+      }
+      if (p == 0) {
+        onesweep_tile<BITS, THREADS, ITEMS, W, true, true>(src, ok, ov, plan.n, (u32)shift, mask, bstart, st, t, smem,
+                                                           &s_q, gate);
+      } else {
+        PairSource in = src;
+        in.ak = which ? buf0_k : buf1_k;
+        in.av = which ? buf0_v : buf1_v;
+        onesweep_tile<BITS, THREADS, ITEMS, W, false, true>(in, ok, ov, plan.n, (u32)shift, mask, bstart + p * RADIX,
+                                                            st, t, smem, &s_q, gate);
+      }
     }
-    queue_done(&gate[4 + p]);
+    if (threadIdx.x == 0) ++s_q.count;
   }
 }
 
@@ -507,6 +543,22 @@ __global__ void copy_source_kernel(const PairSource src, u64* __restrict__ ok, d
 #define LNT_SV_ENTRY(B, T, I, W) {B, T, I, W},
 const SortVariant kVariants[] = {LNT_SORT_VARIANTS(LNT_SV_ENTRY)};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
+
+template <int BITS, int THREADS, int ITEMS, int W>
+int run_sort_queue(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* buf0_v, u64* buf1_k,
+                   double* buf1_v, void* ctrl, cudaStream_t s) {
+  using Sh = OnesweepShape<BITS, THREADS, ITEMS>;
+  static_assert(Sh::smem >= ((63 + BITS) / BITS) * (size_t)Sh::RADIX * 4, "the histogram of every pass fits");
+  auto kern = lsd_queue_kernel<BITS, THREADS, ITEMS, W>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem) != cudaSuccess)
+    return LNT_DEVICE_ERROR;
+  const u32 grid = std::min(plan.ntiles, (u32)(Sh::MINB * sm_count()));
+  ProfScope prof("sort_fallback", s);
+  kern<<<grid, THREADS, Sh::smem, s>>>(src, plan, buf0_k, buf0_v, buf1_k, buf1_v, static_cast<unsigned char*>(ctrl),
+                                       const_cast<u32*>(src.gate));
+  count_launch();
+  return launch_status();
+}
 
 template <int BITS, int THREADS, int ITEMS, int W>
 int run_sort_variant(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* buf0_v, u64* buf1_k,
@@ -597,11 +649,27 @@ int choose_sort_variant(size_t n, int key_bits) {
   return best;
 }
 
+// The shape behind a gate, of three compiled as a queue.  Below 2^22 pairs CTAs of
+// 512 threads, with nine-bit digits where those save a pass; above, 256 threads of
+// twelve keys (clustered keys, 512 and 256 threads: 2^19 pairs of 36 bits 101 and
+// 117 us, 2^21 211 and 227, 2^23 622 and 599, 2^25 2.17 and 1.96 ms).
+#define LNT_QUEUE_VARIANTS(X) \
+  X(8, 512, 8, 16)            \
+  X(9, 512, 8, 16)            \
+  X(8, 256, 12, 16)
+const SortVariant kQueueVariants[] = {LNT_QUEUE_VARIANTS(LNT_SV_ENTRY)};
+
+int choose_queue_variant(size_t n, int key_bits) {
+  if (n >= (1u << 22)) return 2;
+  return (key_bits + 8) / 9 < (key_bits + 7) / 8 ? 1 : 0;
+}
+
 SortPlan make_sort_plan(size_t n, u64 max_key, bool gated) {
   SortPlan p;
   p.key_bits = key_bits_for(max_key);
-  p.variant = gated ? -1 : choose_sort_variant(n, p.key_bits);
-  const SortVariant v = gated ? SortVariant{kQBits, kThreads, kQItems, kQWindow} : kVariants[p.variant];
+  p.variant = gated ? choose_queue_variant(n, p.key_bits) : choose_sort_variant(n, p.key_bits);
+  p.gated = gated;
+  const SortVariant v = gated ? kQueueVariants[p.variant] : kVariants[p.variant];
   p.bits = v.bits;
   p.passes = p.key_bits == 0 ? 0 : (p.key_bits + v.bits - 1) / v.bits;
   p.n = (u32)n;
@@ -614,7 +682,8 @@ SortPlan make_sort_plan(size_t n, u64 max_key, bool gated) {
   p.off_bstart = off;
   off += align_up((size_t)std::max(p.passes, 1) * radix * 4, 256);
   p.off_status = off;
-  off += align_up((size_t)p.passes * p.ntiles * radix * 4, 256);
+  // (behind a gate the passes take turns in two sets of look-back words)
+  off += align_up((size_t)(gated ? std::min(p.passes, 2) : p.passes) * p.ntiles * radix * 4, 256);
   p.off_counters = off;
   off += 256;
   p.ctrl_bytes = off;
@@ -631,20 +700,17 @@ int run_sort(const SortPlan& plan, const PairSource& src, u64* buf0_k, double* b
     count_launch();
     return launch_status();
   }
-  if (plan.variant < 0) {  // behind a gate
-    constexpr size_t sh = QueueShape::smem;
-    static_assert(sh >= 8u * (1u << kQBits) * 4u, "the histogram of eight passes fits");
-    if (cudaFuncSetAttribute(lsd_queue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh) != cudaSuccess)
-      return LNT_DEVICE_ERROR;
-    const u32 grid = std::min(plan.ntiles, (u32)(QueueShape::MINB * sm_count()));
-    ProfScope prof("sort_fallback", s);
-    lsd_queue_kernel<<<grid, kThreads, sh, s>>>(src, plan, buf0_k, buf0_v, buf1_k, buf1_v,
-                                                static_cast<unsigned char*>(ctrl), const_cast<u32*>(src.gate));
-    count_launch();
-    return launch_status();
-  }
   int i = 0;
-#define LNT_SV_CASE(B, T, I, W)                                                          \
+  if (plan.gated) {
+#define LNT_QV_CASE(B, T, I, W)                                                          \
+  if (plan.variant == i) return run_sort_queue<B, T, I, W>(plan, src, buf0_k, buf0_v,   \
+                                                           buf1_k, buf1_v, ctrl, s);     \
+  ++i;
+    LNT_QUEUE_VARIANTS(LNT_QV_CASE)
+#undef LNT_QV_CASE
+    return LNT_UNSUPPORTED;
+  }
+#define LNT_SV_CASE(B, T, I, W)                                                                           \
   if (plan.variant == i) return run_sort_variant<B, T, I, W>(plan, src, buf0_k, buf0_v, \
                                                              buf1_k, buf1_v, ctrl, s);   \
   ++i;

@@ -92,6 +92,7 @@ const SortVariant& sort_variant(int i);
 
 struct SortPlan {
   int variant = 0;
+  bool gated = false;  // one launch behind a gate
   int key_bits = 0;
   int bits = 8;      // digit width
   int passes = 0;
