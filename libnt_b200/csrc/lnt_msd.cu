@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(kHistThreads, 1) msd_hist_kernel(const PairSou
   u64 any = 0;
   constexpr int U = 8;
   // Clustered keys: once a CTA has counted more of one bucket than fits, the rest
-  // need not be read.  Looked for after 2, 4, 8 .. rounds, while at least as many
-  // are left.
+  // need not be read.  Looked for after 2, 8, 32 .. rounds, while at least as many
+  // are left (2 to 3 us each).
   u32 round = 0, next_look = 2;
   bool closed = false;
   const u32 rounds = (u32)(n / ((u64)gridDim.x * (kHistThreads * U)));
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kHistThreads, 1) msd_hist_kernel(const PairSou
         any |= k[u];
       }
     if (++round == next_look && 2 * round <= rounds) {
-      next_look *= 2;
+      next_look *= 4;
       __syncthreads();
       u32 most = 0;
       for (int i = tid; i < nb; i += kHistThreads) most = max(most, sh[i]);
@@ -474,10 +474,10 @@ __device__ __forceinline__ void sort_by_digits(R* s_r, u32* s_cnt, u32* s_tmp, u
   }
 }
 
-// Sub-buckets of more than kSubThread records, which a single thread would sort
-// for long (20 equal keys per sub-bucket: 2000 pairs 69 us, 27 like this): every
-// record of theirs counts the smaller words of its sub-bucket and goes to its
-// rank.  sub_of(word): the word's sub-bucket.
+// Sorts the sub-buckets where some have more than kSubThread records, which a
+// single thread would sort for long (20 equal keys per sub-bucket: 2000 pairs 69
+// us, 27 like this): every record counts the smaller words of its sub-bucket and
+// goes to its rank.  sub_of(word): the word's sub-bucket.
 template <int BT, int I, class R, class SubOf>
 __device__ __forceinline__ void rank_sub_buckets(R* s_r, const u32* s_cnt, const unsigned short* s_base, u32 cnt,
                                               const SubOf sub_of) {
@@ -492,7 +492,7 @@ __device__ __forceinline__ void rank_sub_buckets(R* s_r, const u32* s_cnt, const
       x[j] = s_r[p];
       const u64 w = word_of(x[j]);
       const u32 sub = sub_of(w), sh = 8u * (sub & 3u), c4 = s_cnt[sub >> 2], k = (c4 >> sh) & 0xFFu;
-      if (k > (u32)kSubThread) {
+      if (k > 1u) {
         const u32 lo = s_base[sub >> 2] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
         u32 rank = 0;
         for (u32 q = 0; q < k; ++q) rank += word_of(s_r[lo + q]) < w ? 1u : 0u;
@@ -508,17 +508,6 @@ __device__ __forceinline__ void rank_sub_buckets(R* s_r, const u32* s_cnt, const
     if (p < cnt && at != p) s_r[at] = x[j];
   }
   __syncthreads();
-}
-
-// Sorts the sub-buckets that are too long for a thread, or the whole bucket when
-// it is crowded.  (A function of its own: these paths are rare, and their
-// registers would be taken from the others.)
-template <class G>
-__device__ __noinline__ void sort_long(ulonglong2* s_r, u32* s_cnt, unsigned short* s_base, u32 cnt, int sshift,
-                                       bool crowded) {
-  static_assert(G::kWarps * 256 <= G::kSubWords, "the counts of the sub-buckets hold one per warp and digit");
-  if (crowded) sort_by_digits<G::kBT, G::kItems>(s_r, s_cnt, reinterpret_cast<u32*>(s_base), cnt);
-  else rank_sub_buckets<G::kBT, G::kItems>(s_r, s_cnt, s_base, cnt, [=](u64 w) { return (u32)(w >> sshift); });
 }
 
 // The run of equal keys that starts at each head of row g (32 sorted positions,
@@ -599,7 +588,7 @@ __device__ __forceinline__ void fold_row(const u32* heads, u32 rows, u32 g, u32 
 // sum of its run, and s_kept the mask of the heads that are written.  s_head:
 // room for a mask per 32 positions; first: the bucket begins the sorted array.
 template <int BT>
-__device__ __noinline__ void fold_bucket(ulonglong2* s_r, u32* s_head, u32* s_kept, u32 cnt, int ib,
+__device__ __forceinline__ void fold_bucket(ulonglong2* s_r, u32* s_head, u32* s_kept, u32 cnt, int ib,
                                          int skip_zero_heads, bool first) {
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rows = (cnt + 31) / 32;
   for (u32 g = warp; g < rows; g += BT / 32) {
@@ -622,13 +611,25 @@ __device__ __noinline__ void fold_bucket(ulonglong2* s_r, u32* s_head, u32* s_ke
   }
 }
 
-// Sorts the k records of one sub-bucket by word (one thread); fold adds up its
+// Sorts and folds a bucket that has a sub-bucket too long for a thread, or that is
+// crowded.  (A function of its own: such buckets are rare, and their registers
+// would be taken from the others.)
+template <class G, bool FOLD>
+__device__ __noinline__ void long_bucket(ulonglong2* s_r, u32* s_cnt, unsigned short* s_base, u32* s_head, u32* s_kept,
+                                         u32 cnt, int sshift, bool crowded, int ib, int skip_zero_heads, bool first) {
+  static_assert(G::kWarps * 256 <= G::kSubWords, "the counts of the sub-buckets hold one per warp and digit");
+  if (crowded) sort_by_digits<G::kBT, G::kItems>(s_r, s_cnt, reinterpret_cast<u32*>(s_base), cnt);
+  else rank_sub_buckets<G::kBT, G::kItems>(s_r, s_cnt, s_base, cnt, [=](u64 w) { return (u32)(w >> sshift); });
+  if (FOLD) fold_bucket<G::kBT>(s_r, s_head, s_kept, cnt, ib, skip_zero_heads, first);
+}
+
+// Sorts the k records of one sub-bucket by word (one thread); FOLD adds up its
 // runs of equal keys in that (input) order into their first record and clears
 // the kept bits of the others and of the dropped ones.  `at`: the position of
 // r[0] in the bucket; first: it is the first of the whole sorted array.
 template <bool FOLD>
 __device__ __forceinline__ void fold_sub_bucket(ulonglong2* r, int k, int ib, int skip_zero_heads, bool first, u32 at,
-                                                u32* kept, bool fold) {
+                                                u32* kept) {
   for (int i = 1; i < k; ++i) {  // insertion sort
     const ulonglong2 x = r[i];
     int q = i;
@@ -639,7 +640,7 @@ __device__ __forceinline__ void fold_sub_bucket(ulonglong2* r, int k, int ib, in
     }
     if (q != i) r[q] = x;
   }
-  if (!FOLD || !fold) return;
+  if (!FOLD) return;
   for (int i = 0; i < k;) {
     const u64 low = r[i].x >> ib;
     double sum = __longlong_as_double((long long)r[i].y);
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
   if (FOLD && tid == 0) s_misc[0] = atomicAdd(&c.misc[1], 1u);
 #pragma unroll
   for (int j = 0; j < G::kSubPer; ++j) s_cnt[j * BT + tid] = 0;
-  if (tid == 0) s_misc[1] = s_misc[4] = 0;
+  if (tid == 0) s_misc[1] = 0;
   __syncthreads();
   const u32 b = FOLD ? s_misc[0] : blockIdx.x;  // FOLD: in order of arrival, for the look-back
   const u32 start = c.start[b];
@@ -710,9 +711,9 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
 #pragma unroll
     for (int j = 0; j < P2; ++j) most = __vmaxu2(most, pos[j]);
     most = max(most & 0xFFFFu, most >> 16);
-    if (most >= (u32)kSubThread) s_misc[4] = 1;  // some sub-bucket is too long for a thread
-    // crowded (some slot at the limit): the counts may have run over, and are not used
-    if (most >= (u32)kSubMax) s_misc[1] = 1;
+    // bit 0: some sub-bucket is too long for a thread; bit 1, crowded (some slot
+    // at the limit): the counts may have run over, and are not used
+    if (most >= (u32)kSubThread) atomicOr(&s_misc[1], most >= (u32)kSubMax ? 3u : 1u);
   }
   __syncthreads();
   {  // records before every count word
@@ -749,7 +750,8 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
     *reinterpret_cast<uint4*>(&s_base[tid * 8]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   }
   __syncthreads();
-  const bool ranked = s_misc[1] == 0, by_rows = s_misc[4] != 0;
+  const u32 how = s_misc[1];
+  const bool ranked = how < 2u;
 #pragma unroll
   for (int j = 0; j < I; ++j) {  // place every record in its sub-bucket (crowded: as they are, to be sorted)
     const u32 p = j * BT + tid;
@@ -766,13 +768,11 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
     s_r[q] = r[j];
   }
   __syncthreads();
-  if (by_rows) sort_long<G>(s_r, s_cnt, s_base, cnt, sshift, !ranked);
-  if (ranked) {
-    // sort (and fold, unless the bucket is folded as a whole) the sub-buckets
-    // of two to kSubThread records, each by one thread: about one per thread, of
-    // two records.  Count words go to the threads in turn, so that each gets its
-    // share also when the key has fewer bits than there are sub-buckets.
-    const bool fold_here = FOLD && !by_rows;
+  if (how == 0u) {
+    // sort (and fold) the sub-buckets of more than one record, each by one
+    // thread: about one per thread, of two records.  Count words go to the
+    // threads in turn, so that each gets its share also when the key has
+    // fewer bits than there are sub-buckets.
     u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
       if (k == 2) {  // nearly always
         const bool swap = e1.x < e0.x;
         const ulonglong2 f = swap ? e1 : e0, g = swap ? e0 : e1;
-        if (fold_here) {
+        if (FOLD) {
           const double x = __longlong_as_double((long long)f.y), y = __longlong_as_double((long long)g.y);
           const bool equal = ((f.x ^ g.x) >> ib) == 0;
           u32 drop = equal ? 2u : 0u;  // bit q: position lo + q is not written
@@ -809,14 +809,12 @@ __global__ void __launch_bounds__(G::kBT, G::kMinBlocks)
           s_r[lo] = f;
           s_r[lo + 1] = g;
         }
-      } else if (k <= (u32)kSubThread) {
-        fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept, fold_here);
+      } else {
+        fold_sub_bucket<FOLD>(s_r + lo, (int)k, ib, skip_zero_heads, start + lo == 0, lo, s_kept);
       }
     }
-  }
-  if (FOLD && by_rows) {
-    __syncthreads();
-    fold_bucket<G::kBT>(s_r, s_pre, s_kept, cnt, ib, skip_zero_heads, start == 0);
+  } else {
+    long_bucket<G, FOLD>(s_r, s_cnt, s_base, s_pre, s_kept, cnt, sshift, !ranked, ib, skip_zero_heads, start == 0);
   }
   __syncthreads();
   const u64 prefix = (u64)b << shift;
@@ -960,7 +958,7 @@ __device__ __forceinline__ u32 one_sum(u32 v, u32* s, u32* total) {
   return (warp == 0 ? 0u : before) + inc - v;
 }
 
-// As sort_long; a crowded CTA with one key throughout, and all of its pairs, has
+// As long_bucket, without the fold; a crowded CTA with one key throughout, and all of its pairs, has
 // them in input order.
 __device__ __noinline__ void small_sort_long(u64* s_w, u32* s_cnt, unsigned short* s_base, u32 n, u32 cnt,
                                              u64 first_key, int sshift, bool crowded) {
@@ -1097,8 +1095,9 @@ __global__ void __launch_bounds__(kOneThreads, 1)
     }
     __syncthreads();
   }
-  if (s_misc[43]) small_sort_long(s_w, s_cnt, s_base, n, cnt, first_key, sshift, !ranked);
-  if (ranked) {
+  if (s_misc[43]) {
+    small_sort_long(s_w, s_cnt, s_base, n, cnt, first_key, sshift, !ranked);
+  } else {
     u32 todo = 0;  // bit 4 j + i: count i of word j * BT + tid is above 1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -1111,7 +1110,6 @@ __global__ void __launch_bounds__(kOneThreads, 1)
       const u32 c4 = s_cnt[(i >> 2) * BT + tid];
       u64* r = s_w + s_base[(i >> 2) * BT + tid] + __dp4a(c4 & ((1u << sh) - 1u), 0x01010101u, 0u);
       const int k = (int)((c4 >> sh) & 0xFFu);
-      if (k > kSubThread) continue;
       for (int x = 1; x < k; ++x) {
         const u64 a = r[x];
         int q = x;
