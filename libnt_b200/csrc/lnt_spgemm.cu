@@ -38,8 +38,6 @@
 
 namespace lnt {
 
-int run_collect(const u64* keys, const double* vals, size_t n, int skip_zero_heads, u64* out_k, double* out_v,
-                u64* d_nout, void* ws, cudaStream_t s);
 size_t collect_workspace_bytes(size_t n);
 bool tile_shape_ok(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb);
 size_t tile_workspace_bytes(u64 h, u64 w, u64 wB, u64 d, u64 na, u64 nb, bool buckets);

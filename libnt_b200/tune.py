@@ -71,7 +71,7 @@ def time_sort(L, torch, n, key_bits, variant, reps=5):
 def load_tuned() -> dict:
     if TUNED_JSON.exists():
         return json.loads(TUNED_JSON.read_text())
-    return {"sort": [], "pass8_variant": 0, "batch_chunk": 8, "tile_dense_div": 8}
+    return {"sort": [], "batch_chunk": 8, "tile_dense_div": 8}
 
 
 def render_header(tuned: dict) -> str:
